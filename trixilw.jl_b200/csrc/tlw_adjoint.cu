@@ -916,21 +916,21 @@ template <int N>
 struct AL {
     static void set_attributes() {
         cudaFuncSetAttribute(lw_volume_kernel<N, MODE_STEP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)VolCfg<N>::smem_bytes(4));
+                             (int)VolCfg<N>::lw_bytes());
         cudaFuncSetAttribute(lw_volume_kernel<N, MODE_RHS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)VolCfg<N>::smem_bytes(4));
+                             (int)VolCfg<N>::lw_bytes());
         cudaFuncSetAttribute(adj_volume_kernel<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)AdjCfg<N>::smem_bytes());
         cudaFuncSetAttribute(adj_volume_reg_kernel<N, AdjCfg<N>::MIN_BLOCKS>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AdjCfg<N>::reg_smem_bytes());
         cudaFuncSetAttribute(lw_volume_kernel<N, MODE_STEP, false, 0, false, false, true>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VolCfg<N>::smem_bytes(4));
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VolCfg<N>::lw_bytes());
         cudaFuncSetAttribute(lw_volume_kernel<N, MODE_RHS, false, 0, false, false, true>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VolCfg<N>::smem_bytes(4));
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VolCfg<N>::lw_bytes());
         cudaFuncSetAttribute(mdrk1_volume_kernel<N, MODE_STEP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)VolCfg<N>::smem_bytes(2));
+                             (int)VolCfg<N>::mdrk_bytes());
         cudaFuncSetAttribute(mdrk2_volume_kernel<N, MODE_STEP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)VolCfg<N>::smem_bytes(2));
+                             (int)VolCfg<N>::mdrk_bytes());
         cudaFuncSetAttribute(adj_mdrk_volume_kernel<N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)AdjMdrkCfg<N>::smem_bytes());
         cudaFuncSetAttribute(adj_mdrk_volume_kernel<N, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -940,8 +940,8 @@ struct AL {
     static void forward_mdrk_volume(cudaStream_t s, int stage, const VolArgs& va) {
         using C = VolCfg<N>;
         const int grid = (int)((va.E + C::EB - 1) / C::EB);
-        if (stage == 1) mdrk1_volume_kernel<N, MODE_STEP, false><<<grid, C::THREADS, C::smem_bytes(2), s>>>(va);
-        else mdrk2_volume_kernel<N, MODE_STEP, false><<<grid, C::THREADS, C::smem_bytes(2), s>>>(va);
+        if (stage == 1) mdrk1_volume_kernel<N, MODE_STEP, false><<<grid, C::THREADS, C::mdrk_bytes(), s>>>(va);
+        else mdrk2_volume_kernel<N, MODE_STEP, false><<<grid, C::THREADS, C::mdrk_bytes(), s>>>(va);
     }
     static void adjoint_mdrk(cudaStream_t s, int stage, const AdjSurfArgs& sa, const AdjMdrkArgs& ma) {
         const long long th = (long long)(sa.nx + sa.ny) * (N + 1);
@@ -955,7 +955,7 @@ struct AL {
     static void forward_volume(cudaStream_t s, int mode, const VolArgs& va) {
         using C = VolCfg<N>;
         const int grid = (int)((va.E + C::EB - 1) / C::EB);
-        const size_t sm = C::smem_bytes(4);
+        const size_t sm = C::lw_bytes();
         if (va.dstore) {
             if (mode == MODE_STEP) lw_volume_kernel<N, MODE_STEP, false, 0, false, false, true><<<grid, C::THREADS, sm, s>>>(va);
             else lw_volume_kernel<N, MODE_RHS, false, 0, false, false, true><<<grid, C::THREADS, sm, s>>>(va);
@@ -1158,7 +1158,7 @@ VolArgs fwd_vol_args(tlw_handle* h, const double* u, double* out, double* tU, co
     va.dt = dtp;
     va.basis = h->d_basis;
     va.E = (int)h->E;
-    va.gamma = h->opts.gamma;
+    va.set_gamma(h->opts.gamma);
     va.status = &h->d_step->status;
     va.speed_kind = h->opts.max_speed;
     return va;

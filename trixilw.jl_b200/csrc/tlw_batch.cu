@@ -106,19 +106,19 @@ template <int N>
 struct BLaunch {
     static void set_attributes() {
         cudaFuncSetAttribute(lw_volume_kernel<N, MODE_STEP, false, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)VolCfg<N, 0>::smem_bytes(4));
+                             (int)VolCfg<N, 0>::lw_bytes());
         cudaFuncSetAttribute(lw_volume_kernel<N, MODE_STEP, false, AltEB<N>::v>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VolCfg<N, AltEB<N>::v>::smem_bytes(4));
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VolCfg<N, AltEB<N>::v>::lw_bytes());
     }
     static void volume(cudaStream_t s, int variant, const VolArgs& a) {
         if (variant == 0) {
             using C = VolCfg<N, 0>;
             lw_volume_kernel<N, MODE_STEP, false, 0>
-                <<<(unsigned)((a.E + C::EB - 1) / C::EB), C::THREADS, C::smem_bytes(4), s>>>(a);
+                <<<(unsigned)((a.E + C::EB - 1) / C::EB), C::THREADS, C::lw_bytes(), s>>>(a);
         } else {
             using C = VolCfg<N, AltEB<N>::v>;
             lw_volume_kernel<N, MODE_STEP, false, AltEB<N>::v>
-                <<<(unsigned)((a.E + C::EB - 1) / C::EB), C::THREADS, C::smem_bytes(4), s>>>(a);
+                <<<(unsigned)((a.E + C::EB - 1) / C::EB), C::THREADS, C::lw_bytes(), s>>>(a);
         }
     }
     static void surfaces(cudaStream_t s, const SurfArgs& a) {
@@ -158,7 +158,7 @@ VolArgs vol_args(tlw_batch* b, Group& g, int from) {
     va.inv_jac = g.d_inv_jac;
     va.dt = b->d_dt;
     va.E = (int)g.E;
-    va.gamma = b->opts.gamma;
+    va.set_gamma(b->opts.gamma);
     va.status = &b->d_step->status;
     va.speed_kind = b->opts.max_speed;
     va.inst = g.d_inst;

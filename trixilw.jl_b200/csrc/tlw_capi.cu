@@ -480,7 +480,7 @@ void enqueue_rhs(tlw_handle* h, int stage, int mode, const double* u_flux, const
     va.dt = dt_ptr;
     va.basis = h->d_basis;
     va.E = (int)h->E;
-    va.gamma = h->opts.gamma;
+    va.set_gamma(h->opts.gamma);
     va.alpha = h->d_alpha;
     va.tFn = h->d_tFn;
     va.status = &h->d_step->status;

@@ -138,7 +138,7 @@ __device__ __forceinline__ double checked_sqrt(double x, unsigned* status) {
 
 // Trixi max_abs_speeds: |v1| + c and |v2| + c of a state, computed the same way by every CFL pass
 __device__ __forceinline__ void node_speeds(double gamma, const double* x, unsigned* status, double& l1, double& l2) {
-    const double ir = 1.0 / x[0];
+    const double ir = nr_reciprocal(x[0]);
     const double v1 = x[1] * ir, v2 = x[2] * ir;
     const double p = (gamma - 1.0) * (x[3] - 0.5 * (x[1] * v1 + x[2] * v2));
     const double c = checked_sqrt(gamma * p * ir, status);

@@ -22,7 +22,7 @@ struct LaunchImpl {
     using C = VolCfg<N>;
     template <bool SC>
     static void set_attr_sc() {
-        const int lw = (int)C::smem_bytes(SC ? 8 : 4), md = (int)C::smem_bytes(SC ? 8 : 2);
+        const int lw = (int)C::lw_bytes(SC), md = (int)C::mdrk_bytes(SC);
         cudaFuncSetAttribute(lw_volume_kernel<N, MODE_RHS, SC>, cudaFuncAttributeMaxDynamicSharedMemorySize, lw);
         cudaFuncSetAttribute(lw_volume_kernel<N, MODE_STEP, SC>, cudaFuncAttributeMaxDynamicSharedMemorySize, lw);
         cudaFuncSetAttribute(mdrk1_volume_kernel<N, MODE_RHS, SC>, cudaFuncAttributeMaxDynamicSharedMemorySize, md);
@@ -33,20 +33,20 @@ struct LaunchImpl {
     static void set_attributes() {
         set_attr_sc<false>();
         set_attr_sc<true>();
-        const int lw = (int)C::smem_bytes(4);
+        const int lw = (int)C::lw_bytes();
         cudaFuncSetAttribute(lw_volume_kernel<N, MODE_RHS, false, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lw);
         te_volume(nullptr, VolArgs{}, 0, false, true);
         cudaFuncSetAttribute(lw_volume_kernel<N, MODE_STEP, false, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lw);
         curved_sc_attributes<0>();
         curved_sc_attributes<1>();
         curved_sc_attributes<2>();
-        const int md = (int)C::smem_bytes(2);
+        const int md = (int)C::mdrk_bytes();
         cudaFuncSetAttribute(mdrk1_volume_kernel<N, MODE_RHS, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, md);
         cudaFuncSetAttribute(mdrk1_volume_kernel<N, MODE_STEP, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, md);
         cudaFuncSetAttribute(mdrk2_volume_kernel<N, MODE_RHS, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, md);
         cudaFuncSetAttribute(mdrk2_volume_kernel<N, MODE_STEP, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, md);
         cudaFuncSetAttribute(mdrk2_volume_kernel<N, MODE_STEP, false, false, 0, false, true>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_bytes(5));
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::mdrk_bytes(false, 0, true));
         // source terms (FR)
         cudaFuncSetAttribute(lw_volume_kernel<N, MODE_RHS, false, 0, false, false, false, 0, true>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, lw);
@@ -68,7 +68,7 @@ struct LaunchImpl {
     // source terms (FR volume integral, TreeMesh or curvilinear): LW or an MDRK stage
     template <bool CURVED>
     static void volume_src_on(cudaStream_t s, int stage, int mode, const VolArgs& a, int grid) {
-        const size_t lw = C::smem_bytes(4), md = C::smem_bytes(2);
+        const size_t lw = C::lw_bytes(), md = C::mdrk_bytes();
         if (stage == TLW_STAGE_LW) {
             if (mode == MODE_RHS) lw_volume_kernel<N, MODE_RHS, false, 0, CURVED, false, false, 0, true><<<grid, C::THREADS, lw, s>>>(a);
             else lw_volume_kernel<N, MODE_STEP, false, 0, CURVED, false, false, 0, true><<<grid, C::THREADS, lw, s>>>(a);
@@ -86,7 +86,7 @@ struct LaunchImpl {
     }
     template <bool SC>
     static void volume_sc(cudaStream_t s, int stage, int mode, const VolArgs& a, int grid) {
-        const size_t lw = C::smem_bytes(SC ? 8 : 4), md = C::smem_bytes(SC ? 8 : 2);
+        const size_t lw = C::lw_bytes(SC), md = C::mdrk_bytes(SC);
         if (stage == TLW_STAGE_LW) {
             if (mode == MODE_RHS) lw_volume_kernel<N, MODE_RHS, SC><<<grid, C::THREADS, lw, s>>>(a);
             else lw_volume_kernel<N, MODE_STEP, SC><<<grid, C::THREADS, lw, s>>>(a);
@@ -97,7 +97,7 @@ struct LaunchImpl {
         } else {
             if (mode == MODE_RHS) mdrk2_volume_kernel<N, MODE_RHS, SC><<<grid, C::THREADS, md, s>>>(a);
             else if (!SC && a.compact)
-                mdrk2_volume_kernel<N, MODE_STEP, false, false, 0, false, true><<<grid, C::THREADS, C::smem_bytes(5), s>>>(a);
+                mdrk2_volume_kernel<N, MODE_STEP, false, false, 0, false, true><<<grid, C::THREADS, C::mdrk_bytes(false, 0, true), s>>>(a);
             else mdrk2_volume_kernel<N, MODE_STEP, SC><<<grid, C::THREADS, md, s>>>(a);
         }
     }
@@ -105,7 +105,7 @@ struct LaunchImpl {
     // (REC 2) subcells
     template <int REC>
     static void curved_sc(cudaStream_t s, int stage, int mode, const VolArgs& a, int grid) {
-        const size_t sm = C::smem_bytes(REC ? 12 : 8);
+        const size_t sm = C::mdrk_bytes(true, REC), lw = C::lw_bytes(true, REC);
         if (stage == TLW_STAGE_MDRK1) {
             if (mode == MODE_RHS) mdrk1_volume_kernel<N, MODE_RHS, true, true, REC><<<grid, C::THREADS, sm, s>>>(a);
             else mdrk1_volume_kernel<N, MODE_STEP, true, true, REC><<<grid, C::THREADS, sm, s>>>(a);
@@ -113,15 +113,15 @@ struct LaunchImpl {
             if (mode == MODE_RHS) mdrk2_volume_kernel<N, MODE_RHS, true, true, REC><<<grid, C::THREADS, sm, s>>>(a);
             else mdrk2_volume_kernel<N, MODE_STEP, true, true, REC><<<grid, C::THREADS, sm, s>>>(a);
         } else {
-            if (mode == MODE_RHS) lw_volume_kernel<N, MODE_RHS, true, 0, true, false, false, REC><<<grid, C::THREADS, sm, s>>>(a);
-            else lw_volume_kernel<N, MODE_STEP, true, 0, true, false, false, REC><<<grid, C::THREADS, sm, s>>>(a);
+            if (mode == MODE_RHS) lw_volume_kernel<N, MODE_RHS, true, 0, true, false, false, REC><<<grid, C::THREADS, lw, s>>>(a);
+            else lw_volume_kernel<N, MODE_STEP, true, 0, true, false, false, REC><<<grid, C::THREADS, lw, s>>>(a);
         }
     }
     template <int REC>
     static void curved_sc_attributes() {
-        const int sm = (int)C::smem_bytes(REC ? 12 : 8);
-        cudaFuncSetAttribute(lw_volume_kernel<N, MODE_RHS, true, 0, true, false, false, REC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
-        cudaFuncSetAttribute(lw_volume_kernel<N, MODE_STEP, true, 0, true, false, false, REC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        const int sm = (int)C::mdrk_bytes(true, REC), lw = (int)C::lw_bytes(true, REC);
+        cudaFuncSetAttribute(lw_volume_kernel<N, MODE_RHS, true, 0, true, false, false, REC>, cudaFuncAttributeMaxDynamicSharedMemorySize, lw);
+        cudaFuncSetAttribute(lw_volume_kernel<N, MODE_STEP, true, 0, true, false, false, REC>, cudaFuncAttributeMaxDynamicSharedMemorySize, lw);
         cudaFuncSetAttribute(mdrk1_volume_kernel<N, MODE_RHS, true, true, REC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
         cudaFuncSetAttribute(mdrk1_volume_kernel<N, MODE_STEP, true, true, REC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
         cudaFuncSetAttribute(mdrk2_volume_kernel<N, MODE_RHS, true, true, REC>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
@@ -132,7 +132,7 @@ struct LaunchImpl {
     // memory attributes of every variant instead
     template <bool SC, bool CURVED, int REC>
     static void te_launch(cudaStream_t s, const VolArgs& a, int grid, bool attr_only) {
-        const int sm = (int)C::smem_bytes(!SC ? 4 : REC ? 12 : 8);
+        const int sm = (int)C::lw_bytes(SC, REC);
         if (attr_only)
             cudaFuncSetAttribute(lw_volume_kernel<N, MODE_STEP, SC, 0, CURVED, true, false, REC>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
@@ -172,7 +172,7 @@ struct LaunchImpl {
             return;
         }
         if (a.metrics) {   // curvilinear mesh (LW or MDRK, FR volume integral)
-            const size_t md = C::smem_bytes(2);
+            const size_t md = C::mdrk_bytes();
             if (stage == TLW_STAGE_MDRK1) {
                 if (mode == MODE_RHS) mdrk1_volume_kernel<N, MODE_RHS, false, true><<<grid, C::THREADS, md, s>>>(a);
                 else mdrk1_volume_kernel<N, MODE_STEP, false, true><<<grid, C::THREADS, md, s>>>(a);
@@ -180,9 +180,9 @@ struct LaunchImpl {
                 if (mode == MODE_RHS) mdrk2_volume_kernel<N, MODE_RHS, false, true><<<grid, C::THREADS, md, s>>>(a);
                 else mdrk2_volume_kernel<N, MODE_STEP, false, true><<<grid, C::THREADS, md, s>>>(a);
             } else if (mode == MODE_RHS) {
-                lw_volume_kernel<N, MODE_RHS, false, 0, true><<<grid, C::THREADS, C::smem_bytes(4), s>>>(a);
+                lw_volume_kernel<N, MODE_RHS, false, 0, true><<<grid, C::THREADS, C::lw_bytes(), s>>>(a);
             } else {
-                lw_volume_kernel<N, MODE_STEP, false, 0, true><<<grid, C::THREADS, C::smem_bytes(4), s>>>(a);
+                lw_volume_kernel<N, MODE_STEP, false, 0, true><<<grid, C::THREADS, C::lw_bytes(), s>>>(a);
             }
             return;
         }

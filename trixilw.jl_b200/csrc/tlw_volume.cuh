@@ -2,8 +2,8 @@
 //
 // Work split inside a CTA of EB whole elements (N=3: 8 x 16 nodes in 128 threads, N=4: 5 x 25 in 128,
 // N=5: 7 x 36 in 256):
-//  * node phase - one thread per GLL node ("owner") evaluates the Euler fluxes at the perturbed states and
-//    keeps all LW stage state (u +- ut, u +- 2ut, the time averages U, F, G) in registers;
+//  * node phase - one thread per GLL node ("owner") evaluates the Euler flux products at the perturbed states
+//    (StencilSum) and keeps the LW stage state (u +- ut, u +- 2ut, the time averages F, G) in registers;
 //  * line phase - each 1-D derivative contraction is done by one thread per (variable, element, line
 //    index) that reads a whole row of f and a whole column of g from shared memory once, multiplies by
 //    the derivative matrix held in constant memory (compile-time indices: the matrix entries are FMA
@@ -14,6 +14,10 @@
 // writes 2n. HBM traffic per element: read u once, write du (or u^{n+1}) once, write the face traces of
 // U and F.n for the interface kernels.
 //
+// What bounds it (512^2, N = 4, one B200): the LSU data pipe (shared-memory wavefronts first), 65 % busy, beside the
+// FP64 pipe (57 %) and the issue slots (55 %) at 20 warps an SM. Measured, this build against the one before the
+// stencil sums: N = 3 0.251 -> 0.196 ms, N = 4 0.509 -> 0.431 ms, N = 5 0.809 -> 0.699 ms.
+//
 // Restates, per element (TreeMesh, no source terms):
 //   LW depth 4 (N>=4): lw_volume_kernel_4!  src/solvers/dgsem_tree/dg_2d.jl:918-1249
 //   LW depth 3 (N=3):  lw_volume_kernel_3!  src/solvers/dgsem_tree/dg_2d.jl:674-913
@@ -22,10 +26,11 @@
 //   MDRK stage 1/2:    mdrk_kernel_1!/2!    src/solvers/dgsem_tree/multi_derivative_2d.jl:263-421, 423-555
 // then the Trixi apply_jacobian! factor -J^{-1} is folded into the written result.
 #pragma once
+#include <type_traits>
+
 #include "tlw_device.cuh"
 
 namespace tlw {
-
 // EBX = 0: the default number of elements per CTA; another value selects a tuned variant
 // elements per CTA at N = 5: 3 (108 of 128 threads busy, 5 CTAs per SM) measured 4 % faster than 7 (252 of
 // 256 threads, 2 CTAs per SM) and 10 % faster than 10 on the 512^2 step
@@ -43,21 +48,50 @@ struct VolCfg {
     // whole elements per CTA, chosen so that the CTA is (nearly) full warps
     static constexpr int EB = EBX ? EBX : N == 1 ? 32 : N == 2 ? 14 : N == 3 ? 8 : N == 4 ? 5 : N == 5 ? TLW_EB_N5 : N == 6 ? 5 : 2;
     static constexpr int THREADS = ((EB * nn + 31) / 32) * 32;
-    // resident CTAs per SM the register allocation must allow (5 CTAs of 128 threads: <= 96 registers, measured
-    // 4 % faster than 4 CTAs at 128 registers on the N = 4 workload; 6 CTAs spill)
+    // resident CTAs per SM the register allocation must allow (5 CTAs of 128 threads: <= 96 registers. 512^2, N = 4:
+    // 0.465 ms, against 0.483 with 4 CTAs and 0.505 with 6, which spill; N = 3: 6 CTAs 0.232 against 0.213 ms)
     static constexpr int MIN_BLOCKS = THREADS <= 128 ? TLW_VOLUME_MIN_BLOCKS : 2;
     static constexpr int MDRK_MIN_BLOCKS = THREADS <= 128 ? 5 : 2;
     // curvilinear shock capturing (subcell normals, MUSCL face values): 4 CTAs of 128 threads, 128 registers
     static constexpr int SC_CURVED_MIN_BLOCKS = THREADS <= 128 ? 4 : 2;
-    // plane layout: node (i, j) of (variable v, element e) at (v*EB + e)*P + i + R*j
-    static constexpr int R = n;
-    static constexpr int P = n == 4 ? 19 : nn;
-    static constexpr int PLANES = 4 * EB * P;          // doubles of one 4-variable field
+    // plane layout: node (i, j) of (variable v, element e) at v*PV + e*P + i + R*j, on the Y planes of n = 4
+    // transposed (YI, YJ); line threads take the variable innermost, then the element (LINE_E) or the line index.
+    // P, PV and the order were chosen by counting the shared-memory wavefronts of the owner accesses and of the row
+    // and column accesses (two a 64-bit warp access without conflicts). A contraction of a CTA then takes, against
+    // element planes back to back with the line index innermost: N = 2 272 against 326, N = 3 256 (no conflicts)
+    // against 320, N = 4 268 against 328, N = 5 292 against 340, N = 6 550 against 746, N = 7 320 against 768.
+    static constexpr int R = n, YI = n == 4 ? n : 1, YJ = n == 4 ? 1 : n;
+    static constexpr int P = n == 8 ? 65 : nn;
+    static constexpr int PAD = n == 3 ? 6 : n == 4 ? 1 : n == 5 ? (EB % 2 ? 7 : 2) : n == 6 ? (EB > 3 ? 1 : 0) : n == 7 ? 7 : 0;
+    static constexpr int PV = EB * P + PAD;
+    static constexpr bool LINE_E = !(n == 4 || (n == 6 && EB == 3) || (n == 5 && EB == 10) || n == 7);
+    // n = 4: a warp holds two whole elements, as nodes and as lines, so its phases need no CTA barrier
+    static constexpr bool WARP_LOCAL = n == 4;
+    static constexpr int PLANES = 4 * PV;              // doubles of one 4-variable field
     static constexpr int LINES = 4 * n * EB;           // (variable, element, line index)
-    // regions: X (f / x-results), Y (g / y-results), F0X, F0Y (fluxes at u, kept for stages 2 and 4);
-    // shock capturing adds UU (u), VC (v1, v2, c), FVX, FVY (first-order subcell fluxes)
-    static constexpr size_t smem_bytes(int regions) { return (size_t)regions * PLANES * sizeof(double); }
+    static constexpr int NODES = EB * nn;              // node slots of the CTA
+    // doubles a node of the compact MDRK stage 2 keeps for itself (slot k of the node of thread t at k*NODES + t)
+    static constexpr int MDRK_KEEP = 9;
+    // regions: X (f / x-results), Y (g / y-results); shock capturing adds F0X, F0Y (fluxes at u), UU (u), VC (v1, v2,
+    // c), FVX, FVY (first-order subcell fluxes), and with MUSCL subcells four regions of face values
+    __host__ __device__ static constexpr size_t regions(bool sc, int rec) { return (size_t)(!sc ? 2 : rec ? 12 : 8) * PLANES; }
+    static constexpr size_t lw_bytes(bool sc = false, int rec = 0) { return regions(sc, rec) * sizeof(double); }
+    static constexpr size_t mdrk_bytes(bool sc = false, int rec = 0, bool compact = false) {
+        return (regions(sc, rec) + (size_t)(compact ? MDRK_KEEP : 0) * NODES) * sizeof(double);
+    }
 };
+
+// Taylor weights that are no short immediates: as constant operands they cost no instructions of their own (512^2,
+// N = 4: 0.4366 -> 0.4325 ms)
+static __constant__ double c_tlw_taylor[30] = {
+    1.0, 1.0, 1.0 / 2.0, 1.0 / 6.0, 1.0 / 24.0,                  // 1 / M!
+    2.0, 2.0, 4.0 / 3.0, 2.0 / 3.0,                              // 2^M / M!, M = 1..4
+    0.25, 0.0, 0.0, 0.0,                                         // C_M / (M + 1)!, depth 1
+    0.25, 1.0 / 6.0, 0.0, 0.0,                                   // depth 2
+    1.0 / 24.0, 1.0 / 6.0, 1.0 / 48.0, 0.0,                      // depth 3
+    1.0 / 24.0, 1.0 / 72.0, 1.0 / 48.0, 1.0 / 240.0,             // depth 4
+    // int_0^1 of the quartic through its values at k = 0, 1, -1, 2, -2
+    456.0 / 720.0, 346.0 / 720.0, -74.0 / 720.0, -19.0 / 720.0, 11.0 / 720.0};
 
 enum VolMode { MODE_RHS = 0, MODE_STEP = 1 };
 
@@ -81,7 +115,8 @@ struct VolArgs {
     const double* dt;       // device scalar
     const Basis* basis;
     int E;
-    double gamma;
+    double gamma, gm1, hg, inv_gamma;   // gamma, gamma - 1, (gamma - 1) / 2, 1 / gamma (set_gamma)
+    void set_gamma(double g) { gamma = g; gm1 = g - 1.0; hg = 0.5 * gm1; inv_gamma = 1.0 / g; }
     // shock capturing (VolumeIntegralFRShockCapturing, first-order subcells)
     const double* alpha;    // blending factor per element
     double* tFn;            // first-order subcell flux next to each face [v, l, face, e] (fn_low)
@@ -119,23 +154,41 @@ __device__ __forceinline__ void contravariant(const double* Ja, const double* f,
     }
 }
 
-// owner: store the node's f (into X) and g (into Y)
+// The records (K doubles a node) of the CTA that gets a free slot next, into L2: CTAs start in order, so that is the
+// one as many further on as CTAs are resident, and its first loads then miss DRAM (512^2: N = 3 0.2143 -> 0.2105 ms,
+// N = 4 0.4522 -> 0.4495, N = 5 0.7457 -> 0.7303). Threads ask for one 128-byte line each; nothing past the array.
+template <class C>
+__device__ __forceinline__ void prefetch_next(const double* p, int K, int E, int tid) {
+    constexpr int AHEAD = 148 * C::MIN_BLOCKS;
+    const size_t first = ((size_t)blockIdx.x + AHEAD) * C::NODES * K + (size_t)tid * 16;
+    if (tid * 16 < C::NODES * K && first < (size_t)E * C::nn * K)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p + first));
+}
+
+// barrier between the node phase and the line phase of the same elements
+template <class C>
+__device__ __forceinline__ void phase_sync() {
+    if constexpr (C::WARP_LOCAL) __syncwarp();
+    else __syncthreads();
+}
+
+// owner: the node's f and g into the contraction planes X and Y
+template <int N, class C>
+__device__ __forceinline__ void line_put(double* X, double* Y, int e, int i, int j, const double* f, const double* g) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        X[v * C::PV + e * C::P + i + C::R * j] = f[v];
+        Y[v * C::PV + e * C::P + C::YI * i + C::YJ * j] = g[v];
+    }
+}
+// owner: two fields of the node into two planes of the same layout
 template <int N, class C>
 __device__ __forceinline__ void node_put(double* X, double* Y, int e, int i, int j, const double* f, const double* g) {
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-        const int a = (v * C::EB + e) * C::P + i + C::R * j;
+        const int a = v * C::PV + e * C::P + i + C::R * j;
         X[a] = f[v];
         Y[a] = g[v];
-    }
-}
-template <int N, class C>
-__device__ __forceinline__ void node_get(const double* X, const double* Y, int e, int i, int j, double* f, double* g) {
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        const int a = (v * C::EB + e) * C::P + i + C::R * j;
-        f[v] = X[a];
-        g[v] = Y[a];
     }
 }
 // owner: x-result + y-result at the node
@@ -143,8 +196,8 @@ template <int N, class C>
 __device__ __forceinline__ void node_sum(const double* X, const double* Y, int e, int i, int j, double* d) {
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-        const int a = (v * C::EB + e) * C::P + i + C::R * j;
-        d[v] = X[a] + Y[a];
+        const int a = v * C::PV + e * C::P;
+        d[v] = X[a + i + C::R * j] + Y[a + C::YI * i + C::YJ * j];
     }
 }
 
@@ -159,70 +212,55 @@ __device__ __forceinline__ void node_sum(const double* X, const double* Y, int e
 #define TLW_LINE_EVENODD 1
 #endif
 template <int N, class C, bool HAT>
-__device__ __forceinline__ void line_contract(double* X, double* Y, int tid) {
+__device__ __forceinline__ void line_contract_one(double* X, double* Y, int t) {
     constexpr int n = C::n;
-#if TLW_LINE_EVENODD
-    if constexpr (n >= 5) {
+    const int r = t >> 2;
+    const int e = C::LINE_E ? r % C::EB : r / n, idx = C::LINE_E ? r / C::EB : r % n;
+    const int pb = (t & 3) * C::PV + e * C::P;
+    if constexpr (TLW_LINE_EVENODD && n >= 5) {
         constexpr int h = n / 2;
         constexpr int hh = h * h;
         const double* E = HAT ? c_tlw_Dhat_eo[N] : c_tlw_D_eo[N];
-#pragma unroll 1
-        for (int t = tid; t < C::LINES; t += C::THREADS) {
-            const int idx = t % n;
-            const int r = t / n;
-            const int e = r % C::EB;
-            const int v = r / C::EB;
-            const int pb = (v * C::EB + e) * C::P;
-            // one line at a time (the row of X, then the column of Y) keeps the sums and differences of one
-            // line live, not two
-            auto line = [&](double* L, int base, int stride) {
-                double a[n];
+        // one line at a time (the row of X, then the column of Y) keeps the sums and differences of one line live,
+        // not two
+        auto line = [&](double* L, int base, int stride) {
+            double a[n];
 #pragma unroll
-                for (int k = 0; k < n; ++k) a[k] = L[base + stride * k];
-                double as[h], ad[h];
+            for (int k = 0; k < n; ++k) a[k] = L[base + stride * k];
+            double as[h], ad[h];
 #pragma unroll
-                for (int k = 0; k < h; ++k) {
-                    as[k] = a[k] + a[n - 1 - k];
-                    ad[k] = a[k] - a[n - 1 - k];
+            for (int k = 0; k < h; ++k) {
+                as[k] = a[k] + a[n - 1 - k];
+                ad[k] = a[k] - a[n - 1 - k];
+            }
+#pragma unroll
+            for (int o = 0; o < h; ++o) {
+                double xa = E[o * h] * as[0], xb = E[hh + o * h] * ad[0];
+#pragma unroll
+                for (int k = 1; k < h; ++k) {
+                    xa = fma(E[o * h + k], as[k], xa);
+                    xb = fma(E[hh + o * h + k], ad[k], xb);
                 }
+                if constexpr (n % 2) xa = fma(E[2 * hh + o], a[h], xa);
+                L[base + stride * o] = xb + xa;
+                L[base + stride * (n - 1 - o)] = xb - xa;
+            }
+            if constexpr (n % 2) {
+                double xm = E[2 * hh + h] * ad[0];
 #pragma unroll
-                for (int o = 0; o < h; ++o) {
-                    double xa = E[o * h] * as[0], xb = E[hh + o * h] * ad[0];
-#pragma unroll
-                    for (int k = 1; k < h; ++k) {
-                        xa = fma(E[o * h + k], as[k], xa);
-                        xb = fma(E[hh + o * h + k], ad[k], xb);
-                    }
-                    if constexpr (n % 2) xa = fma(E[2 * hh + o], a[h], xa);
-                    L[base + stride * o] = xb + xa;
-                    L[base + stride * (n - 1 - o)] = xb - xa;
-                }
-                if constexpr (n % 2) {
-                    double xm = E[2 * hh + h] * ad[0];
-#pragma unroll
-                    for (int k = 1; k < h; ++k) xm = fma(E[2 * hh + h + k], ad[k], xm);
-                    L[base + stride * h] = xm;
-                }
-            };
-            line(X, pb + C::R * idx, 1);
-            line(Y, pb + idx, C::R);
-        }
-        return;
-    }
-#endif
-    const double* M = HAT ? c_tlw_Dhat[N] : c_tlw_D[N];
-#pragma unroll 1
-    for (int t = tid; t < C::LINES; t += C::THREADS) {
-        const int idx = t % n;
-        const int r = t / n;
-        const int e = r % C::EB;
-        const int v = r / C::EB;
-        const int pb = (v * C::EB + e) * C::P;
+                for (int k = 1; k < h; ++k) xm = fma(E[2 * hh + h + k], ad[k], xm);
+                L[base + stride * h] = xm;
+            }
+        };
+        line(X, pb + C::R * idx, 1);
+        line(Y, pb + idx, C::R);
+    } else {
+        const double* M = HAT ? c_tlw_Dhat[N] : c_tlw_D[N];
         double a[n], b[n];
 #pragma unroll
         for (int k = 0; k < n; ++k) {
             a[k] = X[pb + k + C::R * idx];
-            b[k] = Y[pb + idx + C::R * k];
+            b[k] = Y[pb + C::YI * idx + C::YJ * k];
         }
 #pragma unroll
         for (int o = 0; o < n; ++o) {
@@ -233,8 +271,17 @@ __device__ __forceinline__ void line_contract(double* X, double* Y, int tid) {
                 sy = fma(M[o * n + k], b[k], sy);
             }
             X[pb + o + C::R * idx] = sx;
-            Y[pb + idx + C::R * o] = sy;
+            Y[pb + C::YI * idx + C::YJ * o] = sy;
         }
+    }
+}
+template <int N, class C, bool HAT>
+__device__ __forceinline__ void line_contract(double* X, double* Y, int tid) {
+    if constexpr (C::LINES <= C::THREADS) {
+        if (tid < C::LINES) line_contract_one<N, C, HAT>(X, Y, tid);
+    } else {
+#pragma unroll 1
+        for (int t = tid; t < C::LINES; t += C::THREADS) line_contract_one<N, C, HAT>(X, Y, t);
     }
 }
 
@@ -257,7 +304,7 @@ template <int N, class C>
 __device__ __forceinline__ void sc_face_flux(const double* UU, const double* VC, const double* FL, int el, int iL,
                                              int jL, int iR, int jR, int orientation, int speed_kind, double* out) {
     const int aL = el * C::P + iL + C::R * jL, aR = el * C::P + iR + C::R * jR;
-    constexpr int PV = C::EB * C::P;   // stride between variable planes
+    constexpr int PV = C::PV;   // stride between variable planes
     const double vL = VC[(orientation == 1 ? 0 : PV) + aL], vR = VC[(orientation == 1 ? 0 : PV) + aR];
     const double cL = VC[2 * PV + aL], cR = VC[2 * PV + aR];
     const double lambda = speed_kind == 0 ? fmax(fabs(vL), fabs(vR)) + fmax(cL, cR)
@@ -271,7 +318,7 @@ __device__ __forceinline__ void sc_face_flux(const double* UU, const double* VC,
 template <int N, class C>
 __device__ __forceinline__ void sc_faces(const double* UU, const double* VC, const double* F0X, const double* F0Y,
                                          double* FVX, double* FVY, int el, int i, int j, int speed_kind) {
-    constexpr int PV = C::EB * C::P;
+    constexpr int PV = C::PV;
     const int a = el * C::P + i + C::R * j;
     double f[NV];
     if (i >= 1) {
@@ -292,7 +339,7 @@ template <int N, class C>
 __device__ __forceinline__ void sc_blend(const VolArgs& a, const double* FVX, const double* FVY, int el, int e, int i,
                                          int j, double alpha, double* acc) {
     constexpr int n = C::n;
-    constexpr int PV = C::EB * C::P;
+    constexpr int PV = C::PV;
     const int base = el * C::P;
     const double iwi = 1.0 / c_tlw_w[N][i], iwj = 1.0 / c_tlw_w[N][j];
 #pragma unroll
@@ -412,7 +459,7 @@ template <int N, class C, int REC>
 __device__ __forceinline__ void sc_muscl_faces(const VolArgs& a, const double* UU, double* UF, int el, int e, int i,
                                                int j, double gm1, double alpha, double dt_fv, double ij) {
     constexpr int n = C::n, nn = n * n;
-    constexpr int PV = C::EB * C::P;
+    constexpr int PV = C::PV;
     const double* sf = a.muscl_geom;           // subcell faces [0..n]
     const double* xe = a.muscl_geom + n + 1;   // extended nodes [0..n+1]
     auto at = [&](int ii, int jj, int v) {
@@ -505,7 +552,7 @@ __device__ __forceinline__ void sc_faces_curved(const VolArgs& a, const double* 
                                                 const double* F0Y, const double* UF, double* FVX, double* FVY, int el,
                                                 int e, int i, int j, bool blended, bool muscl) {
     constexpr int n = C::n;
-    constexpr int PV = C::EB * C::P;
+    constexpr int PV = C::PV;
     const double gm1 = a.gamma - 1.0;
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
@@ -557,7 +604,7 @@ template <int N, class C>
 __device__ __forceinline__ void sc_blend_curved(const VolArgs& a, const double* FVX, const double* FVY, int el, int e,
                                                 int i, int j, double alpha, bool blended, double* acc) {
     constexpr int n = C::n;
-    constexpr int PV = C::EB * C::P;
+    constexpr int PV = C::PV;
     const int base = el * C::P;
     if (blended) {
         const double iwi = 1.0 / c_tlw_w[N][i], iwj = 1.0 / c_tlw_w[N][j];
@@ -588,38 +635,37 @@ __device__ __forceinline__ void sc_blend_curved(const VolArgs& a, const double* 
     }
 }
 
-// out/traces epilogue shared by all volume kernels. acc = Dhat-contraction of (F, G).
-template <int n, int MODE>
-__device__ __forceinline__ void volume_epilogue(const VolArgs& a, int e, int i, int j, int node, double ij, double dt,
-                                                const double* acc, const double* U, const double* F,
-                                                const double* G, double* o, const double* S = nullptr) {
-    const size_t off = ((size_t)e * n * n + node) * NV;
-    if (MODE == MODE_RHS) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) o[v] = -ij * acc[v];
-        if (S) {   // du += S (the source enters unscaled by J^{-1})
-#pragma unroll
-            for (int v = 0; v < NV; ++v) o[v] += S[v];
-        }
-    } else {
-        double ub[NV];
-        load4(a.u_base + off, ub);
-        const double s = -dt * ij;
-        if (S) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) ub[v] = fma(dt, S[v], ub[v]);
-        }
-#pragma unroll
-        for (int v = 0; v < NV; ++v) o[v] = fma(s, acc[v], ub[v]);
-    }
-    store4(a.out + off, o);
-    // face traces [v, l, face, e]; face 0 = -x, 1 = +x, 2 = -y, 3 = +y
+// The face traces [v, l, face, e] of U and F.n of a node (faces -x, +x, -y, +y), written as soon as U, F, G are formed,
+// so that they are not held over the last contraction. One store for the two x faces and one for the two y faces: a
+// 256-bit warp store costs eight wavefronts however few lanes are active.
+template <int n>
+__device__ __forceinline__ void store_traces(const VolArgs& a, int e, int i, int j, const double* U, const double* F,
+                                             const double* G) {
     const size_t tb = (size_t)e * 4 * n * NV;
     const bool nf = a.tG == nullptr;   // UnstructuredMesh2D: the flux traces were written before (physical)
-    if (i == 0) { store4(a.tU + tb + (0 * n + j) * NV, U); if (nf) store4(a.tF + tb + (0 * n + j) * NV, F); }
-    if (i == n - 1) { store4(a.tU + tb + (1 * n + j) * NV, U); if (nf) store4(a.tF + tb + (1 * n + j) * NV, F); }
-    if (j == 0) { store4(a.tU + tb + (2 * n + i) * NV, U); if (nf) store4(a.tF + tb + (2 * n + i) * NV, G); }
-    if (j == n - 1) { store4(a.tU + tb + (3 * n + i) * NV, U); if (nf) store4(a.tF + tb + (3 * n + i) * NV, G); }
+    if (i == 0 || i == n - 1) {
+        const size_t k = tb + ((i == 0 ? 0 : n) + j) * NV;
+        store4w(a.tU + k, U);
+        if (nf) store4w(a.tF + k, F);
+    }
+    if (j == 0 || j == n - 1) {
+        const size_t k = tb + ((j == 0 ? 2 * n : 3 * n) + i) * NV;
+        store4w(a.tU + k, U);
+        if (nf) store4w(a.tF + k, G);
+    }
+}
+
+// The node's result: o = s acc (+ S), the rhs (MODE_RHS, s = -J^{-1}), or base + s acc (+ dt S), the updated state
+// (MODE_STEP, s = -dt J^{-1}). acc = Dhat-contraction of (F, G), S the source's time average.
+template <int MODE>
+__device__ __forceinline__ void store_result(double* out, double s, double dt, const double* acc, const double* base,
+                                             const double* S, double* o) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        if (MODE == MODE_RHS) o[v] = S ? s * acc[v] + S[v] : s * acc[v];   // (S enters unscaled by J^{-1})
+        else o[v] = fma(s, acc[v], S ? fma(dt, S[v], base[v]) : base[v]);
+    }
+    store4w(out, o);
 }
 
 // UnstructuredMesh2D: the physical time-averaged fluxes F (x) and G (y) on every face the node lies on, which its
@@ -720,12 +766,49 @@ __device__ __forceinline__ void write_interior_slots(const VolArgs& a, double* X
     }
 }
 
-// The stage's four flux pairs at upp, up, um, umm. With TLW_VOL_ILP the four reciprocals 1/rho are refined
-// first, as four independent Newton chains, instead of one chain per flux pair; same operations, same bits.
-#ifndef TLW_VOL_ILP
-#define TLW_VOL_ILP 1
-#endif
+// Flux pairs and their stencils. The stencils of the time derivatives of f and g are sums over the perturbed states
+// of products, of which five differ: rho v1^2, rho |v|^2, rho v1 v2, H v1 and H v2 (H = rho e + p); what is linear in
+// the state (rho v1, rho v2 and the rho e part of p) has a stencil of L times the current derivative d of the state,
+// L the stencil's moment, so it is not summed at all: f = (L d_2, a + P, b, x), g = (L d_3, b, (s - a) + P, y) with
+// P = (gamma - 1)(L d_4 - s / 2). A state carries gamma rho e as its last variable, so that H is one multiply-add.
+// A stage of four pairs then takes 60 FP64 instructions instead of 96 (N = 4: about 730 -> 607 a node, counted).
+struct StencilSum {
+    double a, s, b, x, y;
+};
+// the products at p plus (SGN = 1) or minus (SGN = -1) those at m; hg = (gamma - 1) / 2, irp, irm = 1 / rho
+template <int SGN>
+__device__ __forceinline__ StencilSum stencil_pair(double hg, const double* p, double irp, const double* m, double irm) {
+    const double v1 = p[1] * irp, v2 = p[2] * irp, w1 = m[1] * irm, w2 = m[2] * irm;
+    const double ap = p[1] * v1, am = m[1] * w1;
+    const double sp = fma(p[2], v2, ap), sm = fma(m[2], w2, am);
+    const double hp = fma(-hg, sp, p[3]), hm = SGN * fma(-hg, sm, m[3]);
+    return StencilSum{fma((double)SGN, am, ap), fma((double)SGN, sm, sp), fma(SGN * m[1], w2, p[1] * v2),
+                      fma(hm, w1, hp * v1), fma(hm, w2, hp * v2)};
+}
+__device__ __forceinline__ StencilSum stencil_fma(double c, const StencilSum& t, const StencilSum& q) {   // c t + q
+    return StencilSum{fma(c, t.a, q.a), fma(c, t.s, q.s), fma(c, t.b, q.b), fma(c, t.x, q.x), fma(c, t.y, q.y)};
+}
+__device__ __forceinline__ StencilSum stencil_fmsub(double c, const StencilSum& t, const StencilSum& q) {  // c t - q
+    return StencilSum{fma(c, t.a, -q.a), fma(c, t.s, -q.s), fma(c, t.b, -q.b), fma(c, t.x, -q.x), fma(c, t.y, -q.y)};
+}
+__device__ __forceinline__ void stencil_fluxes(double gm1, double hg, double L, const StencilSum& r, const double* d,
+                                               double* f, double* g) {
+    const double P = fma(-hg, r.s, gm1 * (L * d[3]));
+    f[0] = L * d[1]; f[1] = r.a + P; f[2] = r.b; f[3] = r.x;
+    g[0] = L * d[2]; g[1] = r.b; g[2] = (r.s - r.a) + P; g[3] = r.y;
+}
+// the flux pair at u (unscaled rho e) and its products
+__device__ __forceinline__ StencilSum flux_base(double gm1, const double* u, double* f, double* g) {
+    const double ir = nr_reciprocal(u[0]);
+    const double v1 = u[1] * ir, v2 = u[2] * ir;
+    const double a = u[1] * v1, s = fma(u[2], v2, a), b = u[1] * v2;
+    const double p = gm1 * fma(-0.5, s, u[3]), h = u[3] + p;
+    f[0] = u[1]; f[1] = a + p; f[2] = b; f[3] = h * v1;
+    g[0] = u[2]; g[1] = b; g[2] = fma(u[2], v2, p); g[3] = h * v2;
+    return StencilSum{a, s, b, f[3], g[3]};
+}
 
+// the four reciprocals of a stage first, as independent chains
 struct Recip4 {
     double pp, p, m, mm;
 };
@@ -736,6 +819,23 @@ __device__ __forceinline__ Recip4 recip4(const double* upp, const double* up, co
     r.m = nr_reciprocal(um[0]);
     r.mm = nr_reciprocal(umm[0]);
     return r;
+}
+// the stencil of f_t, g_t at u +- d, u +- 2d times 12 (-f(u+2d) + 8 f(u+d) - 8 f(u-d) + f(u-2d)): an MDRK stage
+__device__ __forceinline__ void first_derivative_fluxes(const VolArgs& a, const double* u, const double* d, double* f,
+                                                        double* g) {
+    const double us[NV] = {u[0], u[1], u[2], a.gamma * u[3]}, ds[NV] = {d[0], d[1], d[2], a.gamma * d[3]};
+    double up[NV], um[NV], upp[NV], umm[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        up[v] = us[v] + ds[v];
+        um[v] = us[v] - ds[v];
+        upp[v] = fma(2.0, ds[v], us[v]);
+        umm[v] = fma(-2.0, ds[v], us[v]);
+    }
+    const Recip4 rc = recip4(upp, up, um, umm);
+    const StencilSum t = stencil_pair<-1>(a.hg, up, rc.p, um, rc.m);
+    const StencilSum q = stencil_pair<-1>(a.hg, upp, rc.pp, umm, rc.mm);
+    stencil_fluxes(a.gm1, a.hg, 12.0, stencil_fmsub(8.0, t, q), d, f, g);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -784,16 +884,20 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
     extern __shared__ double smem_d[];
     double* X = smem_d;
     double* Y = X + C::PLANES;
-    double* F0X = Y + C::PLANES;
+    double* F0X = Y + C::PLANES;       // shock capturing only
     double* F0Y = F0X + C::PLANES;
-    double* UU = F0Y + C::PLANES;      // shock capturing only
+    double* UU = F0Y + C::PLANES;
     double* VC = UU + C::PLANES;
     double* FVX = VC + C::PLANES;
     double* FVY = FVX + C::PLANES;
     double* UF = FVY + C::PLANES;      // curvilinear MUSCL: face values, 4 regions (left, right, down, up)
 
     const int tid = threadIdx.x;
-    const double gm1 = a.gamma - 1.0;
+    prefetch_next<C>(a.u, 4, a.E, tid);
+    if (CURVED) {
+        prefetch_next<C>(a.metrics, 4, a.E, tid);
+        prefetch_next<C>(a.inv_jac_node, 1, a.E, tid);
+    }
     const int el = tid / nn;
     const int node = tid - el * nn;
     const int i = node % n, j = node / n;
@@ -813,267 +917,155 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
     // per-element maxima of the interior nodes' speeds for the next step's CFL (plain LW step only)
     constexpr bool SLOTS = MODE == MODE_STEP && !SC && !CURVED;
 
+    // F[1..3] and G[2], G[3] are accumulated stage by stage; F[0], G[0] (the time averages of rho v1, rho v2) follow
+    // from U, and G[1] = F[2]. The states carry gamma rho e as their last variable (see StencilSum).
     double U[NV], F[NV], G[NV], up[NV], um[NV], upp[NV], umm[NV];
     double Ssrc[NV] = {0.0, 0.0, 0.0, 0.0};   // SRC: the source's time average S
     SrcNode sq{};
-    double s0 = 0.0, ij = 0.0;   // s0 = -dt J^{-1} (of the element, or of the node on curvilinear meshes)
-    double Ja[4] = {0.0, 0.0, 0.0, 0.0};
-    double dF[NV], dG[NV], u0[NV];   // TE: the last stage's term of F, G, and u
-    // stage fluxes into the contraction planes (contravariant on curvilinear meshes)
+    double s0 = 0.0;             // -dt J^{-1} (of the element, or of the node on curvilinear meshes)
+    double dF[NV], dG[NV];       // TE: the last stage's term of F, G
+    double ub[NV];               // u again, from the last stage on (the states' registers are free then)
+    auto inverse_jacobian = [&]() {
+        return CURVED ? __ldg(a.inv_jac_node + (size_t)e * nn + node) : __ldg(a.inv_jac + e);
+    };
+    // stage fluxes into the contraction planes (contravariant on curvilinear meshes, whose metric terms come from L1
+    // each time: held in registers they spilled, warped 201 x 167, N = 4)
     auto put = [&](const double* f, const double* g) {
         if (CURVED) {
-            double ft[NV], gt[NV];
+            double ft[NV], gt[NV], Ja[4];
+            load4w(a.metrics + ((size_t)e * nn + node) * 4, Ja);
             contravariant(Ja, f, g, ft, gt);
-            node_put<N, C>(X, Y, el, i, j, ft, gt);
+            line_put<N, C>(X, Y, el, i, j, ft, gt);
         } else {
-            node_put<N, C>(X, Y, el, i, j, f, g);
+            line_put<N, C>(X, Y, el, i, j, f, g);
         }
     };
-    // a flux pair at a perturbed state, from its precomputed 1/rho (TLW_VOL_ILP) or its own reciprocal
-    auto flux = [&](const double* st, double irr, double* f, double* g) {
-        if (TLW_VOL_ILP) euler_fluxes_ir(gm1, irr, st[1], st[2], st[3], f, g);
-        else euler_fluxes(gm1, st[0], st[1], st[2], st[3], f, g);
-    };
+    // u again where it is needed (from L1): the pass is bound by the shared-memory pipe, on which a global record
+    // costs as much as four 64-bit loads, and the products of the flux pair at u are cheaper formed again than kept
+    auto load_u = [&](double* uu) { load4w(a.u + ((size_t)e * nn + node) * NV, uu); };
     // stage 0: f, g at u (dg_2d.jl:941-971; dgsem_structured/dg_2d.jl:1709-1740)
     if (active) {
         double uu[NV], f[NV], g[NV];
-        load4(a.u + ((size_t)e * nn + node) * NV, uu);
-        if (TE) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) u0[v] = uu[v];
-        }
-        if (CURVED) {
-            load4(a.metrics + ((size_t)e * nn + node) * 4, Ja);
-            ij = __ldg(a.inv_jac_node + (size_t)e * nn + node);
-        } else {
-            ij = __ldg(a.inv_jac + e);
-        }
-        s0 = -dt * ij;
+        load4w(a.u + ((size_t)e * nn + node) * NV, uu);
+        s0 = -dt * inverse_jacobian();
         if (SRC) {
             // S = s(u, x, t) (dg_2d.jl:979-987)
             const double* xn = a.xnode + 2 * ((size_t)e * nn + node);
             sq = SrcNode{__ldg(xn), __ldg(xn + 1), *a.tnow, dt, a.gamma};
             src_eval(sq, 0.0, Ssrc);
         }
-        euler_fluxes(gm1, uu[0], uu[1], uu[2], uu[3], f, g);
+        flux_base(a.gm1, uu, f, g);
         put(f, g);
-        if (DEPTH >= 2 || SC) node_put<N, C>(F0X, F0Y, el, i, j, f, g);
+        if (SC) node_put<N, C>(F0X, F0Y, el, i, j, f, g);
         if (SC) sc_park<N, C>(UU, VC, el, i, j, uu, a.gamma, a.status);
+        uu[3] *= a.gamma;
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
-            F[v] = f[v]; G[v] = g[v]; U[v] = uu[v];
+            F[v] = f[v]; G[v] = g[v];
             up[v] = um[v] = upp[v] = umm[v] = uu[v];
         }
     }
-    __syncthreads();
-    line_contract<N, C, false>(X, Y, tid);
-    __syncthreads();
-    if (SC && CURVED && REC >= 1 && muscl) sc_muscl_faces<N, C, REC>(a, UU, UF, el, e, i, j, gm1, alpha_e, dt, ij);
 
-    // stage 1: ut; perturbed states; f_t (dg_2d.jl:972-1023 / :725-775 / :543-582 / :417-454)
-    if (active) {
-        double d[NV], r[NV], q[NV], f[NV], g[NV];
+    // stage M (dg_2d.jl:972-1206; depth 3 :725-875, depth 2 :543-634, depth 1 :417-454): the M-th derivative d of u
+    // (times dt^M), the perturbed states u + k d_1 + ... + k^M / M! d_M, k = +-1, +-2, and the stencil of their fluxes
+    auto stage = [&](auto stage_number) {
+        constexpr int M = decltype(stage_number)::value;
+        constexpr double CM[5] = {1.0, C1, C2, C3, C4};
+        constexpr double LM[5] = {0.0, DEPTH >= 3 ? 12.0 : 2.0, DEPTH == 4 ? 12.0 : 1.0, 2.0, 1.0};
+        constexpr double SIGN = M % 2 ? -1.0 : 1.0;
+        const double W1 = c_tlw_taylor[M], W2 = c_tlw_taylor[4 + M];
+        phase_sync<C>();
+        line_contract<N, C, false>(X, Y, tid);
+        phase_sync<C>();
+        if (M == 1 && SC && CURVED && REC >= 1 && muscl) sc_muscl_faces<N, C, REC>(a, UU, UF, el, e, i, j, a.gm1, alpha_e, dt, inverse_jacobian());
+        if (!active) return;
+        if (M == 2 || M == DEPTH) load_u(ub);
+        double d[NV], f[NV], g[NV];
         node_sum<N, C>(X, Y, el, i, j, d);
+        const double s = s0 * CM[M - 1];
+        double sk[NV];
+        if (SRC && M == 2) {   // s_t from the states after ut: N34 at depths 3, 4, N12 at depth 2 (dg_2d.jl:1027-1040)
+            if (DEPTH >= 3) src_t_N34(sq, sk);
+            else src_t_N12(sq, sk);
+        } else if (SRC && M == 3) {   // s_tt: N23 on the TreeMesh (dg_2d.jl:1093-1104), N4 on curvilinear depth 4
+            if (CURVED && DEPTH == 4) src_tt_N4(sq, sk);
+            else src_tt_N23(sq, sk);
+        } else if (SRC && M == 4) {
+            src_ttt_N34(sq, sk);      // s_ttt (dg_2d.jl:1148-1162)
+        }
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
-            d[v] *= s0;
-            if (SRC) d[v] = fma(dt, Ssrc[v], d[v]);   // ut += dt s
-            U[v] = fma(0.5, d[v], U[v]);
-            up[v] += d[v];
-            um[v] -= d[v];
-            if (DEPTH >= 3) { upp[v] = fma(2.0, d[v], upp[v]); umm[v] = fma(-2.0, d[v], umm[v]); }
+            d[v] *= s;
+            if (SRC && M > 1) Ssrc[v] = fma(W1, sk[v], Ssrc[v]);
+            if (SRC) d[v] = fma(dt, M == 1 ? Ssrc[v] : sk[v], d[v]);
         }
-        if (DSTORE) store_stage_derivative<nn>(a, 1, e, node, d);
+        if (DSTORE) store_stage_derivative<nn>(a, M, e, node, d);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const double dv = v == 3 ? a.gamma * d[3] : d[v];
+            up[v] = fma(W1, dv, up[v]);
+            um[v] = fma(SIGN * W1, dv, um[v]);
+            if (DEPTH >= 3) {
+                upp[v] = fma(W2, dv, upp[v]);
+                umm[v] = fma(SIGN * W2, dv, umm[v]);
+            }
+        }
+        StencilSum r, f0;
+        if (M == 2 || M == 4) f0 = flux_base(a.gm1, ub, f, g);
         if (DEPTH >= 3) {
-            // raw1 = -f(u+2ut) + 8 f(u+ut) - 8 f(u-ut) + f(u-2ut)
-            const Recip4 rc = TLW_VOL_ILP ? recip4(upp, up, um, umm) : Recip4{0.0, 0.0, 0.0, 0.0};
-            flux(upp, rc.pp, f, g);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) { r[v] = -f[v]; q[v] = -g[v]; }
-            flux(up, rc.p, f, g);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) { r[v] = fma(8.0, f[v], r[v]); q[v] = fma(8.0, g[v], q[v]); }
-            flux(um, rc.m, f, g);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) { r[v] = fma(-8.0, f[v], r[v]); q[v] = fma(-8.0, g[v], q[v]); }
-            flux(umm, rc.mm, f, g);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) { r[v] += f[v]; q[v] += g[v]; }
-        } else {
-            // raw1 = f(u+ut) - f(u-ut)
-            euler_fluxes(gm1, up[0], up[1], up[2], up[3], f, g);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) { r[v] = f[v]; q[v] = g[v]; }
-            euler_fluxes(gm1, um[0], um[1], um[2], um[3], f, g);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) { r[v] -= f[v]; q[v] -= g[v]; }
-        }
-#pragma unroll
-        for (int v = 0; v < NV; ++v) { F[v] = fma(0.5 * C1, r[v], F[v]); G[v] = fma(0.5 * C1, q[v], G[v]); }
-        if (DEPTH >= 2) put(r, q);
-    }
-    if (DEPTH >= 2) {
-        __syncthreads();
-        line_contract<N, C, false>(X, Y, tid);
-        __syncthreads();
-        // stage 2: utt; f_tt (dg_2d.jl:1025-1083 / :777-831 / :597-634)
-        if (active) {
-            double d[NV], f0[NV], g0[NV], r[NV], q[NV], f[NV], g[NV];
-            node_sum<N, C>(X, Y, el, i, j, d);
-            node_get<N, C>(F0X, F0Y, el, i, j, f0, g0);
-            const double s = s0 * C1;
-            double sk[NV];
-            if (SRC) {   // s_t from the states after ut: N34 at depths 3, 4, N12 at depth 2 (dg_2d.jl:1027-1040)
-                if (DEPTH >= 3) src_t_N34(sq, sk);
-                else src_t_N12(sq, sk);
-            }
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                d[v] *= s;
-                if (SRC) {
-                    Ssrc[v] = fma(0.5, sk[v], Ssrc[v]);
-                    d[v] = fma(dt, sk[v], d[v]);
-                }
-                U[v] = fma(1.0 / 6.0, d[v], U[v]);
-                up[v] = fma(0.5, d[v], up[v]);
-                um[v] = fma(0.5, d[v], um[v]);
-                if (DEPTH >= 3) { upp[v] = fma(2.0, d[v], upp[v]); umm[v] = fma(2.0, d[v], umm[v]); }
-            }
-            if (DSTORE) store_stage_derivative<nn>(a, 2, e, node, d);
-            if (DEPTH == 4) {
-                // raw2 = -f(upp) + 16 f(up) - 30 f0 + 16 f(um) - f(umm)
-                const Recip4 rc = TLW_VOL_ILP ? recip4(upp, up, um, umm) : Recip4{0.0, 0.0, 0.0, 0.0};
-                flux(upp, rc.pp, f, g);
-#pragma unroll
-                for (int v = 0; v < NV; ++v) {
-                    r[v] = fma(-30.0, f0[v], -f[v]);
-                    q[v] = fma(-30.0, g0[v], -g[v]);
-                }
-                flux(up, rc.p, f, g);
-#pragma unroll
-                for (int v = 0; v < NV; ++v) { r[v] = fma(16.0, f[v], r[v]); q[v] = fma(16.0, g[v], q[v]); }
-                flux(um, rc.m, f, g);
-#pragma unroll
-                for (int v = 0; v < NV; ++v) { r[v] = fma(16.0, f[v], r[v]); q[v] = fma(16.0, g[v], q[v]); }
-                flux(umm, rc.mm, f, g);
-#pragma unroll
-                for (int v = 0; v < NV; ++v) { r[v] -= f[v]; q[v] -= g[v]; }
+            const Recip4 rc = recip4(upp, up, um, umm);
+            const StencilSum t = stencil_pair<M % 2 ? -1 : 1>(a.hg, up, rc.p, um, rc.m);
+            if (M == 2 && DEPTH == 3) {
+                r = stencil_fma(-2.0, f0, t);                     // f(up) - 2 f0 + f(um)
             } else {
-                // raw2 = f(up) - 2 f0 + f(um)
-                euler_fluxes(gm1, up[0], up[1], up[2], up[3], f, g);
-#pragma unroll
-                for (int v = 0; v < NV; ++v) { r[v] = fma(-2.0, f0[v], f[v]); q[v] = fma(-2.0, g0[v], g[v]); }
-                euler_fluxes(gm1, um[0], um[1], um[2], um[3], f, g);
-#pragma unroll
-                for (int v = 0; v < NV; ++v) { r[v] += f[v]; q[v] += g[v]; }
+                const StencilSum q = stencil_pair<M % 2 ? -1 : 1>(a.hg, upp, rc.pp, umm, rc.mm);
+                if (M == 1) r = stencil_fmsub(8.0, t, q);                // -f(upp) + 8 f(up) - 8 f(um) + f(umm)
+                else if (M == 2) r = stencil_fma(16.0, t, stencil_fmsub(-30.0, f0, q));
+                                                                         // -f(upp) + 16 f(up) - 30 f0 + 16 f(um) - f(umm)
+                else if (M == 3) r = stencil_fma(-2.0, t, q);            // f(upp) - 2 f(up) + 2 f(um) - f(umm)
+                else r = stencil_fma(-4.0, t, stencil_fma(6.0, f0, q));
+                                                                         // f(upp) - 4 f(up) + 6 f0 - 4 f(um) + f(umm)
             }
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                F[v] = fma(C2 / 6.0, r[v], F[v]);
-                G[v] = fma(C2 / 6.0, q[v], G[v]);
-            }
-            if (DEPTH >= 3) put(r, q);
+        } else {
+            const double rp = nr_reciprocal(up[0]), rm = nr_reciprocal(um[0]);
+            r = stencil_pair<M % 2 ? -1 : 1>(a.hg, up, rp, um, rm);        // f(up) - f(um)
+            if (M == 2) r = stencil_fma(-2.0, f0, r);             // f(up) - 2 f0 + f(um)
         }
-    }
-    if (DEPTH >= 3) {
-        __syncthreads();
-        line_contract<N, C, false>(X, Y, tid);
-        __syncthreads();
-        // stage 3: uttt; f_ttt (dg_2d.jl:1085-1138 / :833-875)
-        if (active) {
-            double d[NV], r[NV], q[NV], f[NV], g[NV];
-            node_sum<N, C>(X, Y, el, i, j, d);
-            const double s = s0 * C2;
-            double sk[NV];
-            if (SRC) {   // s_tt: N23 at depths 3 and 4 on the TreeMesh (dg_2d.jl:1093-1104), N4 on curvilinear depth 4
-                if (CURVED && DEPTH == 4) src_tt_N4(sq, sk);
-                else src_tt_N23(sq, sk);
-            }
+        stencil_fluxes(a.gm1, a.hg, LM[M], r, d, f, g);
+        const double WC = c_tlw_taylor[9 + (DEPTH - 1) * 4 + M - 1];
 #pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                d[v] *= s;
-                if (SRC) {
-                    Ssrc[v] = fma(1.0 / 6.0, sk[v], Ssrc[v]);
-                    d[v] = fma(dt, sk[v], d[v]);
-                }
-                U[v] = fma(1.0 / 24.0, d[v], U[v]);
-                um[v] = fma(-1.0 / 6.0, d[v], um[v]);
-                up[v] = fma(1.0 / 6.0, d[v], up[v]);
-                umm[v] = fma(-4.0 / 3.0, d[v], umm[v]);
-                upp[v] = fma(4.0 / 3.0, d[v], upp[v]);
-            }
-            if (DSTORE) store_stage_derivative<nn>(a, 3, e, node, d);
-            // raw3 = f(upp) - 2 f(up) + 2 f(um) - f(umm)
-            const Recip4 rc = TLW_VOL_ILP ? recip4(upp, up, um, umm) : Recip4{0.0, 0.0, 0.0, 0.0};
-            flux(upp, rc.pp, f, g);
+        for (int v = 1; v < NV; ++v) F[v] = fma(WC, f[v], F[v]);
 #pragma unroll
-            for (int v = 0; v < NV; ++v) { r[v] = f[v]; q[v] = g[v]; }
-            flux(up, rc.p, f, g);
+        for (int v = 2; v < NV; ++v) G[v] = fma(WC, g[v], G[v]);
+        if (TE && M == DEPTH) {
 #pragma unroll
-            for (int v = 0; v < NV; ++v) { r[v] = fma(-2.0, f[v], r[v]); q[v] = fma(-2.0, g[v], q[v]); }
-            flux(um, rc.m, f, g);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) { r[v] = fma(2.0, f[v], r[v]); q[v] = fma(2.0, g[v], q[v]); }
-            flux(umm, rc.mm, f, g);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                r[v] -= f[v];
-                q[v] -= g[v];
-                F[v] = fma(C3 / 24.0, r[v], F[v]);
-                G[v] = fma(C3 / 24.0, q[v], G[v]);
-                if (TE && DEPTH == 3) { dF[v] = (C3 / 24.0) * r[v]; dG[v] = (C3 / 24.0) * q[v]; }
-            }
-            if (DEPTH >= 4) put(r, q);
+            for (int v = 0; v < NV; ++v) { dF[v] = WC * f[v]; dG[v] = WC * g[v]; }
         }
-    }
-    if (DEPTH >= 4) {
-        __syncthreads();
-        line_contract<N, C, false>(X, Y, tid);
-        __syncthreads();
-        // stage 4: utttt; f_tttt (dg_2d.jl:1140-1206)
-        if (active) {
-            double d[NV], f0[NV], g0[NV], r[NV], q[NV], f[NV], g[NV];
-            node_sum<N, C>(X, Y, el, i, j, d);
-            node_get<N, C>(F0X, F0Y, el, i, j, f0, g0);
-            const double s = s0 * C3;
-            double sk[NV];
-            if (SRC) src_ttt_N34(sq, sk);   // s_ttt (dg_2d.jl:1148-1162)
+        if (M < DEPTH) {
+            put(f, g);
+        } else {
+            // U = int_0^1 of the polynomial through the states at k = -2..2 (or -1..1)
+            const double uu[NV] = {ub[0], ub[1], ub[2], a.gamma * ub[3]};
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
-                d[v] *= s;
-                if (SRC) {
-                    Ssrc[v] = fma(1.0 / 24.0, sk[v], Ssrc[v]);
-                    d[v] = fma(dt, sk[v], d[v]);
-                }
-                U[v] = fma(1.0 / 120.0, d[v], U[v]);
-                um[v] = fma(1.0 / 24.0, d[v], um[v]);
-                up[v] = fma(1.0 / 24.0, d[v], up[v]);
-                umm[v] = fma(2.0 / 3.0, d[v], umm[v]);
-                upp[v] = fma(2.0 / 3.0, d[v], upp[v]);
+                if (DEPTH >= 3)
+                    U[v] = fma(c_tlw_taylor[25], uu[v], fma(c_tlw_taylor[26], up[v], fma(c_tlw_taylor[27], um[v],
+                           fma(c_tlw_taylor[28], upp[v], c_tlw_taylor[29] * umm[v]))));
+                else
+                    U[v] = fma(8.0 / 12.0, uu[v], fma(5.0 / 12.0, up[v], (-1.0 / 12.0) * um[v]));
             }
-            if (DSTORE) store_stage_derivative<nn>(a, 4, e, node, d);
-            // raw4 = f(upp) - 4 f(up) + 6 f0 - 4 f(um) + f(umm)
-            const Recip4 rc = TLW_VOL_ILP ? recip4(upp, up, um, umm) : Recip4{0.0, 0.0, 0.0, 0.0};
-            flux(upp, rc.pp, f, g);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) { r[v] = fma(6.0, f0[v], f[v]); q[v] = fma(6.0, g0[v], g[v]); }
-            flux(up, rc.p, f, g);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) { r[v] = fma(-4.0, f[v], r[v]); q[v] = fma(-4.0, g[v], q[v]); }
-            flux(um, rc.m, f, g);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) { r[v] = fma(-4.0, f[v], r[v]); q[v] = fma(-4.0, g[v], q[v]); }
-            flux(umm, rc.mm, f, g);
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                r[v] += f[v];
-                q[v] += g[v];
-                F[v] = fma(C4 / 120.0, r[v], F[v]);
-                if (TE) { dF[v] = (C4 / 120.0) * r[v]; dG[v] = (C4 / 120.0) * q[v]; }
-                G[v] = fma(C4 / 120.0, q[v], G[v]);
-            }
+            U[3] *= a.inv_gamma;
+            // the flux of rho is rho v1 (rho v2): its time average is U's, up to the stencil's factor C4 of f_tttt
+            constexpr double WU = DEPTH == 4 ? (C4 - 1.0) / 120.0 : 0.0;
+            F[0] = fma(WU, d[1], U[1]);
+            G[0] = fma(WU, d[2], U[2]);
+            G[1] = F[2];
         }
-    }
+    };
+    stage(std::integral_constant<int, 1>{});
+    if constexpr (DEPTH >= 2) stage(std::integral_constant<int, 2>{});
+    if constexpr (DEPTH >= 3) stage(std::integral_constant<int, 3>{});
+    if constexpr (DEPTH >= 4) stage(std::integral_constant<int, 4>{});
     // final: Dhat contraction of the time-averaged fluxes (every owner has read its node's results of
     // the last contraction before writing F, G over them: same address, same thread)
     if (SRC && active) {
@@ -1093,7 +1085,8 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
             if (a.tG) physical_flux_traces<n>(a, e, i, j, F, G);
             // the surface needs the normal fluxes: keep the contravariant time averages F~, G~ (their face
             // values are F . Ja^1 and F . Ja^2)
-            double ft[NV], gt[NV];
+            double ft[NV], gt[NV], Ja[4];
+            load4w(a.metrics + ((size_t)e * nn + node) * 4, Ja);
             contravariant(Ja, F, G, ft, gt);
 #pragma unroll
             for (int v = 0; v < NV; ++v) { F[v] = ft[v]; G[v] = gt[v]; }
@@ -1103,15 +1096,16 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
                 for (int v = 0; v < NV; ++v) { dF[v] = ft[v]; dG[v] = gt[v]; }
             }
         }
-        node_put<N, C>(X, Y, el, i, j, F, G);
+        store_traces<n>(a, e, i, j, U, F, G);
+        line_put<N, C>(X, Y, el, i, j, F, G);
         if (SC) {
             if constexpr (CURVED) sc_faces_curved<N, C, REC>(a, UU, VC, F0X, F0Y, UF, FVX, FVY, el, e, i, j, blended, muscl);
             else sc_faces<N, C>(UU, VC, F0X, F0Y, FVX, FVY, el, i, j, a.speed_kind);
         }
     }
-    __syncthreads();
+    phase_sync<C>();
     line_contract<N, C, true>(X, Y, tid);
-    __syncthreads();
+    phase_sync<C>();
     double l1 = 0.0, l2 = 0.0;
     if (active) {
         double acc[NV], o[NV];
@@ -1120,7 +1114,8 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
             if constexpr (CURVED) sc_blend_curved<N, C>(a, FVX, FVY, el, e, i, j, alpha_e, blended, acc);
             else sc_blend<N, C>(a, FVX, FVY, el, e, i, j, __ldg(a.alpha + e), acc);
         }
-        volume_epilogue<n, MODE>(a, e, i, j, node, ij, dt, acc, U, F, G, o, SRC ? Ssrc : nullptr);
+        store_result<MODE>(a.out + ((size_t)e * nn + node) * NV, MODE == MODE_STEP ? s0 : -inverse_jacobian(), dt, acc, ub,
+                           SRC ? Ssrc : nullptr, o);
         if (SLOTS && a.cfl_slots && i > 0 && i < n - 1 && j > 0 && j < n - 1) node_speeds(a.gamma, o, a.status, l1, l2);
     }
     if (SLOTS && a.cfl_slots) write_interior_slots<N, C>(a, X, active, el, i, j, tid, l1, l2);
@@ -1130,22 +1125,22 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
         // updates u_np1 = u - dt J^{-1} (D F + D G) and u_np1_low with F, G before the last stage's term;
         // temporal_errors[e] = sum over nodes and variables of ((u_np1 - u_np1_low) / (abstol + reltol max))^2
         double un[NV], err = 0.0;
-        __syncthreads();
-        if (active) node_put<N, C>(X, Y, el, i, j, F, G);
-        __syncthreads();
+        phase_sync<C>();
+        if (active) line_put<N, C>(X, Y, el, i, j, F, G);
+        phase_sync<C>();
         line_contract<N, C, false>(X, Y, tid);
-        __syncthreads();
+        phase_sync<C>();
         if (active) {
             double dd[NV];
             node_sum<N, C>(X, Y, el, i, j, dd);
 #pragma unroll
-            for (int v = 0; v < NV; ++v) un[v] = fma(s0, dd[v], u0[v]);
+            for (int v = 0; v < NV; ++v) un[v] = fma(s0, dd[v], ub[v]);
         }
-        __syncthreads();
-        if (active) node_put<N, C>(X, Y, el, i, j, dF, dG);
-        __syncthreads();
+        phase_sync<C>();
+        if (active) line_put<N, C>(X, Y, el, i, j, dF, dG);
+        phase_sync<C>();
         line_contract<N, C, false>(X, Y, tid);
-        __syncthreads();
+        phase_sync<C>();
         if (active) {
             double dd[NV];
             node_sum<N, C>(X, Y, el, i, j, dd);
@@ -1156,7 +1151,7 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
                 err = fma(r, r, err);
             }
         }
-        __syncthreads();
+        phase_sync<C>();
         if (active) X[el * C::P + i + C::R * j] = err;
         __syncthreads();
         const int ee = blockIdx.x * EB + tid;
@@ -1171,28 +1166,15 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
 
 // MDRK stage 1's stored sums from u^n and d = u_t: F2 = f + f_t/6, G2 = g + g_t/6, U2 = u + u_t/6 with f_t the
 // 4-point stencil at u +- d, u +- 2d (multi_derivative_2d.jl:337-371), the operations of mdrk1_volume_kernel
-__device__ __forceinline__ void mdrk_stage1_sums(double gm1, const double* uu, const double* d, double* F2v,
+__device__ __forceinline__ void mdrk_stage1_sums(const VolArgs& a, const double* uu, const double* d, double* F2v,
                                                  double* G2v, double* U2v) {
-    double f0[NV], g0[NV], f[NV], g[NV], ft[NV], gt[NV], s[NV];
-    euler_fluxes(gm1, uu[0], uu[1], uu[2], uu[3], f0, g0);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) s[v] = fma(2.0, d[v], uu[v]);
-    euler_fluxes(gm1, s[0], s[1], s[2], s[3], f, g);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) { ft[v] = -f[v]; gt[v] = -g[v]; s[v] = uu[v] + d[v]; }
-    euler_fluxes(gm1, s[0], s[1], s[2], s[3], f, g);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) { ft[v] = fma(8.0, f[v], ft[v]); gt[v] = fma(8.0, g[v], gt[v]); s[v] = uu[v] - d[v]; }
-    euler_fluxes(gm1, s[0], s[1], s[2], s[3], f, g);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) { ft[v] = fma(-8.0, f[v], ft[v]); gt[v] = fma(-8.0, g[v], gt[v]); s[v] = fma(-2.0, d[v], uu[v]); }
-    euler_fluxes(gm1, s[0], s[1], s[2], s[3], f, g);
+    double f0[NV], g0[NV], ft[NV], gt[NV];
+    flux_base(a.gm1, uu, f0, g0);
+    first_derivative_fluxes(a, uu, d, ft, gt);
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-        ft[v] = (ft[v] + f[v]) * (1.0 / 12.0);
-        gt[v] = (gt[v] + g[v]) * (1.0 / 12.0);
-        F2v[v] = fma(1.0 / 6.0, ft[v], f0[v]);
-        G2v[v] = fma(1.0 / 6.0, gt[v], g0[v]);
+        F2v[v] = fma(1.0 / 72.0, ft[v], f0[v]);
+        G2v[v] = fma(1.0 / 72.0, gt[v], g0[v]);
         U2v[v] = fma(1.0 / 6.0, d[v], uu[v]);
     }
 }
@@ -1227,7 +1209,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     double* FVY = FVX + C::PLANES;
     double* UF = FVY + C::PLANES;      // curvilinear MUSCL: face values, 4 regions (left, right, down, up)
     const int tid = threadIdx.x;
-    const double gm1 = a.gamma - 1.0;
+    prefetch_next<C>(a.u, 4, a.E, tid);
     const int el = tid / nn;
     const int node = tid - el * nn;
     const int i = node % n, j = node / n;
@@ -1248,20 +1230,20 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
         if (CURVED) {
             double ft[NV], gt[NV];
             contravariant(Ja, f, g, ft, gt);
-            node_put<N, C>(X, Y, el, i, j, ft, gt);
+            line_put<N, C>(X, Y, el, i, j, ft, gt);
         } else {
-            node_put<N, C>(X, Y, el, i, j, f, g);
+            line_put<N, C>(X, Y, el, i, j, f, g);
         }
     };
     if (active) {
-        load4(a.u + ((size_t)e * nn + node) * NV, uu);
+        load4w(a.u + ((size_t)e * nn + node) * NV, uu);
         if (CURVED) {
-            load4(a.metrics + ((size_t)e * nn + node) * 4, Ja);
+            load4w(a.metrics + ((size_t)e * nn + node) * 4, Ja);
             ij = __ldg(a.inv_jac_node + (size_t)e * nn + node);
         } else {
             ij = __ldg(a.inv_jac + e);
         }
-        euler_fluxes(gm1, uu[0], uu[1], uu[2], uu[3], f0, g0);
+        flux_base(a.gm1, uu, f0, g0);
         put(f0, g0);
         if (SC) {
             // the subcell FV part uses the instantaneous u^n (multi_derivative_2d.jl:205)
@@ -1269,14 +1251,14 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
             sc_park<N, C>(UU, VC, el, i, j, uu, a.gamma, a.status);
         }
     }
-    __syncthreads();
+    phase_sync<C>();
     // (the MUSCL face values are read by the neighbours after the next barrier)
-    if (SC && CURVED && REC >= 1 && muscl) sc_muscl_faces<N, C, REC>(a, UU, UF, el, e, i, j, gm1, alpha_e, 0.5 * dt, ij);
+    if (SC && CURVED && REC >= 1 && muscl) sc_muscl_faces<N, C, REC>(a, UU, UF, el, e, i, j, a.gm1, alpha_e, 0.5 * dt, ij);
     line_contract<N, C, false>(X, Y, tid);
-    __syncthreads();
+    phase_sync<C>();
     double U[NV], F[NV], G[NV], Ssrc[NV] = {0.0, 0.0, 0.0, 0.0};
     if (active) {
-        double d[NV], ft[NV], gt[NV], f[NV], g[NV], s[NV];
+        double d[NV], ft[NV], gt[NV];
         node_sum<N, C>(X, Y, el, i, j, d);
         const double s0 = -dt * ij;
 #pragma unroll
@@ -1290,37 +1272,24 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
 #pragma unroll
             for (int v = 0; v < NV; ++v) d[v] = fma(dt, sn[v], d[v]);
         }
-#pragma unroll
-        for (int v = 0; v < NV; ++v) s[v] = fma(2.0, d[v], uu[v]);
-        euler_fluxes(gm1, s[0], s[1], s[2], s[3], f, g);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) { ft[v] = -f[v]; gt[v] = -g[v]; s[v] = uu[v] + d[v]; }
-        euler_fluxes(gm1, s[0], s[1], s[2], s[3], f, g);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) { ft[v] = fma(8.0, f[v], ft[v]); gt[v] = fma(8.0, g[v], gt[v]); s[v] = uu[v] - d[v]; }
-        euler_fluxes(gm1, s[0], s[1], s[2], s[3], f, g);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) { ft[v] = fma(-8.0, f[v], ft[v]); gt[v] = fma(-8.0, g[v], gt[v]); s[v] = fma(-2.0, d[v], uu[v]); }
-        euler_fluxes(gm1, s[0], s[1], s[2], s[3], f, g);
+        first_derivative_fluxes(a, uu, d, ft, gt);
         double U2v[NV], F2v[NV], G2v[NV];
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
-            ft[v] = (ft[v] + f[v]) * (1.0 / 12.0);
-            gt[v] = (gt[v] + g[v]) * (1.0 / 12.0);
-            F[v] = fma(0.125, ft[v], 0.5 * f0[v]);
-            G[v] = fma(0.125, gt[v], 0.5 * g0[v]);
+            F[v] = fma(0.125 / 12.0, ft[v], 0.5 * f0[v]);
+            G[v] = fma(0.125 / 12.0, gt[v], 0.5 * g0[v]);
             U[v] = fma(0.125, d[v], 0.5 * uu[v]);
-            F2v[v] = fma(1.0 / 6.0, ft[v], f0[v]);
-            G2v[v] = fma(1.0 / 6.0, gt[v], g0[v]);
+            F2v[v] = fma(1.0 / 72.0, ft[v], f0[v]);
+            G2v[v] = fma(1.0 / 72.0, gt[v], g0[v]);
             U2v[v] = fma(1.0 / 6.0, d[v], uu[v]);
         }
         const size_t off = ((size_t)e * nn + node);
         if (COMPACT) {
-            store4(a.U2 + off * NV, d);
+            store4w(a.U2 + off * NV, d);
         } else {
-            store4(a.U2 + off * NV, U2v);
-            store4(a.F2 + off * 2 * NV, F2v);
-            store4(a.F2 + off * 2 * NV + NV, G2v);
+            store4w(a.U2 + off * NV, U2v);
+            store4w(a.F2 + off * 2 * NV, F2v);
+            store4w(a.F2 + off * 2 * NV + NV, G2v);
         }
         if (SRC) {
             double st[NV], S2v[NV];
@@ -1330,7 +1299,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
                 Ssrc[v] = fma(0.125, st[v], 0.5 * sn[v]);
                 S2v[v] = fma(1.0 / 6.0, st[v], sn[v]);
             }
-            store4(a.S2 + off * NV, S2v);
+            store4w(a.S2 + off * NV, S2v);
         }
         if (CURVED) {
             double ft2[NV], gt2[NV];
@@ -1338,15 +1307,16 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
 #pragma unroll
             for (int v = 0; v < NV; ++v) { F[v] = ft2[v]; G[v] = gt2[v]; }
         }
-        node_put<N, C>(X, Y, el, i, j, F, G);
+        store_traces<n>(a, e, i, j, U, F, G);
+        line_put<N, C>(X, Y, el, i, j, F, G);
         if (SC) {
             if constexpr (CURVED) sc_faces_curved<N, C, REC>(a, UU, VC, F0X, F0Y, UF, FVX, FVY, el, e, i, j, blended, muscl);
             else sc_faces<N, C>(UU, VC, F0X, F0Y, FVX, FVY, el, i, j, a.speed_kind);
         }
     }
-    __syncthreads();
+    phase_sync<C>();
     line_contract<N, C, true>(X, Y, tid);
-    __syncthreads();
+    phase_sync<C>();
     if (active) {
         double acc[NV];
         node_sum<N, C>(X, Y, el, i, j, acc);
@@ -1354,8 +1324,10 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
             if constexpr (CURVED) sc_blend_curved<N, C>(a, FVX, FVY, el, e, i, j, alpha_e, blended, acc);
             else sc_blend<N, C>(a, FVX, FVY, el, e, i, j, __ldg(a.alpha + e), acc);
         }
-        double o[NV];
-        volume_epilogue<n, MODE>(a, e, i, j, node, ij, dt, acc, U, F, G, o, SRC ? Ssrc : nullptr);
+        double o[NV], ub[NV];
+        if (MODE == MODE_STEP) load4w(a.u_base + ((size_t)e * nn + node) * NV, ub);
+        store_result<MODE>(a.out + ((size_t)e * nn + node) * NV, MODE == MODE_STEP ? -dt * ij : -ij, dt, acc, ub,
+                           SRC ? Ssrc : nullptr, o);
     }
 }
 
@@ -1366,8 +1338,8 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
 // CURVED (mdrk_kernel_2!, src/solvers/dgsem_structured/multi_derivative_2d.jl:245-445): as in stage 1.
 // SRC (FR volume integral): u*_t += dt s(u*); S = S2 + s_t(u*)/3 (multi_derivative_2d.jl:484-550), the source at
 // t + dt/2 on the TreeMesh and at t on curvilinear meshes (dgsem_structured/multi_derivative_2d.jl:325-361).
-// COMPACT: F2, G2, U2 recomputed from u^n (a.u_base) and stage 1's u_t (a.U2) at the start, parked in shared memory
-// (three more planes) until the stage's own sums are formed.
+// COMPACT: F2, G2, U2 recomputed from u^n (a.u_base) and stage 1's u_t (a.U2) at the start, parked in the node's
+// shared-memory slots until the stage's own sums are formed.
 template <int N, int MODE, bool SC, bool CURVED = false, int REC = 0, bool SRC = false, bool COMPACT = false>
 static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? VolCfg<N>::SC_CURVED_MIN_BLOCKS
                                                                          : VolCfg<N>::MDRK_MIN_BLOCKS)
@@ -1388,7 +1360,11 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     double* FVY = FVX + C::PLANES;
     double* UF = FVY + C::PLANES;      // curvilinear MUSCL: face values, 4 regions (left, right, down, up)
     const int tid = threadIdx.x;
-    const double gm1 = a.gamma - 1.0;
+    prefetch_next<C>(a.u, 4, a.E, tid);
+    if (COMPACT) {
+        prefetch_next<C>(a.u_base, 4, a.E, tid);
+        prefetch_next<C>(a.U2, 4, a.E, tid);
+    }
     const int el = tid / nn;
     const int node = tid - el * nn;
     const int i = node % n, j = node / n;
@@ -1403,51 +1379,55 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     }
     // dt of this element's instance (batched form) or the single dt
     const double dt = a.inst ? a.dt[__ldg(a.inst + min(e, a.E - 1))] : *a.dt;
+    double* keep = smem_d + C::regions(SC, REC) + tid;   // COMPACT: the node's slots
+    constexpr int K = C::NODES;
     double us[NV], ij = 0.0, Ja[4] = {0.0, 0.0, 0.0, 0.0};
     if (active) {
         double f[NV], g[NV];
-        load4(a.u + ((size_t)e * nn + node) * NV, us);
+        load4w(a.u + ((size_t)e * nn + node) * NV, us);
         if (CURVED) {
-            load4(a.metrics + ((size_t)e * nn + node) * 4, Ja);
+            load4w(a.metrics + ((size_t)e * nn + node) * 4, Ja);
             ij = __ldg(a.inv_jac_node + (size_t)e * nn + node);
         } else {
             ij = __ldg(a.inv_jac + e);
         }
-        euler_fluxes(gm1, us[0], us[1], us[2], us[3], f, g);
+        euler_fluxes(a.gm1, us[0], us[1], us[2], us[3], f, g);
         if (CURVED) {
             double ft[NV], gt[NV];
             contravariant(Ja, f, g, ft, gt);
-            node_put<N, C>(X, Y, el, i, j, ft, gt);
+            line_put<N, C>(X, Y, el, i, j, ft, gt);
         } else {
-            node_put<N, C>(X, Y, el, i, j, f, g);
+            line_put<N, C>(X, Y, el, i, j, f, g);
         }
         if (COMPACT) {
-            // stage 1's F2, G2 (into the F0X, F0Y planes) and U2 (the UU plane) from u^n and u_t
+            // stage 1's U2, F2 and G2 from u^n and u_t (F2 and G2 of rho are U2 of rho v1, rho v2), in the node's slots
             double un[NV], dn[NV], F2v[NV], G2v[NV], U2v[NV];
             const size_t off = ((size_t)e * nn + node);
-            load4(a.u_base + off * NV, un);
-            load4(a.U2 + off * NV, dn);
-            mdrk_stage1_sums(gm1, un, dn, F2v, G2v, U2v);
-            node_put<N, C>(F0X, F0Y, el, i, j, F2v, G2v);
-            node_put<N, C>(UU, UU, el, i, j, U2v, U2v);
+            load4w(a.u_base + off * NV, un);
+            load4w(a.U2 + off * NV, dn);
+            mdrk_stage1_sums(a, un, dn, F2v, G2v, U2v);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) keep[v * K] = U2v[v];
+            keep[4 * K] = F2v[1]; keep[5 * K] = F2v[2]; keep[6 * K] = F2v[3];
+            keep[7 * K] = G2v[2]; keep[8 * K] = G2v[3];
         }
         if (SC) {
             // the subcell FV part uses the instantaneous u^n, not u* (multi_derivative_2d.jl:257)
             double un[NV], fn0[NV], gn0[NV];
-            load4(a.u_base + ((size_t)e * nn + node) * NV, un);
-            euler_fluxes(gm1, un[0], un[1], un[2], un[3], fn0, gn0);
+            load4w(a.u_base + ((size_t)e * nn + node) * NV, un);
+            euler_fluxes(a.gm1, un[0], un[1], un[2], un[3], fn0, gn0);
             node_put<N, C>(F0X, F0Y, el, i, j, fn0, gn0);
             sc_park<N, C>(UU, VC, el, i, j, un, a.gamma, a.status);
         }
     }
-    __syncthreads();
+    phase_sync<C>();
     // (the MUSCL face values are read by the neighbours after the next barrier)
-    if (SC && CURVED && REC >= 1 && muscl) sc_muscl_faces<N, C, REC>(a, UU, UF, el, e, i, j, gm1, alpha_e, dt, ij);
+    if (SC && CURVED && REC >= 1 && muscl) sc_muscl_faces<N, C, REC>(a, UU, UF, el, e, i, j, a.gm1, alpha_e, dt, ij);
     line_contract<N, C, false>(X, Y, tid);
-    __syncthreads();
+    phase_sync<C>();
     double U[NV], F[NV], G[NV], Ssrc[NV] = {0.0, 0.0, 0.0, 0.0};
     if (active) {
-        double d[NV], ft[NV], gt[NV], f[NV], g[NV], s[NV];
+        double d[NV], ft[NV], gt[NV];
         node_sum<N, C>(X, Y, el, i, j, d);
         const double s0 = -dt * ij;
 #pragma unroll
@@ -1462,38 +1442,27 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
 #pragma unroll
             for (int v = 0; v < NV; ++v) d[v] = fma(dt, sn[v], d[v]);
             src_t_N34(sq, st);
-            load4(a.S2 + ((size_t)e * nn + node) * NV, sn);
+            load4w(a.S2 + ((size_t)e * nn + node) * NV, sn);
 #pragma unroll
             for (int v = 0; v < NV; ++v) Ssrc[v] = fma(1.0 / 3.0, st[v], sn[v]);
         }
-#pragma unroll
-        for (int v = 0; v < NV; ++v) s[v] = fma(2.0, d[v], us[v]);
-        euler_fluxes(gm1, s[0], s[1], s[2], s[3], f, g);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) { ft[v] = -f[v]; gt[v] = -g[v]; s[v] = us[v] + d[v]; }
-        euler_fluxes(gm1, s[0], s[1], s[2], s[3], f, g);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) { ft[v] = fma(8.0, f[v], ft[v]); gt[v] = fma(8.0, g[v], gt[v]); s[v] = us[v] - d[v]; }
-        euler_fluxes(gm1, s[0], s[1], s[2], s[3], f, g);
-#pragma unroll
-        for (int v = 0; v < NV; ++v) { ft[v] = fma(-8.0, f[v], ft[v]); gt[v] = fma(-8.0, g[v], gt[v]); s[v] = fma(-2.0, d[v], us[v]); }
-        euler_fluxes(gm1, s[0], s[1], s[2], s[3], f, g);
+        first_derivative_fluxes(a, us, d, ft, gt);
         const size_t off = ((size_t)e * nn + node);
         double U2v[NV], F2v[NV], G2v[NV];
         if (COMPACT) {
-            node_get<N, C>(F0X, F0Y, el, i, j, F2v, G2v);
-            node_get<N, C>(UU, UU, el, i, j, U2v, U2v);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) U2v[v] = keep[v * K];
+            F2v[0] = U2v[1]; F2v[1] = keep[4 * K]; F2v[2] = keep[5 * K]; F2v[3] = keep[6 * K];
+            G2v[0] = U2v[2]; G2v[1] = F2v[2]; G2v[2] = keep[7 * K]; G2v[3] = keep[8 * K];
         } else {
-            load4(a.U2 + off * NV, U2v);
-            load4(a.F2 + off * 2 * NV, F2v);
-            load4(a.F2 + off * 2 * NV + NV, G2v);
+            load4w(a.U2 + off * NV, U2v);
+            load4w(a.F2 + off * 2 * NV, F2v);
+            load4w(a.F2 + off * 2 * NV + NV, G2v);
         }
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
-            ft[v] = (ft[v] + f[v]) * (1.0 / 12.0);
-            gt[v] = (gt[v] + g[v]) * (1.0 / 12.0);
-            F[v] = fma(1.0 / 3.0, ft[v], F2v[v]);
-            G[v] = fma(1.0 / 3.0, gt[v], G2v[v]);
+            F[v] = fma(1.0 / 36.0, ft[v], F2v[v]);
+            G[v] = fma(1.0 / 36.0, gt[v], G2v[v]);
             U[v] = fma(1.0 / 3.0, d[v], U2v[v]);
         }
         if (CURVED) {
@@ -1502,15 +1471,16 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
 #pragma unroll
             for (int v = 0; v < NV; ++v) { F[v] = ft2[v]; G[v] = gt2[v]; }
         }
-        node_put<N, C>(X, Y, el, i, j, F, G);
+        store_traces<n>(a, e, i, j, U, F, G);
+        line_put<N, C>(X, Y, el, i, j, F, G);
         if (SC) {
             if constexpr (CURVED) sc_faces_curved<N, C, REC>(a, UU, VC, F0X, F0Y, UF, FVX, FVY, el, e, i, j, blended, muscl);
             else sc_faces<N, C>(UU, VC, F0X, F0Y, FVX, FVY, el, i, j, a.speed_kind);
         }
     }
-    __syncthreads();
+    phase_sync<C>();
     line_contract<N, C, true>(X, Y, tid);
-    __syncthreads();
+    phase_sync<C>();
     // the step's final values: per-element CFL slots as the LW kernel writes them (plain TreeMesh MDRK step)
     constexpr bool SLOTS = MODE == MODE_STEP && !SC && !CURVED;
     double l1 = 0.0, l2 = 0.0;
@@ -1521,8 +1491,10 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
             if constexpr (CURVED) sc_blend_curved<N, C>(a, FVX, FVY, el, e, i, j, alpha_e, blended, acc);
             else sc_blend<N, C>(a, FVX, FVY, el, e, i, j, __ldg(a.alpha + e), acc);
         }
-        double o[NV];
-        volume_epilogue<n, MODE>(a, e, i, j, node, ij, dt, acc, U, F, G, o, SRC ? Ssrc : nullptr);
+        double o[NV], ub[NV];
+        if (MODE == MODE_STEP) load4w(a.u_base + ((size_t)e * nn + node) * NV, ub);
+        store_result<MODE>(a.out + ((size_t)e * nn + node) * NV, MODE == MODE_STEP ? -dt * ij : -ij, dt, acc, ub,
+                           SRC ? Ssrc : nullptr, o);
         if (SLOTS && a.cfl_slots && i > 0 && i < n - 1 && j > 0 && j < n - 1) node_speeds(a.gamma, o, a.status, l1, l2);
     }
     if (SLOTS && a.cfl_slots) write_interior_slots<N, C>(a, X, active, el, i, j, tid, l1, l2);
