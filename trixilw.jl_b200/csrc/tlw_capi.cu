@@ -156,8 +156,8 @@ template <int N> struct CSpd {
 };
 template <int N> struct Spd {
     static void run(cudaStream_t s, const double* u, const double* ij, int E, double g, StepState* st, bool speed,
-                    bool ind, const IndicatorArgs& ia) {
-        Launch<N>::max_speed(s, u, ij, E, g, st, speed, ind, ia);
+                    bool ind, const IndicatorArgs& ia, unsigned long long* target = nullptr) {
+        Launch<N>::max_speed(s, u, ij, E, g, st, speed, ind, ia, target);
     }
 };
 
@@ -203,7 +203,8 @@ void enqueue_indicator(tlw_handle* h, const double* u, bool speed) {
 }
 
 // the step's final values all come from the volume and interface kernels: the plain LW step on a periodic
-// conforming TreeMesh (no boundaries, mortars, shock capturing, curvilinear or parabolic terms)
+// conforming TreeMesh (no boundaries, mortars, shock capturing, curvilinear or parabolic terms). With the limiter the
+// per-element CFL slots keep the maxima (the limiter rewrites those of the elements it changes).
 bool use_slots(const tlw_handle* h) {
     return h->d_slots && !h->sc && !h->curved && !h->parabolic && h->nb == 0 && h->nmx + h->nmy == 0 && h->nh == 0;
 }
@@ -223,6 +224,22 @@ bool use_slots(const tlw_handle* h) {
 bool use_surface_pass(const tlw_handle* h) {
     return TLW_SURFACE_PASS && h->d_nbr && !h->curved && (!h->sc || TLW_SURFACE_PASS_SC) && h->nmx + h->nmy == 0 &&
            h->nh == 0;
+}
+
+// the partial CFL maxima of the state in buffer k
+unsigned long long* ring_slot(tlw_handle* h, int k) { return h->d_ring + (size_t)k * RING_WAYS * RING_STRIDE; }
+
+// a step that keeps its own CFL maximum: its surface pass reduces the new state's into ring_slot, and the next
+// step's first kernel takes dt from there (begin_step). Not with the limiter, which changes the state afterwards.
+bool fused_cfl(const tlw_handle* h) {
+    return h->d_slots && use_surface_pass(h) && !h->sc && !h->parabolic && h->lim_count == 0;
+}
+
+// Whether the volume kernel of a fused step forms dt itself: it costs each CTA about 1 % (512^2: N = 3 0.195 -> 0.200,
+// N = 4 0.430 -> 0.434, N = 5 0.699 -> 0.707 ms), a dt launch about 3 us, so up to 16 resident sets of CTAs (148 SMs x 5
+// CTAs of about 128 nodes). Not with source terms, whose kernels are not built that way.
+bool begin_in_volume(const tlw_handle* h) {
+    return !h->source && (int64_t)h->E * h->nn <= (int64_t)16 * 148 * 5 * 128;
 }
 
 // the halo faces of one class (cls 0: x, 1: y) as kernel arguments
@@ -420,7 +437,7 @@ BndArgs boundary_args(tlw_handle* h, int stage, int mode, const double* u_jump, 
 // 7: all of it. The split step runs 1 | 2 before the exchange and 4 after it.
 void enqueue_rhs(tlw_handle* h, int stage, int mode, const double* u_flux, const double* u_jump, const double* u_base,
                  double* out, const double* dt_ptr, const PhaseEvents* ev = nullptr, bool alpha_ready = false,
-                 int phases = 7) {
+                 int phases = 7, bool fused = false, int ring = 0) {
     if (h->sc && !alpha_ready) enqueue_indicator(h, u_jump, false);   // indicator of the instantaneous u
     if (h->parabolic) {
         // BR1 gradients, parabolic LW volume kernel, then the interfaces with the viscous traces
@@ -486,14 +503,22 @@ void enqueue_rhs(tlw_handle* h, int stage, int mode, const double* u_flux, const
     va.status = &h->d_step->status;
     va.speed_kind = h->opts.max_speed;
     // the stage that produces the step's final values (LW, or MDRK stage 2) fills the next step's CFL slots
-    if (mode == MODE_STEP && stage != TLW_STAGE_MDRK1 && use_slots(h) && !h->te_request) va.cfl_slots = h->d_slots;
+    va.cfl_stride = fused ? 2 : CFL_SLOTS;
+    if (mode == MODE_STEP && stage != TLW_STAGE_MDRK1 && (fused || (use_slots(h) && !fused_cfl(h))) && !h->te_request)
+        va.cfl_slots = h->d_slots;
+    if (fused && stage != TLW_STAGE_MDRK2 && begin_in_volume(h)) {
+        va.step = h->d_step;
+        va.ring = ring_slot(h, ring);
+        va.ring_next = ring_slot(h, 1 - ring);
+    }
     // an MDRK step on a plain TreeMesh passes only u_t between its stages (stage 2 rebuilds U2 and F2)
     va.compact = TLW_MDRK_COMPACT && mode == MODE_STEP && stage != TLW_STAGE_LW && !h->sc && !h->curved &&
                  !h->source && !h->parabolic;
     if (h->source) {
         va.source = h->source;
         va.xnode = h->d_xnode;
-        va.tnow = dt_ptr == &h->d_step->dt_call ? &h->d_step->t_call : &h->d_step->t_step;
+        // (a fused step moves t on at its end, and its first kernel writes t_step)
+        va.tnow = dt_ptr == &h->d_step->dt_call ? &h->d_step->t_call : fused ? &h->d_step->t : &h->d_step->t_step;
         va.S2 = h->d_S2;
     }
     if (h->te_request) {
@@ -548,7 +573,13 @@ void enqueue_rhs(tlw_handle* h, int stage, int mode, const double* u_flux, const
     sa.jac_first = h->jac_first;
     sa.w_first = h->h_basis.weights[0];
     sa.w_last = h->h_basis.weights[h->n - 1];
-    sa.cfl_slots = va.cfl_slots;
+    if (!fused) {
+        sa.cfl_slots = va.cfl_slots;
+    } else if (stage != TLW_STAGE_MDRK1) {
+        sa.cfl_interior = (const double*)h->d_slots;
+        sa.cfl_max = ring_slot(h, 1 - ring);
+        sa.advance = h->d_step;
+    }
 
     BndArgs ba = boundary_args(h, stage, mode, u_jump, out, dt_ptr);
 
@@ -611,7 +642,14 @@ void enqueue_rhs(tlw_handle* h, int stage, int mode, const double* u_flux, const
 void enqueue_step(tlw_handle* h, int from, cudaEvent_t after_dt = nullptr, const PhaseEvents* ev = nullptr) {
     const double* u = h->d_state[from];
     double* unew = h->d_state[1 - from];
-    if (use_slots(h) && h->slots_valid) {
+    const bool fused = fused_cfl(h);
+    if (fused) {
+        if (!h->slots_valid) {   // the first step of a state: its CFL maximum by a pass over it
+            cudaMemsetAsync(ring_slot(h, from), 0, RING_WAYS * RING_STRIDE * sizeof(unsigned long long), h->stream);
+            dispatch<Spd>(h->N, h->stream, u, (const double*)h->d_inv_jac, (int)h->E, h->opts.gamma, h->d_step, true, false,
+                          indicator_args(h), ring_slot(h, from));
+        }
+    } else if (use_slots(h) && h->slots_valid) {
         // the previous step left the per-element maxima of this state
         const int grid = std::min<int>((int)((h->E + 255) / 256), 4 * 148);
         cfl_slots_reduce_kernel<<<grid, 256, 0, h->stream>>>(h->d_slots, h->d_inv_jac, (int)h->E, h->d_step);
@@ -621,17 +659,20 @@ void enqueue_step(tlw_handle* h, int from, cudaEvent_t after_dt = nullptr, const
                                        h->opts.gamma, h->d_step);
     else dispatch<Spd>(h->N, h->stream, u, (const double*)h->d_inv_jac, (int)h->E, h->opts.gamma, h->d_step, true,
                        false, indicator_args(h));
-    if (h->parabolic) par_finalize_dt_kernel<<<1, 1, 0, h->stream>>>(h->d_step, h->d_visc, h->N, h->curved ? 1 : 0);
+    if (fused) {
+        if (!begin_in_volume(h))
+            begin_step_kernel<<<1, 1, 0, h->stream>>>(h->d_step, ring_slot(h, from), ring_slot(h, 1 - from), h->n);
+    } else if (h->parabolic) par_finalize_dt_kernel<<<1, 1, 0, h->stream>>>(h->d_step, h->d_visc, h->N, h->curved ? 1 : 0);
     else finalize_dt_kernel<<<1, 1, 0, h->stream>>>(h->d_step, h->n);
     if (after_dt) cudaEventRecord(after_dt, h->stream);
     const double* dtp = &h->d_step->dt;
     if (h->opts.time_discretization == TLW_LW) {
-        enqueue_rhs(h, TLW_STAGE_LW, MODE_STEP, u, u, u, unew, dtp, ev, true);
+        enqueue_rhs(h, TLW_STAGE_LW, MODE_STEP, u, u, u, unew, dtp, ev, true, 7, fused, from);
         // solve_lwfr limits twice per LW step: in perform_step! (src/solvers/lwfr.jl:226) and in its loop (:257)
         enqueue_limiter(h, unew, 2, use_slots(h) ? h->d_slots : nullptr);
     } else {
-        enqueue_rhs(h, TLW_STAGE_MDRK1, MODE_STEP, u, u, u, h->d_us, dtp, ev, true);
-        enqueue_rhs(h, TLW_STAGE_MDRK2, MODE_STEP, h->d_us, u, u, unew, dtp, ev ? ev + 1 : nullptr, true);
+        enqueue_rhs(h, TLW_STAGE_MDRK1, MODE_STEP, u, u, u, h->d_us, dtp, ev, true, 7, fused, from);
+        enqueue_rhs(h, TLW_STAGE_MDRK2, MODE_STEP, h->d_us, u, u, unew, dtp, ev ? ev + 1 : nullptr, true, 7, fused, from);
         // once per MDRK step (the loop); perform_step!'s mid-step call (src/solvers/mdrk.jl:19) acts on u^n,
         // which the previous step's application has limited already
         enqueue_limiter(h, unew, 1, use_slots(h) ? h->d_slots : nullptr);
@@ -723,6 +764,11 @@ int tlw_create(const tlw_opts* opts, tlw_handle** out) {
         if (cudaMalloc(&h->d_basis, sizeof(tlw::Basis)) != cudaSuccess) { rc = fail(h, TLW_E_CUDA, "alloc basis"); break; }
         if (upload_on(h->stream, h->d_basis, &h->h_basis, sizeof(tlw::Basis)) != cudaSuccess) { rc = fail(h, TLW_E_CUDA, "copy basis"); break; }
         if (cudaMalloc(&h->d_step, sizeof(StepState)) != cudaSuccess) { rc = fail(h, TLW_E_CUDA, "alloc step"); break; }
+        const size_t ring_bytes = 2 * RING_WAYS * RING_STRIDE * sizeof(unsigned long long);
+        if (cudaMalloc(&h->d_ring, ring_bytes) != cudaSuccess || zero_on(h->stream, h->d_ring, ring_bytes) != cudaSuccess) {
+            rc = fail(h, TLW_E_CUDA, "alloc ring");
+            break;
+        }
         StepState st{};
         st.cfl = 1.0;
         st.t_end = INFINITY;
@@ -753,6 +799,7 @@ int tlw_destroy(tlw_handle* h) {
     free_mesh(h);
     dfree(h->d_basis);
     dfree(h->d_step);
+    dfree(h->d_ring);
     if (h->s_comm) cudaStreamSynchronize(h->s_comm);
     for (cudaEvent_t ev : {h->ev_up, h->ev_computed, h->ev_prior, h->ev_lib, h->ev_comm})
         if (ev) cudaEventDestroy(ev);
@@ -1591,6 +1638,7 @@ int tlw_set_positivity_limiter(tlw_handle* h, int32_t count, const double* thres
     }
     drop_graphs(h);
     h->lim_count = count;
+    h->slots_valid = false;   // the steps keep their CFL maximum another way with and without the limiter
     for (int p = 0; p < count; ++p) { h->lim_thr[p] = thresholds[p]; h->lim_var[p] = variables[p]; }
     return TLW_OK;
 }
@@ -2018,8 +2066,8 @@ int tlw_step(tlw_handle* h, int32_t nsteps, double cfl, double fixed_dt, double 
     // parameters into the device step state (cfl, fixed_dt, t_end are contiguous after t)
     double params[3] = {t_end, cfl, fixed_dt};
     TLW_CUDA(h, cudaMemcpyAsync(&h->d_step->t_end, params, sizeof(params), cudaMemcpyHostToDevice, h->stream));
-    if (use_slots(h) && !h->slots_valid) {
-        // one step with the full CFL pass; it leaves the per-element slots that later steps reduce
+    if ((use_slots(h) || fused_cfl(h)) && !h->slots_valid) {
+        // one step with the full CFL pass; it leaves the maxima that later steps reduce
         enqueue_step(h, h->cur);
         h->cur ^= 1;
         h->slots_valid = true;
@@ -2092,7 +2140,7 @@ int tlw_step_timed(tlw_handle* h, int32_t nsteps, double cfl, double fixed_dt, d
         cudaEventRecord(e_start, h->stream);
         enqueue_step(h, h->cur, e_dt, pe);
         h->cur ^= 1;
-        if (use_slots(h)) h->slots_valid = true;
+        if (use_slots(h) || fused_cfl(h)) h->slots_valid = true;
     }
     TLW_CUDA(h, cudaGetLastError());
     TLW_CUDA(h, cudaStreamSynchronize(h->stream));

@@ -153,6 +153,64 @@ __device__ __forceinline__ void node_speeds(double gamma, const double* x, unsig
 // with corners (y interfaces). The next step reduces them instead of reading the whole state again.
 constexpr int CFL_SLOTS = 10;
 
+struct StepState {
+    unsigned long long max_bits;   // bits of max_e J^{-1}(lambda1 + lambda2) (non-negative doubles order as ints)
+    double dt;                     // time step used by the current step
+    double t;                      // time at the start of the next step
+    double t_end;
+    double cfl;
+    double fixed_dt;               // > 0: use this dt instead of the CFL estimate
+    long long steps;               // accepted steps
+    unsigned status;               // STATUS_* bits
+    int pad;
+    double dt_call;                // dt for the rhs entry points (set from the host)
+    double t_step;                 // time at the start of the current step (source terms)
+    double t_call;                 // t of the rhs entry points (set from the host; source terms)
+};
+// A step that keeps its own CFL maximum: bits of the maximum over the elements of the state in state buffer k, at
+// [k][RING_WAYS][RING_STRIDE]: partial maxima on lines of their own, so that the warps' atomics spread.
+constexpr int RING_WAYS = 8, RING_STRIDE = 16;
+
+// isfinished: t ≈ t_end (src/solvers/lwfr.jl:146-148) with Julia's isapprox (rtol = sqrt(eps(Float64)),
+// never true against an infinite t_end unless equal); t >= t_end cannot happen after the set_dt! clamp and
+// only guards against an endless run.
+__device__ __forceinline__ bool run_finished(double t, double te) {
+    if (t == te) return true;
+    if (!isfinite(t) || !isfinite(te)) return false;
+    return fabs(t - te) <= 1.4901161193847656e-8 * fmax(fabs(t), fabs(te)) || t >= te;
+}
+
+// The time step of a state whose scaled maximum speed has the bits `bits`: cfl * 2 / (n * max), or the fixed dt,
+// clamped so that t + dt <= t_end (set_dt!, src/solvers/lwfr.jl:76-90); 0 for a finished run, whose remaining steps
+// are then exact no-ops on the state.
+__device__ __forceinline__ double step_size(const StepState* s, unsigned long long bits, int n, bool& finished) {
+    double maxs = __longlong_as_double((long long)bits);
+    const double tiny = 4.9406564584124654e-324;   // nextfloat(0.0)
+    if (!(maxs > tiny)) maxs = tiny;
+    const double t = s->t, te = s->t_end;
+    finished = run_finished(t, te);
+    const double dt = s->fixed_dt > 0.0 ? s->fixed_dt : s->cfl * (2.0 / (n * maxs));
+    return finished ? 0.0 : t + dt > te ? te - t : dt;
+}
+
+// dt of a step that keeps its own CFL maximum, from the partial maxima at ring; `write`: into the step state, with the
+// partial maxima at ring_next cleared for this step's surface pass (which moves t on at the end)
+__device__ __forceinline__ double begin_step_dt(StepState* s, const unsigned long long* ring, unsigned long long* ring_next,
+                                                int n, bool write) {
+    unsigned long long bits = 0ull;
+#pragma unroll
+    for (int k = 0; k < RING_WAYS; ++k) bits = max(bits, __ldg(ring + k * RING_STRIDE));
+    bool finished;
+    const double dt = step_size(s, bits, n, finished);
+    if (write) {
+        s->dt = dt;
+        s->t_step = s->t;
+#pragma unroll
+        for (int k = 0; k < RING_WAYS; ++k) ring_next[k * RING_STRIDE] = 0ull;
+    }
+    return dt;
+}
+
 // Trixi max_abs_speed_naive (kind 0) / max_abs_speed (kind 1) for CompressibleEulerEquations2D
 __device__ __forceinline__ double max_abs_speed(double gamma, const double* ul, const double* ur, int orientation,
                                                 int kind, unsigned* status) {

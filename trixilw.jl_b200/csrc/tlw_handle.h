@@ -127,6 +127,7 @@ struct tlw_handle {
     // per-element CFL slots of the state in d_state[cur] (plain LW step on a periodic conforming TreeMesh)
     unsigned long long* d_slots = nullptr;
     bool slots_valid = false;
+    unsigned long long* d_ring = nullptr;   // [state buffer][RING_WAYS][RING_STRIDE] partial CFL maxima of fused steps
     // compressible Navier-Stokes (TreeMesh, periodic, LW): BR1 gradients, viscous traces, viscous dt bound
     bool parabolic = false;
     double ns_mu = 0.0, ns_Pr = 0.72;

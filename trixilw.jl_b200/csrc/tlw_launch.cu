@@ -45,6 +45,10 @@ struct LaunchImpl {
         cudaFuncSetAttribute(mdrk1_volume_kernel<N, MODE_STEP, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, md);
         cudaFuncSetAttribute(mdrk2_volume_kernel<N, MODE_RHS, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, md);
         cudaFuncSetAttribute(mdrk2_volume_kernel<N, MODE_STEP, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, md);
+        cudaFuncSetAttribute(lw_volume_kernel<N, MODE_STEP, false, 0, false, false, false, 0, false, true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, lw);
+        cudaFuncSetAttribute(mdrk1_volume_kernel<N, MODE_STEP, false, false, 0, false, true, true>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, md);
         cudaFuncSetAttribute(mdrk2_volume_kernel<N, MODE_STEP, false, false, 0, false, true>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::mdrk_bytes(false, 0, true));
         // source terms (FR)
@@ -89,9 +93,12 @@ struct LaunchImpl {
         const size_t lw = C::lw_bytes(SC), md = C::mdrk_bytes(SC);
         if (stage == TLW_STAGE_LW) {
             if (mode == MODE_RHS) lw_volume_kernel<N, MODE_RHS, SC><<<grid, C::THREADS, lw, s>>>(a);
+            else if (!SC && a.step) lw_volume_kernel<N, MODE_STEP, false, 0, false, false, false, 0, false, true><<<grid, C::THREADS, lw, s>>>(a);
             else lw_volume_kernel<N, MODE_STEP, SC><<<grid, C::THREADS, lw, s>>>(a);
         } else if (stage == TLW_STAGE_MDRK1) {
             if (mode == MODE_RHS) mdrk1_volume_kernel<N, MODE_RHS, SC><<<grid, C::THREADS, md, s>>>(a);
+            else if (!SC && a.compact && a.step)
+                mdrk1_volume_kernel<N, MODE_STEP, false, false, 0, false, true, true><<<grid, C::THREADS, md, s>>>(a);
             else if (!SC && a.compact) mdrk1_volume_kernel<N, MODE_STEP, false, false, 0, false, true><<<grid, C::THREADS, md, s>>>(a);
             else mdrk1_volume_kernel<N, MODE_STEP, SC><<<grid, C::THREADS, md, s>>>(a);
         } else {
@@ -385,8 +392,10 @@ template <int N> void Launch<N>::halo(cudaStream_t s, const HaloArgs& a, bool pa
 template <int N> void Launch<N>::limiter(cudaStream_t s, const LimiterArgs& a) { LimImpl<N>::run(s, a); }
 template <int N>
 void Launch<N>::max_speed(cudaStream_t s, const double* u, const double* ij, int E, double gamma, StepState* st,
-                          bool speed, bool ind, const IndicatorArgs& ia) {
-    LaunchImpl<N>::max_speed(s, u, ij, E, gamma, st, speed, ind, ia);
+                          bool speed, bool ind, const IndicatorArgs& ia, unsigned long long* target) {
+    BatchSpeedArgs bs{};
+    bs.target = target;
+    LaunchImpl<N>::max_speed(s, u, ij, E, gamma, st, speed, ind, ia, bs);
 }
 
 #ifdef TLW_LAUNCH_N

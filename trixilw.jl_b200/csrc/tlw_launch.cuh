@@ -38,7 +38,7 @@ struct Launch {
     static void halo(cudaStream_t s, const HaloArgs& a, bool pack);
     static void limiter(cudaStream_t s, const LimiterArgs& a);
     static void max_speed(cudaStream_t s, const double* u, const double* ij, int E, double gamma, StepState* st,
-                          bool speed, bool ind, const IndicatorArgs& ia);
+                          bool speed, bool ind, const IndicatorArgs& ia, unsigned long long* target = nullptr);
 };
 
 }  // namespace tlw

@@ -47,6 +47,13 @@ struct SurfArgs {
     unsigned long long* cfl_slots;   // plain LW step: per-element CFL slots of the nodes finalised here
     const int* nbr;          // surface_kernel: the element across each face [4, e] (-x, +x, -y, +y)
     int E;                   // surface_kernel: number of elements
+    // surface_kernel of a step that keeps its own CFL maximum (null otherwise): the elements' interior maxima
+    // [e][2] the volume kernel left, and where the partial maxima of J^{-1} (l1 + l2) over the elements go (the batched
+    // form keeps its pass over the states: 64 instances, 50 steps 16.3 ms with the maxima kept here, 16.1 with the pass);
+    // advance: the step state whose t and step count this launch, the step's last, moves on
+    const double* cfl_interior;
+    unsigned long long* cfl_max;
+    StepState* advance;
 };
 
 __device__ __forceinline__ bool admissible(double gm1, const double* u) {
@@ -374,12 +381,15 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, (BND || SC) ? TLW_
         }
     }
     __syncthreads();
-    double l1 = 0.0, l2 = 0.0;
+    double l1 = 0.0, l2 = 0.0, ij = 0.0;
+    double2 in = make_double2(0.0, 0.0);
     if (has2) {
         if (!TLW_SURF_PREFETCH) load4w_rw(o2, x);
+        // (with the face node, not where it is needed: the CTA's end would wait for it)
+        if (a.cfl_max && b == 0) in = __ldg(reinterpret_cast<const double2*>(a.cfl_interior) + e2);
         const double dt = a.inst ? a.dt[__ldg(a.inst + e2)] : *a.dt;
         const double dts = a.step_mode ? dt : 1.0;
-        const double ij = __ldg(a.inv_jac + e2);
+        ij = __ldg(a.inv_jac + e2);
         const double sMinus = ij * a.inv_w_first * dts;   // the element is the right (upper) one of the interface
         const double sPlus = -ij * a.inv_w_last * dts;    // the element is the left (lower) one
         const double* F = sF + el2 * 4 * n * NV;
@@ -396,18 +406,17 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, (BND || SC) ? TLW_
             for (int v = 0; v < NV; ++v) x[v] = fma(s, p[v], x[v]);
         }
         store4w(o2, x);
-        if (a.cfl_slots) node_speeds(a.gamma, x, a.status, l1, l2);
+        if (a.cfl_slots || a.cfl_max) node_speeds(a.gamma, x, a.status, l1, l2);
     }
-    if (a.cfl_slots && 32 % NB == 0) {
+    if (!a.cfl_slots && !a.cfl_max) return;
+    if constexpr (32 % NB == 0) {
         // the element's NB phase-2 threads are NB aligned consecutive lanes of one warp: reduce by shuffles
 #pragma unroll
         for (int o = NB / 2; o > 0; o >>= 1) {
             l1 = fmax(l1, __shfl_xor_sync(0xffffffffu, l1, o));
             l2 = fmax(l2, __shfl_xor_sync(0xffffffffu, l2, o));
         }
-        if (has2 && b < 2)
-            a.cfl_slots[(size_t)e2 * CFL_SLOTS + 2 + b] = (unsigned long long)__double_as_longlong(b ? l2 : l1);
-    } else if (a.cfl_slots) {
+    } else {
         // the element's face-node maxima through shared memory (NB consecutive threads per element)
         __syncthreads();
         if (has2) {
@@ -415,12 +424,36 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, (BND || SC) ? TLW_
             sF[EB * NB + tid] = l2;
         }
         __syncthreads();
+        double m = 0.0;
         if (has2 && b < 2) {
             const double* p = sF + b * EB * NB + el2 * NB;
-            double m = 0.0;
 #pragma unroll
             for (int k = 0; k < NB; ++k) m = fmax(m, p[k]);
-            a.cfl_slots[(size_t)e2 * CFL_SLOTS + 2 + b] = (unsigned long long)__double_as_longlong(m);
+        }
+        // threads 0 and 1 of an element are neighbouring lanes (NB is even): both get both maxima
+        const double other = __shfl_xor_sync(0xffffffffu, m, 1);
+        l1 = b == 0 ? m : other;
+        l2 = b == 0 ? other : m;
+    }
+    if (a.cfl_slots) {
+        if (has2 && b < 2)
+            a.cfl_slots[(size_t)e2 * CFL_SLOTS + 2 + b] = (unsigned long long)__double_as_longlong(b ? l2 : l1);
+        return;
+    }
+    // the element's scaled speed with the interior maxima; one atomic per warp
+    unsigned long long m = 0ull;
+    if (has2 && b == 0) m = (unsigned long long)__double_as_longlong(ij * (fmax(l1, in.x) + fmax(l2, in.y)));
+    // the largest of the warp's 64-bit words: the largest upper half, then the largest lower half below it
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(m >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(m >> 32) == hi ? (unsigned)m : 0u);
+    if ((tid & 31) == 0 && (hi | lo))
+        atomicMax(a.cfl_max + (blockIdx.x % RING_WAYS) * RING_STRIDE, (unsigned long long)hi << 32 | lo);
+    if (a.advance && blockIdx.x == 0 && tid == 0) {
+        StepState* s = a.advance;
+        const double t = s->t;
+        if (!run_finished(t, s->t_end)) {
+            s->t = t + s->dt;
+            s->steps += 1;
         }
     }
 }
@@ -429,21 +462,6 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, (BND || SC) ? TLW_
 // ------------------------------------------------------------------------------------------------
 // CFL time step on the device.
 // ------------------------------------------------------------------------------------------------
-struct StepState {
-    unsigned long long max_bits;   // bits of max_e J^{-1}(lambda1 + lambda2) (non-negative doubles order as ints)
-    double dt;                     // time step used by the current step
-    double t;                      // time at the start of the next step
-    double t_end;
-    double cfl;
-    double fixed_dt;               // > 0: use this dt instead of the CFL estimate
-    long long steps;               // accepted steps
-    unsigned status;               // STATUS_* bits
-    int pad;
-    double dt_call;                // dt for the rhs entry points (set from the host)
-    double t_step;                 // time at the start of the current step (source terms)
-    double t_call;                 // t of the rhs entry points (set from the host; source terms)
-};
-
 constexpr int MS_THREADS = 256;
 template <int N>
 struct MsCfg {
@@ -470,6 +488,7 @@ struct IndicatorArgs {
 struct BatchSpeedArgs {
     const int* inst;                // instance of each element, or null
     unsigned long long* inst_max;   // [instance] bits of the max scaled speed
+    unsigned long long* target;     // not batched: where the maximum goes instead of StepState::max_bits, or null
 };
 
 // CSPEED (curvilinear meshes): the speeds of curved_max_speed_kernel, |Ja^d . (l1, l2)| |J^{-1}| per node, and the
@@ -585,21 +604,12 @@ static __global__ void __launch_bounds__(MS_THREADS) max_speed_kernel(const doub
         if (threadIdx.x == 0) {
             double b = wmax[0];
             for (int w = 1; w < MS_THREADS / 32; ++w) b = fmax(b, wmax[w]);
-            if (b > 0.0) atomicMax(&s->max_bits, (unsigned long long)__double_as_longlong(b));
+            if (b > 0.0) atomicMax(bs.target ? bs.target : &s->max_bits, (unsigned long long)__double_as_longlong(b));
         }
     }
 }
 
 // batched form: dt of every instance from its max scaled speed (finalize_dt_kernel per instance)
-// isfinished: t ≈ t_end (src/solvers/lwfr.jl:146-148) with Julia's isapprox (rtol = sqrt(eps(Float64)),
-// never true against an infinite t_end unless equal); t >= t_end cannot happen after the set_dt! clamp and
-// only guards against an endless run.
-__device__ __forceinline__ bool run_finished(double t, double te) {
-    if (t == te) return true;
-    if (!isfinite(t) || !isfinite(te)) return false;
-    return fabs(t - te) <= 1.4901161193847656e-8 * fmax(fabs(t), fabs(te)) || t >= te;
-}
-
 struct BatchTime {
     unsigned long long* max_bits;
     double* dt;
@@ -640,22 +650,21 @@ static __global__ void alpha_smooth_kernel(const int* __restrict__ left, const i
     atomicMax(ab + r, (unsigned long long)__double_as_longlong(0.5 * __ldg(alpha_raw + l)));
 }
 
-// dt = cfl * 2 / (n * max_scaled_speed), clamped so that t + dt <= t_end; a finished run gets dt = 0
-// (the remaining launches of a captured step are then exact no-ops on the state).
+// dt of the step from the CFL maximum in max_bits, and the time after it
 static __global__ void finalize_dt_kernel(StepState* s, int n) {
-    double maxs = __longlong_as_double((long long)s->max_bits);
-    const double tiny = 4.9406564584124654e-324;   // nextfloat(0.0)
-    if (!(maxs > tiny)) maxs = tiny;
-    double dt = s->fixed_dt > 0.0 ? s->fixed_dt : s->cfl * (2.0 / (n * maxs));
-    const double t = s->t, te = s->t_end;
-    const bool finished = run_finished(t, te);
-    if (finished) dt = 0.0;
-    else if (t + dt > te) dt = te - t;
+    bool finished;
+    const double dt = step_size(s, s->max_bits, n, finished);
+    const double t = s->t;
     s->t_step = t;
     s->dt = dt;
     s->t = finished ? t : t + dt;
     if (!finished) s->steps += 1;
     s->max_bits = 0ull;
+}
+
+// dt of a step that keeps its own CFL maximum, where its first kernel does not form it
+static __global__ void begin_step_kernel(StepState* s, const unsigned long long* ring, unsigned long long* ring_next, int n) {
+    begin_step_dt(s, ring, ring_next, n, true);
 }
 
 // the next step's CFL maximum from the per-element slots: max_e J^{-1} (max_s l1 + max_s l2)

@@ -127,7 +127,12 @@ struct VolArgs {
     // inverse Jacobian per node [i, j, e] (inv_jac is then unused)
     const double* metrics;
     const double* inv_jac_node;
-    unsigned long long* cfl_slots;   // plain LW step on a periodic TreeMesh: per-element CFL slots (or null)
+    unsigned long long* cfl_slots;   // plain step on a TreeMesh: per-element CFL slots (or null)
+    int cfl_stride;                  // words per element there: CFL_SLOTS, or 2 (the interior maxima alone)
+    // BEGIN kernels (begin_step); null selects the others, whose dt is final
+    StepState* step;
+    const unsigned long long* ring;
+    unsigned long long* ring_next;
     // temporal error estimate of the Adaptive step control (lw_volume_kernel_4!'s u_np1 / u_np1_low tail)
     double* temporal_errors;          // [e]
     double abstol, reltol;
@@ -165,13 +170,20 @@ __device__ __forceinline__ void prefetch_next(const double* p, int K, int E, int
         asm volatile("prefetch.global.L2 [%0];" ::"l"(p + first));
 }
 
+// BEGIN kernels, the first of a step that keeps its own CFL maximum: dt by one thread of each CTA before the CTA's first
+// barrier, from the partial maxima at a.ring; block 0 leaves it in the step state and clears a.ring_next for this
+// step's surface pass. Its loads and division hide behind the other warps' loads of u, and the step needs no dt launch
+// (the rule that picks these kernels is begin_in_volume).
+template <class C>
+__device__ __forceinline__ void begin_step(const VolArgs& a, double* s_dt, int tid) {
+    if (tid == 0) *s_dt = begin_step_dt(a.step, a.ring, a.ring_next, C::n, blockIdx.x == 0);
+}
 // barrier between the node phase and the line phase of the same elements
 template <class C>
 __device__ __forceinline__ void phase_sync() {
     if constexpr (C::WARP_LOCAL) __syncwarp();
     else __syncthreads();
 }
-
 // owner: the node's f and g into the contraction planes X and Y
 template <int N, class C>
 __device__ __forceinline__ void line_put(double* X, double* Y, int e, int i, int j, const double* f, const double* g) {
@@ -759,10 +771,12 @@ __device__ __forceinline__ void write_interior_slots(const VolArgs& a, double* X
         for (int jj = 1; jj < n - 1; ++jj)
 #pragma unroll
             for (int ii = 1; ii < n - 1; ++ii) m = fmax(m, p[ii + C::R * jj]);
-        unsigned long long* sl = a.cfl_slots + (size_t)ee * CFL_SLOTS;
+        unsigned long long* sl = a.cfl_slots + (size_t)ee * a.cfl_stride;
         sl[tid & 1] = (unsigned long long)__double_as_longlong(m);
+        if (a.cfl_stride == CFL_SLOTS) {
 #pragma unroll
-        for (int k = 1; k < CFL_SLOTS / 2; ++k) sl[2 * k + (tid & 1)] = 0ull;
+            for (int k = 1; k < CFL_SLOTS / 2; ++k) sl[2 * k + (tid & 1)] = 0ull;
+        }
     }
 }
 
@@ -863,13 +877,14 @@ __device__ __forceinline__ void store_stage_derivative(const VolArgs& a, int m, 
 // kernel of depth 4 takes the 5-point s_tt (calc_source_tt_N4, dgsem_structured/dg_2d.jl:1886) where the TreeMesh
 // one takes the 3-point calc_source_tt_N23 (dgsem_tree/dg_2d.jl:1093-1104).
 template <int N, int MODE, bool SC, int EBX = 0, bool CURVED = false, bool TE = false, bool DSTORE = false, int REC = 0,
-          bool SRC = false>
+          bool SRC = false, bool BEGIN = false>
 static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED) ? VolCfg<N, EBX>::SC_CURVED_MIN_BLOCKS
                                                                   : SRC ? VolCfg<N, EBX>::MDRK_MIN_BLOCKS - 1
                                                                         : VolCfg<N, EBX>::MIN_BLOCKS)
     lw_volume_kernel(VolArgs a) {
     static_assert(REC == 0 || (SC && CURVED), "MUSCL subcells: curvilinear shock capturing");
     static_assert(!SRC || (!SC && !TE && !DSTORE), "source terms: the FR volume integral, without the error estimate");
+    static_assert(!BEGIN || (MODE == MODE_STEP && !SC && !CURVED && !TE && !DSTORE && !SRC), "dt in the kernel: the plain step");
     // the temporal error estimate of the Adaptive step control: the TreeMesh computes it at depth 4 only
     // (lw_volume_kernel_3! of dgsem_tree has none), the curvilinear kernels at depths 3 and 4
     static_assert(!TE || (CURVED ? N >= 3 : N >= 4), "temporal errors: TreeMesh N >= 4, curvilinear N >= 3");
@@ -912,8 +927,10 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
         blended = !(fabs(alpha_e) <= 1e-12);
         muscl = REC >= 1 && blended && !__ldg(a.atb + e);
     }
-    // dt of this element's instance (batched form) or the single dt
-    const double dt = a.inst ? a.dt[__ldg(a.inst + min(e, a.E - 1))] : *a.dt;
+    double dt = 0.0;
+    __shared__ double s_dt;
+    if constexpr (BEGIN) begin_step<C>(a, &s_dt, tid);
+    else dt = a.inst ? a.dt[__ldg(a.inst + min(e, a.E - 1))] : *a.dt;
     // per-element maxima of the interior nodes' speeds for the next step's CFL (plain LW step only)
     constexpr bool SLOTS = MODE == MODE_STEP && !SC && !CURVED;
 
@@ -947,7 +964,7 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
     if (active) {
         double uu[NV], f[NV], g[NV];
         load4w(a.u + ((size_t)e * nn + node) * NV, uu);
-        s0 = -dt * inverse_jacobian();
+        s0 = BEGIN ? -inverse_jacobian() : -dt * inverse_jacobian();   // (BEGIN: dt after the first barrier)
         if (SRC) {
             // S = s(u, x, t) (dg_2d.jl:979-987)
             const double* xn = a.xnode + 2 * ((size_t)e * nn + node);
@@ -974,7 +991,13 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
         constexpr double LM[5] = {0.0, DEPTH >= 3 ? 12.0 : 2.0, DEPTH == 4 ? 12.0 : 1.0, 2.0, 1.0};
         constexpr double SIGN = M % 2 ? -1.0 : 1.0;
         const double W1 = c_tlw_taylor[M], W2 = c_tlw_taylor[4 + M];
-        phase_sync<C>();
+        if (BEGIN && M == 1) {
+            __syncthreads();
+            dt = s_dt;
+            s0 *= dt;
+        } else {
+            phase_sync<C>();
+        }
         line_contract<N, C, false>(X, Y, tid);
         phase_sync<C>();
         if (M == 1 && SC && CURVED && REC >= 1 && muscl) sc_muscl_faces<N, C, REC>(a, UU, UF, el, e, i, j, a.gm1, alpha_e, dt, inverse_jacobian());
@@ -1189,10 +1212,12 @@ __device__ __forceinline__ void mdrk_stage1_sums(const VolArgs& a, const double*
 // (multi_derivative_2d.jl:321-400; dgsem_structured/multi_derivative_2d.jl:151-239).
 // COMPACT (the plain TreeMesh step): store only u_t (into a.U2) instead of U2 and F2; stage 2 recomputes them from
 // u^n and u_t with this kernel's operations (64 instead of 192 bytes a node between the stages).
-template <int N, int MODE, bool SC, bool CURVED = false, int REC = 0, bool SRC = false, bool COMPACT = false>
+template <int N, int MODE, bool SC, bool CURVED = false, int REC = 0, bool SRC = false, bool COMPACT = false,
+          bool BEGIN = false>
 static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? VolCfg<N>::SC_CURVED_MIN_BLOCKS
                                                                          : VolCfg<N>::MDRK_MIN_BLOCKS)
     mdrk1_volume_kernel(VolArgs a) {
+    static_assert(!BEGIN || COMPACT, "dt in the kernel: the plain step");
     static_assert(REC == 0 || (SC && CURVED), "MUSCL subcells: curvilinear shock capturing");
     static_assert(!SRC || !SC, "source terms: the FR volume integral");
     static_assert(!COMPACT || (!SC && !CURVED && !SRC && MODE == MODE_STEP), "compact stages: the plain TreeMesh step");
@@ -1222,8 +1247,10 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
         blended = !(fabs(alpha_e) <= 1e-12);
         muscl = REC >= 1 && blended && !__ldg(a.atb + e);
     }
-    // dt of this element's instance (batched form) or the single dt
-    const double dt = a.inst ? a.dt[__ldg(a.inst + min(e, a.E - 1))] : *a.dt;
+    double dt = 0.0;
+    __shared__ double s_dt;
+    if constexpr (BEGIN) begin_step<C>(a, &s_dt, tid);
+    else dt = a.inst ? a.dt[__ldg(a.inst + min(e, a.E - 1))] : *a.dt;
     double uu[NV], f0[NV], g0[NV], ij = 0.0, Ja[4] = {0.0, 0.0, 0.0, 0.0};
     // a flux pair into the contraction planes (contravariant on curvilinear meshes)
     auto put = [&](const double* f, const double* g) {
@@ -1251,7 +1278,12 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
             sc_park<N, C>(UU, VC, el, i, j, uu, a.gamma, a.status);
         }
     }
-    phase_sync<C>();
+    if (BEGIN) {
+        __syncthreads();
+        dt = s_dt;
+    } else {
+        phase_sync<C>();
+    }
     // (the MUSCL face values are read by the neighbours after the next barrier)
     if (SC && CURVED && REC >= 1 && muscl) sc_muscl_faces<N, C, REC>(a, UU, UF, el, e, i, j, a.gm1, alpha_e, 0.5 * dt, ij);
     line_contract<N, C, false>(X, Y, tid);
