@@ -970,7 +970,7 @@ struct AL {
             sa.nbr = h->d_nbr;
             sa.E = (int)h->E;
             using C = SurfCfg<N>;
-            surface_kernel<N, false, false><<<(unsigned)((sa.E + C::EB - 1) / C::EB), C::THREADS, 0, s>>>(sa, BndArgs{});
+            surface_kernel<N, false, false><<<(unsigned)((sa.E + C::EB - 1) / C::EB), C::THREADS, 0, s>>>(sa, BndArgs{}, MortarArgs{});
             return;
         }
         sa.left = h->d_xl; sa.right = h->d_xr; sa.count = h->nx; sa.orientation = 1;

@@ -123,7 +123,7 @@ struct BLaunch {
     }
     static void surfaces(cudaStream_t s, const SurfArgs& a) {
         using C = SurfCfg<N>;
-        surface_kernel<N, false, false><<<(unsigned)((a.E + C::EB - 1) / C::EB), C::THREADS, 0, s>>>(a, BndArgs{});
+        surface_kernel<N, false, false><<<(unsigned)((a.E + C::EB - 1) / C::EB), C::THREADS, 0, s>>>(a, BndArgs{}, MortarArgs{});
     }
     static void interfaces(cudaStream_t s, int block, const SurfArgs& a) {
         const long long threads = (long long)a.count * (N + 1);

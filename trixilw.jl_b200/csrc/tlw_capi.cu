@@ -55,6 +55,7 @@ void free_mesh(tlw_handle* h) {
     drop_graphs(h);
     dfree(h->d_inv_jac);
     dfree(h->d_xl); dfree(h->d_xr); dfree(h->d_yl); dfree(h->d_yr); dfree(h->d_nbr);
+    h->nbr_open.clear();
     dfree(h->d_xnode); dfree(h->d_S2);
     h->source = 0;
     dfree(h->d_b_elem); dfree(h->d_b_dir); dfree(h->d_bx); dfree(h->d_by);
@@ -132,7 +133,7 @@ template <int N> struct Vol {
 };
 template <int N> struct Ifc { static void run(cudaStream_t s, const SurfArgs& a) { Launch<N>::interfaces(s, a); } };
 template <int N> struct Srf {
-    static void run(cudaStream_t s, const SurfArgs& a, const BndArgs& b) { Launch<N>::surfaces(s, a, b); }
+    static void run(cudaStream_t s, const SurfArgs& a, const BndArgs& b, const MortarArgs& m) { Launch<N>::surfaces(s, a, b, m); }
 };
 template <int N> struct Bnd { static void run(cudaStream_t s, const BndArgs& a) { Launch<N>::boundaries(s, a); } };
 template <int N> struct Par {
@@ -222,8 +223,8 @@ bool use_slots(const tlw_handle* h) {
 #define TLW_SURFACE_PASS_SC 0
 #endif
 bool use_surface_pass(const tlw_handle* h) {
-    return TLW_SURFACE_PASS && h->d_nbr && !h->curved && (!h->sc || TLW_SURFACE_PASS_SC) && h->nmx + h->nmy == 0 &&
-           h->nh == 0;
+    return TLW_SURFACE_PASS && h->d_nbr && !h->curved && (!h->sc || TLW_SURFACE_PASS_SC) && h->nh == 0 &&
+           (h->nmx + h->nmy == 0 || h->nbr_mortars);
 }
 
 // the partial CFL maxima of the state in buffer k
@@ -466,7 +467,7 @@ void enqueue_rhs(tlw_handle* h, int stage, int mode, const double* u_flux, const
         if (use_surface_pass(h)) {
             sp.nbr = h->d_nbr;
             sp.E = (int)h->E;
-            dispatch<Srf>(h->N, h->stream, sp, bp);
+            dispatch<Srf>(h->N, h->stream, sp, bp, MortarArgs{});
             if (ev) {
                 cudaEventRecord(ev->after_x, h->stream);
                 cudaEventRecord(ev->after_y, h->stream);
@@ -603,7 +604,10 @@ void enqueue_rhs(tlw_handle* h, int stage, int mode, const double* u_flux, const
         if (!(phases & 2)) return;
         sa.nbr = h->d_nbr;
         sa.E = (int)h->E;
-        dispatch<Srf>(h->N, h->stream, sa, ba);
+        if (h->nmx + h->nmy > 0) {
+            ma.lower = h->d_ml; ma.upper = h->d_mu; ma.large = h->d_mg; ma.large_side = h->d_ms;
+        }
+        dispatch<Srf>(h->N, h->stream, sa, ba, ma);
         if (ev) {
             cudaEventRecord(ev->after_x, h->stream);
             cudaEventRecord(ev->after_y, h->stream);
@@ -876,9 +880,9 @@ int tlw_set_tree_mesh(tlw_handle* h, int64_t n_elements, const double* inverse_j
         (rc = up_i(h->d_by, by)))
         return rc;
     h->nx = (int)xl.size(); h->ny = (int)yl.size();
-    if (2 * (int64_t)(xl.size() + yl.size()) + n_boundaries == 4 * n_elements) {
+    {
         // every face a conforming interface or a boundary: the element-centric surface pass takes the element
-        // across each face, or -(k + 1) for boundary k
+        // across each face, or -(k + 1) for boundary k (the mortars' faces follow in tlw_set_tree_mortars)
         constexpr int unset = std::numeric_limits<int>::min();
         std::vector<int> nbr((size_t)4 * n_elements, unset);
         bool ok = true;
@@ -890,7 +894,11 @@ int tlw_set_tree_mesh(tlw_handle* h, int64_t n_elements, const double* inverse_j
         for (size_t k = 0; k < xl.size(); ++k) { put(xl[k], 1, xr[k]); put(xr[k], 0, xl[k]); }
         for (size_t k = 0; k < yl.size(); ++k) { put(yl[k], 3, yr[k]); put(yr[k], 2, yl[k]); }
         for (size_t k = 0; k < belem.size(); ++k) put(belem[k], bdir[k] - 1, -(int)k - 1);
-        if (ok && (rc = up_i(h->d_nbr, nbr))) return rc;
+        if (ok && std::find(nbr.begin(), nbr.end(), unset) == nbr.end()) {
+            if ((rc = up_i(h->d_nbr, nbr))) return rc;
+        } else if (ok) {
+            h->nbr_open = std::move(nbr);
+        }
     }
     h->jac_first = inverse_jacobian[0];
     if (h->sc) {
@@ -1167,6 +1175,31 @@ int tlw_set_tree_mortars(tlw_handle* h, int64_t n_mortars, const int64_t* mortar
     drop_graphs(h);
     dfree(h->d_ml); dfree(h->d_mu); dfree(h->d_mg); dfree(h->d_ms);
     if (h->d_mface) { cudaFree(h->d_mface); h->d_mface = nullptr; }
+    h->slots_valid = false;
+    if (!h->nbr_open.empty()) dfree(h->d_nbr);
+    h->nbr_mortars = false;
+    if (n_mortars > 0 && !h->nbr_open.empty()) {
+        constexpr int unset = std::numeric_limits<int>::min();
+        std::vector<int> nbr(h->nbr_open);
+        bool ok = true;
+        auto put = [&](int e, int f, int m, int role) {
+            int& slot = nbr[(size_t)4 * e + f];
+            if (slot != unset) ok = false;
+            slot = NBR_MORTAR + (m << 2 | role);
+        };
+        for (int d = 0, m = 0; d < 2; ++d)
+            for (size_t k = 0; k < ml[d].size(); ++k, ++m) {
+                const int large_face = ms[d][k] == 1 ? 2 * d + 1 : 2 * d, small_face = large_face ^ 1;
+                put(ml[d][k], small_face, m, 0);
+                put(mu[d][k], small_face, m, 1);
+                put(mg[d][k], large_face, m, 2);
+            }
+        if (ok && std::find(nbr.begin(), nbr.end(), unset) == nbr.end()) {
+            TLW_CUDA(h, cudaMalloc(&h->d_nbr, nbr.size() * sizeof(int)));
+            TLW_CUDA(h, upload_on(h->stream, h->d_nbr, nbr.data(), nbr.size() * sizeof(int)));
+            h->nbr_mortars = true;
+        }
+    }
     h->nmx = (int)ml[0].size();
     h->nmy = (int)ml[1].size();
     if (n_mortars > 0) {

@@ -90,7 +90,11 @@ struct tlw_handle {
     int64_t E = 0;
     double* d_inv_jac = nullptr;
     int *d_xl = nullptr, *d_xr = nullptr, *d_yl = nullptr, *d_yr = nullptr;
-    int* d_nbr = nullptr;   // [4, E] element across each face when every face is a conforming interface
+    // [4, E] the element across each face, boundary or mortar side (surface_kernel), when every face has one; the host
+    // copy of a mesh whose faces the interfaces and boundaries leave open, for its mortars
+    int* d_nbr = nullptr;
+    std::vector<int> nbr_open;
+    bool nbr_mortars = false;               // d_nbr has the mortar sides
     // source terms (TreeMesh, FR volume integral): kind, node coordinates [2, i, j, e], MDRK stage 1's S2
     int source = 0;
     double* d_xnode = nullptr;

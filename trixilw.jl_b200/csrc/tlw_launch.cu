@@ -201,16 +201,19 @@ struct LaunchImpl {
         if (threads == 0) return;
         interface_kernel<N><<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(a);
     }
-    static void surfaces(cudaStream_t s, const SurfArgs& a, const BndArgs& b) {
+    static void surfaces(cudaStream_t s, const SurfArgs& a, const BndArgs& b, const MortarArgs& m) {
         if (a.E <= 0) return;
         using C = SurfCfg<N>;
         const unsigned grid = (unsigned)((a.E + C::EB - 1) / C::EB);
-        if (a.shock_capturing) {
-            if (b.element) surface_kernel<N, true, true><<<grid, C::THREADS, 0, s>>>(a, b);
-            else surface_kernel<N, false, true><<<grid, C::THREADS, 0, s>>>(a, b);
+        if (m.lower) {
+            if (b.element) surface_kernel<N, true, false, true><<<grid, C::THREADS, 0, s>>>(a, b, m);
+            else surface_kernel<N, false, false, true><<<grid, C::THREADS, 0, s>>>(a, b, m);
+        } else if (a.shock_capturing) {
+            if (b.element) surface_kernel<N, true, true><<<grid, C::THREADS, 0, s>>>(a, b, m);
+            else surface_kernel<N, false, true><<<grid, C::THREADS, 0, s>>>(a, b, m);
         } else {
-            if (b.element) surface_kernel<N, true, false><<<grid, C::THREADS, 0, s>>>(a, b);
-            else surface_kernel<N, false, false><<<grid, C::THREADS, 0, s>>>(a, b);
+            if (b.element) surface_kernel<N, true, false><<<grid, C::THREADS, 0, s>>>(a, b, m);
+            else surface_kernel<N, false, false><<<grid, C::THREADS, 0, s>>>(a, b, m);
         }
     }
     static void parabolic(cudaStream_t s, const tlw_handle* h, int mode, const double* u, double* out,
@@ -352,8 +355,8 @@ template <int N> void Launch<N>::volume(cudaStream_t s, int stage, int mode, boo
     LaunchImpl<N>::volume(s, stage, mode, sc, a);
 }
 template <int N> void Launch<N>::interfaces(cudaStream_t s, const SurfArgs& a) { LaunchImpl<N>::interfaces(s, a); }
-template <int N> void Launch<N>::surfaces(cudaStream_t s, const SurfArgs& a, const BndArgs& b) {
-    LaunchImpl<N>::surfaces(s, a, b);
+template <int N> void Launch<N>::surfaces(cudaStream_t s, const SurfArgs& a, const BndArgs& b, const MortarArgs& m) {
+    LaunchImpl<N>::surfaces(s, a, b, m);
 }
 template <int N> void Launch<N>::boundaries(cudaStream_t s, const BndArgs& a) { LaunchImpl<N>::boundaries(s, a); }
 template <int N>

@@ -56,6 +56,54 @@ __device__ __forceinline__ int tree_face_node(int n, int f, int l) {
     return f == 0 ? n * l : f == 1 ? (n - 1) + n * l : f == 2 ? l : l + n * (n - 1);
 }
 
+// The LW flux along +x / +y at node l of half h (0 lower, 1 upper) of mortar k (calc_mortar_flux!): the large face's
+// traces interpolated to the half's node against the small element's
+template <int N>
+__device__ __forceinline__ void mortar_node_flux(const MortarArgs& a, int o, int k, int h, int l, double* fstar) {
+    constexpr int n = N + 1, nn = n * n;
+    const int se = h ? __ldg(a.upper + k) : __ldg(a.lower + k), lg = __ldg(a.large + k);
+    const bool left = __ldg(a.large_side + k) == 1;
+    const int small_face = left ? (o == 1 ? 0 : 2) : (o == 1 ? 1 : 3);
+    const int large_face = left ? (o == 1 ? 1 : 3) : (o == 1 ? 0 : 2);
+    const int ns = tree_face_node(n, small_face, l);
+    double us[NV], Us[NV], Fs[NV], ul[NV] = {0, 0, 0, 0}, Ul[NV] = {0, 0, 0, 0}, Fl[NV] = {0, 0, 0, 0};
+    load4w(a.u + ((size_t)se * nn + ns) * NV, us);
+    const size_t ts = (((size_t)se * 4 + small_face) * n + l) * NV;
+    load4w(a.tU + ts, Us);
+    load4w(a.tF + ts, Fs);
+    const double* fwd = c_tlw_mortar[N][h ? 0 : 1];
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+        double x[NV], y[NV], z[NV];
+        load4w(a.u + ((size_t)lg * nn + tree_face_node(n, large_face, j)) * NV, x);
+        const size_t tl = (((size_t)lg * 4 + large_face) * n + j) * NV;
+        load4w(a.tU + tl, y);
+        load4w(a.tF + tl, z);
+        const double c = fwd[l * n + j];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            ul[v] = fma(c, x[v], ul[v]);
+            Ul[v] = fma(c, y[v], Ul[v]);
+            Fl[v] = fma(c, z[v], Fl[v]);
+        }
+    }
+    if (left) lw_surface_flux(a.gamma, a.flux_kind, a.speed_kind, Fl, Fs, Ul, Us, ul, us, o, fstar, a.status);
+    else lw_surface_flux(a.gamma, a.flux_kind, a.speed_kind, Fs, Fl, Us, Ul, us, ul, o, fstar, a.status);
+}
+// the large face's flux at its node l: the L2 projection of the halves' fluxes (node q at lower + q * NV, upper + q * NV)
+template <int N>
+__device__ __forceinline__ void mortar_projection(const double* lower, const double* upper, int l, double* p) {
+    constexpr int n = N + 1;
+    const double* ru = c_tlw_mortar[N][2];
+    const double* rl = c_tlw_mortar[N][3];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) p[v] = 0.0;
+#pragma unroll
+    for (int q = 0; q < n; ++q)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) p[v] = fma(ru[l * n + q], upper[q * NV + v], fma(rl[l * n + q], lower[q * NV + v], p[v]));
+}
+
 template <int N>
 static __global__ void __launch_bounds__(128) mortar_kernel(MortarArgs a) {
     using C = MortarCfg<N>;
@@ -79,30 +127,8 @@ static __global__ void __launch_bounds__(128) mortar_kernel(MortarArgs a) {
         small_face = left ? (o == 1 ? 0 : 2) : (o == 1 ? 1 : 3);
         large_face = left ? (o == 1 ? 1 : 3) : (o == 1 ? 0 : 2);
         const int ns = tree_face_node(n, small_face, l);
-        double us[NV], Us[NV], Fs[NV], ul[NV] = {0, 0, 0, 0}, Ul[NV] = {0, 0, 0, 0}, Fl[NV] = {0, 0, 0, 0};
-        load4(a.u + ((size_t)se * nn + ns) * NV, us);
-        const size_t ts = (((size_t)se * 4 + small_face) * n + l) * NV;
-        load4(a.tU + ts, Us);
-        load4(a.tF + ts, Fs);
-        const double* fwd = c_tlw_mortar[N][h ? 0 : 1];
-#pragma unroll
-        for (int j = 0; j < n; ++j) {
-            double x[NV], y[NV], z[NV];
-            load4(a.u + ((size_t)lg * nn + tree_face_node(n, large_face, j)) * NV, x);
-            const size_t tl = (((size_t)lg * 4 + large_face) * n + j) * NV;
-            load4(a.tU + tl, y);
-            load4(a.tF + tl, z);
-            const double c = fwd[l * n + j];
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                ul[v] = fma(c, x[v], ul[v]);
-                Ul[v] = fma(c, y[v], Ul[v]);
-                Fl[v] = fma(c, z[v], Fl[v]);
-            }
-        }
         double fstar[NV];
-        if (left) lw_surface_flux(a.gamma, a.flux_kind, a.speed_kind, Fl, Fs, Ul, Us, ul, us, o, fstar, a.status);
-        else lw_surface_flux(a.gamma, a.flux_kind, a.speed_kind, Fs, Fl, Us, Ul, us, ul, o, fstar, a.status);
+        mortar_node_flux<N>(a, o, k, h, l, fstar);
         dts = a.step_mode ? *a.dt : 1.0;
         // small element: fstar is the flux along +x / +y through its face
         const double cs = left ? dts * __ldg(a.inv_jac + se) * a.inv_w_first : -dts * __ldg(a.inv_jac + se) * a.inv_w_last;
@@ -118,13 +144,8 @@ static __global__ void __launch_bounds__(128) mortar_kernel(MortarArgs a) {
     }
     __syncthreads();
     if (active && h == 0) {
-        const double* ru = c_tlw_mortar[N][2];
-        const double* rl = c_tlw_mortar[N][3];
-        double p[NV] = {0, 0, 0, 0};
-#pragma unroll
-        for (int q = 0; q < n; ++q)
-#pragma unroll
-            for (int v = 0; v < NV; ++v) p[v] = fma(ru[l * n + q], fs[g][1][q][v], fma(rl[l * n + q], fs[g][0][q][v], p[v]));
+        double p[NV];
+        mortar_projection<N>(&fs[g][0][0][0], &fs[g][1][0][0], l, p);
         const double cl = left ? -dts * __ldg(a.inv_jac + lg) * a.inv_w_last : dts * __ldg(a.inv_jac + lg) * a.inv_w_first;
         double* ol = a.out + ((size_t)lg * nn + tree_face_node(n, large_face, l)) * NV;
         double x[NV];
