@@ -665,7 +665,7 @@ void enqueue_step(tlw_handle* h, int from, cudaEvent_t after_dt = nullptr, const
                        false, indicator_args(h));
     if (fused) {
         if (!begin_in_volume(h))
-            begin_step_kernel<<<1, 1, 0, h->stream>>>(h->d_step, ring_slot(h, from), ring_slot(h, 1 - from), h->n);
+            launch_dependent(h->stream, begin_step_kernel, 1, 1, 0, h->d_step, ring_slot(h, from), ring_slot(h, 1 - from), h->n);
     } else if (h->parabolic) par_finalize_dt_kernel<<<1, 1, 0, h->stream>>>(h->d_step, h->d_visc, h->N, h->curved ? 1 : 0);
     else finalize_dt_kernel<<<1, 1, 0, h->stream>>>(h->d_step, h->n);
     if (after_dt) cudaEventRecord(after_dt, h->stream);

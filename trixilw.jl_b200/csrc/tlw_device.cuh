@@ -10,6 +10,27 @@ constexpr int NV = 4;   // compressible Euler 2D: rho, rho v1, rho v2, rho e
 // status bits written by kernels (never a trap): the host maps them to TLW_E_* codes
 constexpr unsigned STATUS_NONADMISSIBLE = 1u;   // sqrt of a negative number (reference: DomainError)
 
+// Programmatic dependent launch: a kernel launched by launch_dependent may start before the one in front of it on its
+// stream has ended. It waits here, before its first access to global memory; the kernel in front lets it start once all
+// of its own CTAs have (dependents_may_start), so that the launch latency and the CTA set-up of a chain of short kernels
+// overlap. Both are no-ops in a kernel launched the ordinary way.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <class... P, class... A>
+inline void launch_dependent(cudaStream_t s, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, const A&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 struct Basis {
     double D[16 * 16];      // derivative matrix, D[a*n + b] = l_b'(x_a)
     double Dhat[16 * 16];   // -M^{-1} D^T M

@@ -92,20 +92,20 @@ struct LaunchImpl {
     static void volume_sc(cudaStream_t s, int stage, int mode, const VolArgs& a, int grid) {
         const size_t lw = C::lw_bytes(SC), md = C::mdrk_bytes(SC);
         if (stage == TLW_STAGE_LW) {
-            if (mode == MODE_RHS) lw_volume_kernel<N, MODE_RHS, SC><<<grid, C::THREADS, lw, s>>>(a);
-            else if (!SC && a.step) lw_volume_kernel<N, MODE_STEP, false, 0, false, false, false, 0, false, true><<<grid, C::THREADS, lw, s>>>(a);
-            else lw_volume_kernel<N, MODE_STEP, SC><<<grid, C::THREADS, lw, s>>>(a);
+            if (mode == MODE_RHS) launch_dependent(s, lw_volume_kernel<N, MODE_RHS, SC>, grid, C::THREADS, lw, a);
+            else if (!SC && a.step) launch_dependent(s, lw_volume_kernel<N, MODE_STEP, false, 0, false, false, false, 0, false, true>, grid, C::THREADS, lw, a);
+            else launch_dependent(s, lw_volume_kernel<N, MODE_STEP, SC>, grid, C::THREADS, lw, a);
         } else if (stage == TLW_STAGE_MDRK1) {
-            if (mode == MODE_RHS) mdrk1_volume_kernel<N, MODE_RHS, SC><<<grid, C::THREADS, md, s>>>(a);
+            if (mode == MODE_RHS) launch_dependent(s, mdrk1_volume_kernel<N, MODE_RHS, SC>, grid, C::THREADS, md, a);
             else if (!SC && a.compact && a.step)
-                mdrk1_volume_kernel<N, MODE_STEP, false, false, 0, false, true, true><<<grid, C::THREADS, md, s>>>(a);
-            else if (!SC && a.compact) mdrk1_volume_kernel<N, MODE_STEP, false, false, 0, false, true><<<grid, C::THREADS, md, s>>>(a);
-            else mdrk1_volume_kernel<N, MODE_STEP, SC><<<grid, C::THREADS, md, s>>>(a);
+                launch_dependent(s, mdrk1_volume_kernel<N, MODE_STEP, false, false, 0, false, true, true>, grid, C::THREADS, md, a);
+            else if (!SC && a.compact) launch_dependent(s, mdrk1_volume_kernel<N, MODE_STEP, false, false, 0, false, true>, grid, C::THREADS, md, a);
+            else launch_dependent(s, mdrk1_volume_kernel<N, MODE_STEP, SC>, grid, C::THREADS, md, a);
         } else {
-            if (mode == MODE_RHS) mdrk2_volume_kernel<N, MODE_RHS, SC><<<grid, C::THREADS, md, s>>>(a);
+            if (mode == MODE_RHS) launch_dependent(s, mdrk2_volume_kernel<N, MODE_RHS, SC>, grid, C::THREADS, md, a);
             else if (!SC && a.compact)
-                mdrk2_volume_kernel<N, MODE_STEP, false, false, 0, false, true><<<grid, C::THREADS, C::mdrk_bytes(false, 0, true), s>>>(a);
-            else mdrk2_volume_kernel<N, MODE_STEP, SC><<<grid, C::THREADS, md, s>>>(a);
+                launch_dependent(s, mdrk2_volume_kernel<N, MODE_STEP, false, false, 0, false, true>, grid, C::THREADS, C::mdrk_bytes(false, 0, true), a);
+            else launch_dependent(s, mdrk2_volume_kernel<N, MODE_STEP, SC>, grid, C::THREADS, md, a);
         }
     }
     // curvilinear shock capturing: LW or an MDRK stage with first-order (REC 0), MUSCL (REC 1) or MUSCL-Hancock
@@ -206,14 +206,14 @@ struct LaunchImpl {
         using C = SurfCfg<N>;
         const unsigned grid = (unsigned)((a.E + C::EB - 1) / C::EB);
         if (m.lower) {
-            if (b.element) surface_kernel<N, true, false, true><<<grid, C::THREADS, 0, s>>>(a, b, m);
-            else surface_kernel<N, false, false, true><<<grid, C::THREADS, 0, s>>>(a, b, m);
+            if (b.element) launch_dependent(s, surface_kernel<N, true, false, true>, grid, C::THREADS, 0, a, b, m);
+            else launch_dependent(s, surface_kernel<N, false, false, true>, grid, C::THREADS, 0, a, b, m);
         } else if (a.shock_capturing) {
-            if (b.element) surface_kernel<N, true, true><<<grid, C::THREADS, 0, s>>>(a, b, m);
-            else surface_kernel<N, false, true><<<grid, C::THREADS, 0, s>>>(a, b, m);
+            if (b.element) launch_dependent(s, surface_kernel<N, true, true>, grid, C::THREADS, 0, a, b, m);
+            else launch_dependent(s, surface_kernel<N, false, true>, grid, C::THREADS, 0, a, b, m);
         } else {
-            if (b.element) surface_kernel<N, true, false><<<grid, C::THREADS, 0, s>>>(a, b, m);
-            else surface_kernel<N, false, false><<<grid, C::THREADS, 0, s>>>(a, b, m);
+            if (b.element) launch_dependent(s, surface_kernel<N, true, false>, grid, C::THREADS, 0, a, b, m);
+            else launch_dependent(s, surface_kernel<N, false, false>, grid, C::THREADS, 0, a, b, m);
         }
     }
     static void parabolic(cudaStream_t s, const tlw_handle* h, int mode, const double* u, double* out,

@@ -357,6 +357,8 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, (BND || SC || MORT
     constexpr int n = N + 1, EB = C::EB, NB = 4 * (n - 1);
     __shared__ double sF[EB * 4 * n * NV], sG[MORTAR ? EB * 4 * n * NV : 1];
     const int tid = threadIdx.x;
+    wait_for_previous();
+    dependents_may_start();
     bool large = false;   // MORTAR: this thread's face is a mortar's large one
     // TLW_SURF_REVERSE: the CTAs take the elements from the last one down, so that the first ones read the traces
     // and face nodes the volume kernel wrote last (still in L2), and the next volume kernel, which starts from the
@@ -693,6 +695,7 @@ static __global__ void finalize_dt_kernel(StepState* s, int n) {
 
 // dt of a step that keeps its own CFL maximum, where its first kernel does not form it
 static __global__ void begin_step_kernel(StepState* s, const unsigned long long* ring, unsigned long long* ring_next, int n) {
+    wait_for_previous();
     begin_step_dt(s, ring, ring_next, n, true);
 }
 

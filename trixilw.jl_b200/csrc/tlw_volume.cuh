@@ -908,6 +908,8 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
     double* UF = FVY + C::PLANES;      // curvilinear MUSCL: face values, 4 regions (left, right, down, up)
 
     const int tid = threadIdx.x;
+    wait_for_previous();
+    dependents_may_start();
     prefetch_next<C>(a.u, 4, a.E, tid);
     if (CURVED) {
         prefetch_next<C>(a.metrics, 4, a.E, tid);
@@ -1234,6 +1236,8 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     double* FVY = FVX + C::PLANES;
     double* UF = FVY + C::PLANES;      // curvilinear MUSCL: face values, 4 regions (left, right, down, up)
     const int tid = threadIdx.x;
+    wait_for_previous();
+    dependents_may_start();
     prefetch_next<C>(a.u, 4, a.E, tid);
     const int el = tid / nn;
     const int node = tid - el * nn;
@@ -1392,6 +1396,8 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     double* FVY = FVX + C::PLANES;
     double* UF = FVY + C::PLANES;      // curvilinear MUSCL: face values, 4 regions (left, right, down, up)
     const int tid = threadIdx.x;
+    wait_for_previous();
+    dependents_may_start();
     prefetch_next<C>(a.u, 4, a.E, tid);
     if (COMPACT) {
         prefetch_next<C>(a.u_base, 4, a.E, tid);
