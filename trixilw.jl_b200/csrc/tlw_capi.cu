@@ -49,6 +49,9 @@ void drop_graphs(tlw_handle* h) {
         if (h->g_two[k]) cudaGraphExecDestroy(h->g_two[k]);
         h->g_one[k] = h->g_two[k] = nullptr;
     }
+    if (h->g_many) cudaGraphExecDestroy(h->g_many);
+    h->g_many = nullptr;
+    h->replayed = 0;
 }
 
 void free_mesh(tlw_handle* h) {
@@ -2134,11 +2137,19 @@ int tlw_step(tlw_handle* h, int32_t nsteps, double cfl, double fixed_dt, double 
     if ((rc = capture(0, 1, h->g_one[0])) || (rc = capture(1, 1, h->g_one[1])) || (rc = capture(0, 2, h->g_two[0])))
         return rc;
     int left = nsteps;
+    h->replayed += left;
     if (h->cur == 1) {
         if ((rc = capture(1, 1, h->g_one[1]))) return rc;
         TLW_CUDA(h, cudaGraphLaunch(h->g_one[1], h->stream));
         h->cur = 0;
         --left;
+    }
+    // long runs in graphs of many steps (the gap between two graphs falls between fewer steps), once the steps replayed
+    // have paid for their capture
+    constexpr int many = tlw_handle::MANY_STEPS;
+    if (left >= many && h->replayed >= tlw_handle::MANY_AFTER) {
+        if ((rc = capture(0, many, h->g_many))) return rc;
+        for (; left >= many; left -= many) TLW_CUDA(h, cudaGraphLaunch(h->g_many, h->stream));
     }
     if (left >= 2) {
         if ((rc = capture(0, 2, h->g_two[0]))) return rc;

@@ -210,6 +210,9 @@ struct tlw_handle {
     // graphs: [start buffer] one step, two steps
     cudaGraphExec_t g_one[2] = {nullptr, nullptr};
     cudaGraphExec_t g_two[2] = {nullptr, nullptr};
+    cudaGraphExec_t g_many = nullptr;       // MANY_STEPS steps from buffer 0, captured once replayed reaches that many
+    static constexpr int MANY_STEPS = 8, MANY_AFTER = 24;
+    long long replayed = 0;                 // steps replayed from these graphs
     // discrete adjoint
     tlw::AdjointBuffers adj;
 };
