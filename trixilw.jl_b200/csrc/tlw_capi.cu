@@ -95,6 +95,8 @@ void free_mesh(tlw_handle* h) {
     if (h->d_adapt) { cudaFree(h->d_adapt); h->d_adapt = nullptr; }
     h->color_off.clear();
     h->face_used.clear();
+    dfree(h->d_cnbr);
+    h->cnbr_open.clear();
     for (int** d : {&h->d_he, &h->d_hf, &h->d_hs})
         if (*d) { cudaFree(*d); *d = nullptr; }
     dfree(h->d_send); dfree(h->d_recv); dfree(h->d_asend); dfree(h->d_arecv);
@@ -154,9 +156,13 @@ template <int N> struct CBnd { static void run(cudaStream_t s, const CurvedBndAr
 template <int N> struct Lim { static void run(cudaStream_t s, const LimiterArgs& a) { Launch<N>::limiter(s, a); } };
 template <int N> struct Const { static void run(const Basis* all, cudaError_t* e) { if (*e == cudaSuccess) *e = Launch<N>::upload_constants(all); } };
 template <int N> struct CSpd {
-    static void run(cudaStream_t s, const double* u, const double* Ja, const double* ij, int E, double g, StepState* st) {
-        Launch<N>::curved_speed(s, u, Ja, ij, E, g, st);
+    static void run(cudaStream_t s, const double* u, const double* Ja, const double* ij, int E, double g, StepState* st,
+                    unsigned long long* target = nullptr) {
+        Launch<N>::curved_speed(s, u, Ja, ij, E, g, st, target);
     }
+};
+template <int N> struct CSrf {
+    static void run(cudaStream_t s, const CurvedSurfArgs& a, const CurvedBndArgs& b) { Launch<N>::curved_surfaces(s, a, b); }
 };
 template <int N> struct Spd {
     static void run(cudaStream_t s, const double* u, const double* ij, int E, double g, StepState* st, bool speed,
@@ -197,9 +203,8 @@ void enqueue_indicator(tlw_handle* h, const double* u, bool speed) {
     // interfaces for the smoothing: the TreeMesh list, or the curvilinear mesh's (primary, secondary) pairs
     const int ni = h->curved ? (h->color_off.empty() ? 0 : h->color_off.back()) : h->ni;
     if (h->opts.alpha_smooth && ni > 0)
-        alpha_smooth_kernel<<<(ni + 255) / 256, 256, 0, h->stream>>>(h->curved ? h->d_cp : h->d_il,
-                                                                    h->curved ? h->d_cs : h->d_ir, ni,
-                                                                    h->d_alpha_raw, h->d_alpha);
+        launch_dependent(h->stream, alpha_smooth_kernel, (ni + 255) / 256, 256, 0, h->curved ? h->d_cp : h->d_il,
+                         h->curved ? h->d_cs : h->d_ir, ni, h->d_alpha_raw, h->d_alpha);
     // and over the curvilinear mesh's mortars (each small element with the large one)
     if (h->opts.alpha_smooth && h->curved && h->ncms > 0)
         alpha_smooth_kernel<<<(h->ncms + 255) / 256, 256, 0, h->stream>>>(h->d_cmsl, h->d_cmsr, h->ncms,
@@ -230,20 +235,25 @@ bool use_surface_pass(const tlw_handle* h) {
            (h->nmx + h->nmy == 0 || h->nbr_mortars);
 }
 
+// one element-centric pass for all faces of a curvilinear mesh instead of a launch per colour and boundary class (not
+// with shock capturing, whose flux is too long to evaluate on both sides: the warped 150 x 133 blast, MUSCL, took 125 us
+// a step with it against 112 by colours)
+bool use_curved_pass(const tlw_handle* h) { return h->curved && h->d_cnbr && h->ncm == 0 && !h->sc; }
+
 // the partial CFL maxima of the state in buffer k
 unsigned long long* ring_slot(tlw_handle* h, int k) { return h->d_ring + (size_t)k * RING_WAYS * RING_STRIDE; }
 
 // a step that keeps its own CFL maximum: its surface pass reduces the new state's into ring_slot, and the next
 // step's first kernel takes dt from there (begin_step). Not with the limiter, which changes the state afterwards.
 bool fused_cfl(const tlw_handle* h) {
-    return h->d_slots && use_surface_pass(h) && !h->sc && !h->parabolic && h->lim_count == 0;
+    return h->d_slots && (use_surface_pass(h) || use_curved_pass(h)) && !h->sc && !h->parabolic && h->lim_count == 0;
 }
 
 // Whether the volume kernel of a fused step forms dt itself: it costs each CTA about 1 % (512^2: N = 3 0.195 -> 0.200,
 // N = 4 0.430 -> 0.434, N = 5 0.699 -> 0.707 ms), a dt launch about 3 us, so up to 16 resident sets of CTAs (148 SMs x 5
 // CTAs of about 128 nodes). Not with source terms, whose kernels are not built that way.
 bool begin_in_volume(const tlw_handle* h) {
-    return !h->source && (int64_t)h->E * h->nn <= (int64_t)16 * 148 * 5 * 128;
+    return !h->source && !h->curved && (int64_t)h->E * h->nn <= (int64_t)16 * 148 * 5 * 128;
 }
 
 // the halo faces of one class (cls 0: x, 1: y) as kernel arguments
@@ -301,7 +311,7 @@ void enqueue_limiter(tlw_handle* h, double* u, int reps, unsigned long long* slo
 // the surfaces of a curvilinear mesh: interfaces colour by colour (no two threads of a launch share a node),
 // then the xi-face and the eta-face boundaries; with the viscous traces for Navier-Stokes
 void enqueue_curved_surfaces(tlw_handle* h, int mode, const double* u_jump, double* out, const double* dt_ptr,
-                             const PhaseEvents* ev, double scaling_factor = 1.0) {
+                             const PhaseEvents* ev, double scaling_factor = 1.0, bool keep_cfl = false, int ring = 0) {
     CurvedSurfArgs ca{};
     ca.u = u_jump;
     ca.out = out;
@@ -327,6 +337,49 @@ void enqueue_curved_surfaces(tlw_handle* h, int mode, const double* u_jump, doub
     if (h->unstructured) {
         ca.tG = h->d_tG;
         ca.unorm = h->d_unorm;
+    }
+    CurvedBndArgs cb{};
+    if (h->ncb > 0) {
+        cb.u = u_jump;
+        cb.out = out;
+        cb.tU = h->d_tU;
+        cb.tF = h->d_tF;
+        cb.tFv = h->parabolic ? h->d_tFv : nullptr;
+        cb.metrics = h->d_Ja;
+        cb.inv_jac = h->d_ijn;
+        cb.wall_kind = h->d_wkind;
+        cb.wall = h->d_wall;
+        cb.dt = dt_ptr;
+        cb.step_mode = mode == MODE_STEP;
+        cb.gamma = h->opts.gamma;
+        cb.flux_kind = h->opts.surface_flux;
+        cb.speed_kind = h->opts.max_speed;
+        cb.inv_w_first = h->h_basis.inv_w_first;
+        cb.inv_w_last = h->h_basis.inv_w_last;
+        cb.status = &h->d_step->status;
+        cb.levels = h->d_levels;
+        cb.weights = h->d_basis->weights;
+        cb.scaling_factor = scaling_factor;
+        cb.elem = h->d_cbe;
+        cb.face = h->d_cbf;
+        cb.kind = h->d_cbk;
+        cb.index = h->d_cbi;
+        cb.count = h->ncb;
+    }
+    if (use_curved_pass(h)) {
+        ca.nbr = h->d_cnbr;
+        ca.E = (int)h->E;
+        if (keep_cfl) {
+            ca.cfl_interior = (const double*)h->d_slots;
+            ca.cfl_max = ring_slot(h, 1 - ring);
+            ca.advance = h->d_step;
+        }
+        dispatch<CSrf>(h->N, h->stream, ca, cb);
+        if (ev) {
+            cudaEventRecord(ev->after_x, h->stream);
+            cudaEventRecord(ev->after_y, h->stream);
+        }
+        return;
     }
     for (size_t c = 0; c + 1 < h->color_off.size(); ++c) {
         const int b = h->color_off[c];
@@ -372,27 +425,6 @@ void enqueue_curved_surfaces(tlw_handle* h, int mode, const double* u_jump, doub
         }
     }
     if (h->ncb > 0) {
-        CurvedBndArgs cb{};
-        cb.u = u_jump;
-        cb.out = out;
-        cb.tU = h->d_tU;
-        cb.tF = h->d_tF;
-        cb.tFv = h->parabolic ? h->d_tFv : nullptr;
-        cb.metrics = h->d_Ja;
-        cb.inv_jac = h->d_ijn;
-        cb.wall_kind = h->d_wkind;
-        cb.wall = h->d_wall;
-        cb.dt = dt_ptr;
-        cb.step_mode = mode == MODE_STEP;
-        cb.gamma = h->opts.gamma;
-        cb.flux_kind = h->opts.surface_flux;
-        cb.speed_kind = h->opts.max_speed;
-        cb.inv_w_first = h->h_basis.inv_w_first;
-        cb.inv_w_last = h->h_basis.inv_w_last;
-        cb.status = &h->d_step->status;
-        cb.levels = h->d_levels;
-        cb.weights = h->d_basis->weights;
-        cb.scaling_factor = scaling_factor;
         const int first[2] = {0, h->ncbx}, count[2] = {h->ncbx, h->ncb - h->ncbx};
         for (int cls = 0; cls < 2; ++cls) {
             cb.elem = h->d_cbe + first[cls];
@@ -553,7 +585,8 @@ void enqueue_rhs(tlw_handle* h, int stage, int mode, const double* u_flux, const
         if (!(phases & 2)) return;
         // MDRK stage 1 scales the Dirichlet time averages by 1/2, as the P4estMesh path does
         // (src/solvers/dgsem_tree/multi_derivative_2d.jl:34)
-        enqueue_curved_surfaces(h, mode, u_jump, out, dt_ptr, ev, stage == TLW_STAGE_MDRK1 ? 0.5 : 1.0);
+        enqueue_curved_surfaces(h, mode, u_jump, out, dt_ptr, ev, stage == TLW_STAGE_MDRK1 ? 0.5 : 1.0,
+                                fused && stage != TLW_STAGE_MDRK1, ring);
         return;
     }
 
@@ -653,6 +686,10 @@ void enqueue_step(tlw_handle* h, int from, cudaEvent_t after_dt = nullptr, const
     if (fused) {
         if (!h->slots_valid) {   // the first step of a state: its CFL maximum by a pass over it
             cudaMemsetAsync(ring_slot(h, from), 0, RING_WAYS * RING_STRIDE * sizeof(unsigned long long), h->stream);
+            if (h->curved)
+                dispatch<CSpd>(h->N, h->stream, u, (const double*)h->d_Ja, (const double*)h->d_ijn, (int)h->E, h->opts.gamma,
+                               h->d_step, ring_slot(h, from));
+            else
             dispatch<Spd>(h->N, h->stream, u, (const double*)h->d_inv_jac, (int)h->E, h->opts.gamma, h->d_step, true, false,
                           indicator_args(h), ring_slot(h, from));
         }
@@ -669,8 +706,8 @@ void enqueue_step(tlw_handle* h, int from, cudaEvent_t after_dt = nullptr, const
     if (fused) {
         if (!begin_in_volume(h))
             launch_dependent(h->stream, begin_step_kernel, 1, 1, 0, h->d_step, ring_slot(h, from), ring_slot(h, 1 - from), h->n);
-    } else if (h->parabolic) par_finalize_dt_kernel<<<1, 1, 0, h->stream>>>(h->d_step, h->d_visc, h->N, h->curved ? 1 : 0);
-    else finalize_dt_kernel<<<1, 1, 0, h->stream>>>(h->d_step, h->n);
+    } else if (h->parabolic) launch_dependent(h->stream, par_finalize_dt_kernel, 1, 1, 0, h->d_step, h->d_visc, h->N, h->curved ? 1 : 0);
+    else launch_dependent(h->stream, finalize_dt_kernel, 1, 1, 0, h->d_step, h->n);
     if (after_dt) cudaEventRecord(after_dt, h->stream);
     const double* dtp = &h->d_step->dt;
     if (h->opts.time_discretization == TLW_LW) {
@@ -1086,10 +1123,23 @@ int tlw_set_curved_mesh(tlw_handle* h, int64_t n_elements, const double* contrav
     if ((rc = up_i(h->d_cp, cp)) || (rc = up_i(h->d_cs, cs)) || (rc = up_i(h->d_cf, cf))) return rc;
     h->color_off = off;
     h->face_used.assign((size_t)n_elements * 4, 0);
+    constexpr int unset = std::numeric_limits<int>::min();
+    std::vector<int2> cnbr((size_t)n_elements * 4, int2{unset, 0});
     for (const Ifc& f : all) {
-        h->face_used[(size_t)f.p * 4 + (f.code & 3)] = 1;
-        h->face_used[(size_t)f.s * 4 + ((f.code >> 2) & 3)] = 1;
+        const int pf = f.code & 3, sf = (f.code >> 2) & 3, rv = (f.code >> 4) & 1;
+        h->face_used[(size_t)f.p * 4 + pf] = 1;
+        h->face_used[(size_t)f.s * 4 + sf] = 1;
+        cnbr[(size_t)f.p * 4 + pf] = int2{f.s, sf | rv << 2};
+        cnbr[(size_t)f.s * 4 + sf] = int2{f.p, pf | rv << 2 | 8};
     }
+    if (4 * n_elements == 2 * n_interfaces) {
+        TLW_CUDA(h, cudaMalloc(&h->d_cnbr, cnbr.size() * sizeof(int2)));
+        TLW_CUDA(h, upload_on(h->stream, h->d_cnbr, cnbr.data(), cnbr.size() * sizeof(int2)));
+    } else {
+        h->cnbr_open = std::move(cnbr);
+    }
+    TLW_CUDA(h, cudaMalloc(&h->d_slots, (size_t)n_elements * 2 * sizeof(unsigned long long)));
+    h->slots_valid = false;
     h->nx = h->ny = 0;
     h->nb = 0; h->nbx = h->nby = 0;
     const size_t sd = state_doubles(h), td = trace_doubles(h);
@@ -1594,6 +1644,19 @@ int tlw_set_curved_boundaries(tlw_handle* h, int64_t n_boundaries, const int64_t
     dfree(h->d_wall);
     h->ncb = (int)n_boundaries;
     h->ncbx = (int)be[0].size();
+    if (!h->cnbr_open.empty()) {
+        dfree(h->d_cnbr);
+        std::vector<int2> cnbr(h->cnbr_open);
+        for (int c = 0, k = 0; c < 2; ++c)
+            for (size_t i = 0; i < be[c].size(); ++i, ++k) cnbr[(size_t)be[c][i] * 4 + bf[c][i]] = int2{-k - 1, 0};
+        bool open = false;
+        for (const int2& f : cnbr) open = open || f.x == std::numeric_limits<int>::min();
+        if (!open) {
+            TLW_CUDA(h, cudaMalloc(&h->d_cnbr, cnbr.size() * sizeof(int2)));
+            TLW_CUDA(h, upload_on(h->stream, h->d_cnbr, cnbr.data(), cnbr.size() * sizeof(int2)));
+        }
+    }
+    h->slots_valid = false;
     h->bnd_dirichlet = dirichlet;
     h->have_bdata = false;
     dfree(h->d_levels); dfree(h->d_now);

@@ -13,7 +13,9 @@ constexpr unsigned STATUS_NONADMISSIBLE = 1u;   // sqrt of a negative number (re
 // Programmatic dependent launch: a kernel launched by launch_dependent may start before the one in front of it on its
 // stream has ended. It waits here, before its first access to global memory; the kernel in front lets it start once all
 // of its own CTAs have (dependents_may_start), so that the launch latency and the CTA set-up of a chain of short kernels
-// overlap. Both are no-ops in a kernel launched the ordinary way.
+// overlap. Both are no-ops in a kernel launched the ordinary way. A kernel whose CTAs fill the SM's shared memory does not
+// call dependents_may_start: what started beside it would run on with the small L1 it leaves (the blast on the warped
+// 150 x 133 mesh, 48 KB a CTA: 126 us a step with the interfaces started early, 115 without).
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <class... P, class... A>
@@ -165,6 +167,13 @@ __device__ __forceinline__ void node_speeds(double gamma, const double* x, unsig
     const double c = checked_sqrt(gamma * p * ir, status);
     l1 = fabs(v1) + c;
     l2 = fabs(v2) + c;
+}
+
+// the contravariant speeds of a curvilinear mesh's node from its |v1| + c and |v2| + c
+__device__ __forceinline__ void curved_speeds(const double* J, double inv_jac, double& l1, double& l2) {
+    const double ij = fabs(inv_jac), a = l1, b = l2;
+    l1 = fabs(J[0] * a + J[1] * b) * ij;
+    l2 = fabs(J[2] * a + J[3] * b) * ij;
 }
 
 // Per-element CFL slots written by the kernels that produce the final values of a step (plain LW on a

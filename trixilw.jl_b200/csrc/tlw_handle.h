@@ -173,6 +173,10 @@ struct tlw_handle {
     int *d_cp = nullptr, *d_cs = nullptr, *d_cf = nullptr;   // interfaces sorted by colour
     std::vector<int> color_off;             // colour c covers [color_off[c], color_off[c + 1])
     std::vector<signed char> face_used;     // [e * 4 + face]: 1 when an interface covers the face
+    // what lies across each face (curved_surface_kernel), when every face has an interface or a boundary; the host copy
+    // of a mesh whose interfaces leave faces open, for its boundaries
+    int2* d_cnbr = nullptr;
+    std::vector<int2> cnbr_open;
     // boundary faces of the curvilinear mesh: xi faces [0, ncbx), then eta faces [ncbx, ncb); element, face,
     // slip-wall kind and the boundary's index in the caller's order (wall data)
     int ncb = 0, ncbx = 0;

@@ -74,14 +74,14 @@ struct LaunchImpl {
     static void volume_src_on(cudaStream_t s, int stage, int mode, const VolArgs& a, int grid) {
         const size_t lw = C::lw_bytes(), md = C::mdrk_bytes();
         if (stage == TLW_STAGE_LW) {
-            if (mode == MODE_RHS) lw_volume_kernel<N, MODE_RHS, false, 0, CURVED, false, false, 0, true><<<grid, C::THREADS, lw, s>>>(a);
-            else lw_volume_kernel<N, MODE_STEP, false, 0, CURVED, false, false, 0, true><<<grid, C::THREADS, lw, s>>>(a);
+            if (mode == MODE_RHS) launch_dependent(s, lw_volume_kernel<N, MODE_RHS, false, 0, CURVED, false, false, 0, true>, grid, C::THREADS, lw, a);
+            else launch_dependent(s, lw_volume_kernel<N, MODE_STEP, false, 0, CURVED, false, false, 0, true>, grid, C::THREADS, lw, a);
         } else if (stage == TLW_STAGE_MDRK1) {
-            if (mode == MODE_RHS) mdrk1_volume_kernel<N, MODE_RHS, false, CURVED, 0, true><<<grid, C::THREADS, md, s>>>(a);
-            else mdrk1_volume_kernel<N, MODE_STEP, false, CURVED, 0, true><<<grid, C::THREADS, md, s>>>(a);
+            if (mode == MODE_RHS) launch_dependent(s, mdrk1_volume_kernel<N, MODE_RHS, false, CURVED, 0, true>, grid, C::THREADS, md, a);
+            else launch_dependent(s, mdrk1_volume_kernel<N, MODE_STEP, false, CURVED, 0, true>, grid, C::THREADS, md, a);
         } else {
-            if (mode == MODE_RHS) mdrk2_volume_kernel<N, MODE_RHS, false, CURVED, 0, true><<<grid, C::THREADS, md, s>>>(a);
-            else mdrk2_volume_kernel<N, MODE_STEP, false, CURVED, 0, true><<<grid, C::THREADS, md, s>>>(a);
+            if (mode == MODE_RHS) launch_dependent(s, mdrk2_volume_kernel<N, MODE_RHS, false, CURVED, 0, true>, grid, C::THREADS, md, a);
+            else launch_dependent(s, mdrk2_volume_kernel<N, MODE_STEP, false, CURVED, 0, true>, grid, C::THREADS, md, a);
         }
     }
     static void volume_src(cudaStream_t s, int stage, int mode, const VolArgs& a, int grid) {
@@ -114,14 +114,14 @@ struct LaunchImpl {
     static void curved_sc(cudaStream_t s, int stage, int mode, const VolArgs& a, int grid) {
         const size_t sm = C::mdrk_bytes(true, REC), lw = C::lw_bytes(true, REC);
         if (stage == TLW_STAGE_MDRK1) {
-            if (mode == MODE_RHS) mdrk1_volume_kernel<N, MODE_RHS, true, true, REC><<<grid, C::THREADS, sm, s>>>(a);
-            else mdrk1_volume_kernel<N, MODE_STEP, true, true, REC><<<grid, C::THREADS, sm, s>>>(a);
+            if (mode == MODE_RHS) launch_dependent(s, mdrk1_volume_kernel<N, MODE_RHS, true, true, REC>, grid, C::THREADS, sm, a);
+            else launch_dependent(s, mdrk1_volume_kernel<N, MODE_STEP, true, true, REC>, grid, C::THREADS, sm, a);
         } else if (stage == TLW_STAGE_MDRK2) {
-            if (mode == MODE_RHS) mdrk2_volume_kernel<N, MODE_RHS, true, true, REC><<<grid, C::THREADS, sm, s>>>(a);
-            else mdrk2_volume_kernel<N, MODE_STEP, true, true, REC><<<grid, C::THREADS, sm, s>>>(a);
+            if (mode == MODE_RHS) launch_dependent(s, mdrk2_volume_kernel<N, MODE_RHS, true, true, REC>, grid, C::THREADS, sm, a);
+            else launch_dependent(s, mdrk2_volume_kernel<N, MODE_STEP, true, true, REC>, grid, C::THREADS, sm, a);
         } else {
-            if (mode == MODE_RHS) lw_volume_kernel<N, MODE_RHS, true, 0, true, false, false, REC><<<grid, C::THREADS, lw, s>>>(a);
-            else lw_volume_kernel<N, MODE_STEP, true, 0, true, false, false, REC><<<grid, C::THREADS, lw, s>>>(a);
+            if (mode == MODE_RHS) launch_dependent(s, lw_volume_kernel<N, MODE_RHS, true, 0, true, false, false, REC>, grid, C::THREADS, lw, a);
+            else launch_dependent(s, lw_volume_kernel<N, MODE_STEP, true, 0, true, false, false, REC>, grid, C::THREADS, lw, a);
         }
     }
     template <int REC>
@@ -181,15 +181,15 @@ struct LaunchImpl {
         if (a.metrics) {   // curvilinear mesh (LW or MDRK, FR volume integral)
             const size_t md = C::mdrk_bytes();
             if (stage == TLW_STAGE_MDRK1) {
-                if (mode == MODE_RHS) mdrk1_volume_kernel<N, MODE_RHS, false, true><<<grid, C::THREADS, md, s>>>(a);
-                else mdrk1_volume_kernel<N, MODE_STEP, false, true><<<grid, C::THREADS, md, s>>>(a);
+                if (mode == MODE_RHS) launch_dependent(s, mdrk1_volume_kernel<N, MODE_RHS, false, true>, grid, C::THREADS, md, a);
+                else launch_dependent(s, mdrk1_volume_kernel<N, MODE_STEP, false, true>, grid, C::THREADS, md, a);
             } else if (stage == TLW_STAGE_MDRK2) {
-                if (mode == MODE_RHS) mdrk2_volume_kernel<N, MODE_RHS, false, true><<<grid, C::THREADS, md, s>>>(a);
-                else mdrk2_volume_kernel<N, MODE_STEP, false, true><<<grid, C::THREADS, md, s>>>(a);
+                if (mode == MODE_RHS) launch_dependent(s, mdrk2_volume_kernel<N, MODE_RHS, false, true>, grid, C::THREADS, md, a);
+                else launch_dependent(s, mdrk2_volume_kernel<N, MODE_STEP, false, true>, grid, C::THREADS, md, a);
             } else if (mode == MODE_RHS) {
-                lw_volume_kernel<N, MODE_RHS, false, 0, true><<<grid, C::THREADS, C::lw_bytes(), s>>>(a);
+                launch_dependent(s, lw_volume_kernel<N, MODE_RHS, false, 0, true>, grid, C::THREADS, C::lw_bytes(), a);
             } else {
-                lw_volume_kernel<N, MODE_STEP, false, 0, true><<<grid, C::THREADS, C::lw_bytes(), s>>>(a);
+                launch_dependent(s, lw_volume_kernel<N, MODE_STEP, false, 0, true>, grid, C::THREADS, C::lw_bytes(), a);
             }
             return;
         }
@@ -199,7 +199,7 @@ struct LaunchImpl {
     static void interfaces(cudaStream_t s, const SurfArgs& a) {
         const long long threads = (long long)a.count * (N + 1);
         if (threads == 0) return;
-        interface_kernel<N><<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(a);
+        launch_dependent(s, interface_kernel<N>, (unsigned)((threads + 127) / 128), 128, 0, a);
     }
     static void surfaces(cudaStream_t s, const SurfArgs& a, const BndArgs& b, const MortarArgs& m) {
         if (a.E <= 0) return;
@@ -223,7 +223,22 @@ struct LaunchImpl {
             using P = ParCfg<N>;
             const int grid = (E + P::EB - 1) / P::EB;
             const double iwf = h->h_basis.inv_w_first, iwl = h->h_basis.inv_w_last;
-            if (h->curved) {
+            GradFaces gf{};
+            gf.nbr = h->d_nbr;
+            gf.cnbr = h->d_cnbr;
+            gf.boundary = h->d_cbi;
+            gf.wall_kind = h->d_wkind;
+            gf.wall = h->d_wall;
+            gf.gamma = h->opts.gamma;
+            gf.inv_w_first = iwf;
+            gf.inv_w_last = iwl;
+            if (h->curved && h->d_cnbr) {
+                launch_dependent(s, grad_volume_kernel<N, true, true>, grid, P::THREADS, 0, u, h->d_ijn, E, h->d_gx, h->d_gy,
+                                 h->d_Ja, gf);
+            } else if (!h->curved && h->d_nbr) {
+                launch_dependent(s, grad_volume_kernel<N, false, true>, grid, P::THREADS, 0, u, h->d_inv_jac, E, h->d_gx,
+                                 h->d_gy, nullptr, gf);
+            } else if (h->curved) {
                 grad_volume_kernel<N, true><<<grid, P::THREADS, 0, s>>>(u, h->d_ijn, E, h->d_gx, h->d_gy, h->d_Ja);
                 for (size_t c = 0; c + 1 < h->color_off.size(); ++c) {
                     const int b = h->color_off[c], cnt = h->color_off[c + 1] - b;
@@ -270,11 +285,11 @@ struct LaunchImpl {
             if (h->curved) {
                 pa.inv_jac = h->d_ijn;
                 pa.metrics = h->d_Ja;
-                if (mode == MODE_RHS) par_volume_kernel<N, MODE_RHS, true><<<grid, P::THREADS, P::smem_bytes(), s>>>(pa);
-                else par_volume_kernel<N, MODE_STEP, true><<<grid, P::THREADS, P::smem_bytes(), s>>>(pa);
+                if (mode == MODE_RHS) launch_dependent(s, par_volume_kernel<N, MODE_RHS, true>, grid, P::THREADS, P::smem_bytes(), pa);
+                else launch_dependent(s, par_volume_kernel<N, MODE_STEP, true>, grid, P::THREADS, P::smem_bytes(), pa);
             } else {
-                if (mode == MODE_RHS) par_volume_kernel<N, MODE_RHS><<<grid, P::THREADS, P::smem_bytes(), s>>>(pa);
-                else par_volume_kernel<N, MODE_STEP><<<grid, P::THREADS, P::smem_bytes(), s>>>(pa);
+                if (mode == MODE_RHS) launch_dependent(s, par_volume_kernel<N, MODE_RHS>, grid, P::THREADS, P::smem_bytes(), pa);
+                else launch_dependent(s, par_volume_kernel<N, MODE_STEP>, grid, P::THREADS, P::smem_bytes(), pa);
             }
         }
     }
@@ -284,8 +299,8 @@ struct LaunchImpl {
             const int grid = (E + MsCfg<N>::ELEMS - 1) / MsCfg<N>::ELEMS;
             if (h->curved) {
                 // the CFL maximum of the curvilinear max_dt and the parabolic max_dt's own maxima, one pass
-                curved_par_speed_kernel<N><<<grid, MS_THREADS, 0, s>>>(u, h->d_Ja, h->d_ijn, E, ns_params(h),
-                                                                        h->d_step, h->d_visc, h->d_visc + 1);
+                launch_dependent(s, curved_par_speed_kernel<N>, grid, MS_THREADS, 0, u, h->d_Ja, h->d_ijn, E, ns_params(h),
+                                 h->d_step, h->d_visc, h->d_visc + 1);
             } else {
                 par_speed_kernel<N><<<grid, MS_THREADS, 0, s>>>(u, h->d_inv_jac, E, ns_params(h), h->d_step,
                                                                  h->d_visc, &h->d_step->max_bits);
@@ -312,27 +327,36 @@ struct LaunchImpl {
     static void curved_interfaces(cudaStream_t s, const CurvedSurfArgs& a) {
         const long long threads = (long long)a.count * (N + 1);
         if (threads == 0) return;
-        curved_interface_kernel<N><<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(a);
+        launch_dependent(s, curved_interface_kernel<N>, (unsigned)((threads + 127) / 128), 128, 0, a);
+    }
+    static void curved_surfaces(cudaStream_t s, const CurvedSurfArgs& a, const CurvedBndArgs& b) {
+        if (a.E <= 0) return;
+        using C = SurfCfg<N>;
+        const unsigned grid = (unsigned)((a.E + C::EB - 1) / C::EB);
+        const bool plain = !b.elem && !a.alpha && !a.tG && !a.tFv;
+        if (plain) launch_dependent(s, curved_surface_kernel<N, true>, grid, C::THREADS, 0, a, b);
+        else launch_dependent(s, curved_surface_kernel<N, false>, grid, C::THREADS, 0, a, b);
     }
     static void curved_speed(cudaStream_t s, const double* u, const double* Ja, const double* ij, int E, double g,
-                             StepState* st) {
+                             StepState* st, unsigned long long* target) {
         if (E == 0) return;
-        curved_max_speed_kernel<N><<<(E + MsCfg<N>::ELEMS - 1) / MsCfg<N>::ELEMS, MS_THREADS, 0, s>>>(u, Ja, ij, E, g, st);
+        launch_dependent(s, curved_max_speed_kernel<N>, (E + MsCfg<N>::ELEMS - 1) / MsCfg<N>::ELEMS, MS_THREADS, 0, u, Ja, ij, E, g,
+                         st, target);
     }
     static void boundaries(cudaStream_t s, const BndArgs& a) {
         const long long threads = (long long)a.count * (N + 1);
         if (threads == 0) return;
-        boundary_kernel<N><<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(a);
+        launch_dependent(s, boundary_kernel<N>, (unsigned)((threads + 127) / 128), 128, 0, a);
     }
     // speed: CFL reduction; ind: Hennemann-Gassner indicator (both read u once)
     static void max_speed(cudaStream_t s, const double* u, const double* ij, int E, double gamma, StepState* st,
                           bool speed, bool ind, const IndicatorArgs& ia, BatchSpeedArgs bs = BatchSpeedArgs{}) {
         if (E == 0) return;
         const int grid = (E + MsCfg<N>::ELEMS - 1) / MsCfg<N>::ELEMS;
-        if (speed && ind && ia.metrics) max_speed_kernel<N, true, true, true><<<grid, MS_THREADS, 0, s>>>(u, ij, E, gamma, st, ia, bs);
-        else if (speed && ind) max_speed_kernel<N, true, true><<<grid, MS_THREADS, 0, s>>>(u, ij, E, gamma, st, ia, bs);
-        else if (speed) max_speed_kernel<N, true, false><<<grid, MS_THREADS, 0, s>>>(u, ij, E, gamma, st, ia, bs);
-        else if (ind) max_speed_kernel<N, false, true><<<grid, MS_THREADS, 0, s>>>(u, ij, E, gamma, st, ia, bs);
+        if (speed && ind && ia.metrics) launch_dependent(s, max_speed_kernel<N, true, true, true>, grid, MS_THREADS, 0, u, ij, E, gamma, st, ia, bs);
+        else if (speed && ind) launch_dependent(s, max_speed_kernel<N, true, true>, grid, MS_THREADS, 0, u, ij, E, gamma, st, ia, bs);
+        else if (speed) launch_dependent(s, max_speed_kernel<N, true, false>, grid, MS_THREADS, 0, u, ij, E, gamma, st, ia, bs);
+        else if (ind) launch_dependent(s, max_speed_kernel<N, false, true>, grid, MS_THREADS, 0, u, ij, E, gamma, st, ia, bs);
     }
 };
 
@@ -379,12 +403,15 @@ template <int N> void Launch<N>::curved_interfaces(cudaStream_t s, const CurvedS
 template <int N> void Launch<N>::curved_boundaries(cudaStream_t s, const CurvedBndArgs& a) {
     const long long threads = (long long)a.count * (N + 1);
     if (threads == 0) return;
-    curved_boundary_kernel<N><<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(a);
+    launch_dependent(s, curved_boundary_kernel<N>, (unsigned)((threads + 127) / 128), 128, 0, a);
 }
 template <int N>
 void Launch<N>::curved_speed(cudaStream_t s, const double* u, const double* Ja, const double* ij, int E, double g,
-                             StepState* st) {
-    LaunchImpl<N>::curved_speed(s, u, Ja, ij, E, g, st);
+                             StepState* st, unsigned long long* target) {
+    LaunchImpl<N>::curved_speed(s, u, Ja, ij, E, g, st, target);
+}
+template <int N> void Launch<N>::curved_surfaces(cudaStream_t s, const CurvedSurfArgs& a, const CurvedBndArgs& b) {
+    LaunchImpl<N>::curved_surfaces(s, a, b);
 }
 template <int N> void Launch<N>::halo(cudaStream_t s, const HaloArgs& a, bool pack) {
     const long long threads = (long long)a.count * (N + 1);

@@ -33,8 +33,10 @@ struct Launch {
     static void curved_mortars(cudaStream_t s, const CurvedMortarArgs& a);
     static void curved_interfaces(cudaStream_t s, const CurvedSurfArgs& a);
     static void curved_boundaries(cudaStream_t s, const CurvedBndArgs& a);
+    // all faces of a curvilinear mesh whose every face is an interface or a boundary, one pass
+    static void curved_surfaces(cudaStream_t s, const CurvedSurfArgs& a, const CurvedBndArgs& b);
     static void curved_speed(cudaStream_t s, const double* u, const double* Ja, const double* ij, int E, double g,
-                             StepState* st);
+                             StepState* st, unsigned long long* target = nullptr);
     static void halo(cudaStream_t s, const HaloArgs& a, bool pack);
     static void limiter(cudaStream_t s, const LimiterArgs& a);
     static void max_speed(cudaStream_t s, const double* u, const double* ij, int E, double gamma, StepState* st,

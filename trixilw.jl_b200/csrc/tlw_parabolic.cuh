@@ -63,6 +63,10 @@ struct ParCfg {
     static constexpr int EB = VolCfg<N>::EB;
     static constexpr int THREADS = VolCfg<N>::THREADS;
     static constexpr int DEPTH = N >= 4 ? 4 : 3;
+#ifndef TLW_PAR_MB
+#define TLW_PAR_MB 3
+#endif
+    static constexpr int MIN_BLOCKS = THREADS <= 128 ? TLW_PAR_MB : 1;
     static constexpr int TILE = NV * EB * nn;   // 4 values per node of the CTA
     // D, Dhat; contraction tiles X, Y, W; perturbed states P (4) and their gradients GX, GY (4 + 4)
     static constexpr size_t smem_bytes() { return (size_t)(2 * nn + 15 * TILE) * sizeof(double); }
@@ -72,15 +76,34 @@ struct ParCfg {
 // (metrics [4, i, j, e], inv_jac per node) the two reference derivatives r_xi, r_eta mix as
 // gx = J^{-1} (Ja^1_1 r_xi + Ja^2_1 r_eta), gy = J^{-1} (Ja^1_2 r_xi + Ja^2_2 r_eta) (Trixi calc_gradient! for
 // P4estMesh{2})
-template <int N, bool CURVED = false>
+// The face terms of grad_volume_kernel<..., FACES>: what lies across each face (TreeMesh: nbr as surface_kernel takes it;
+// curvilinear: cnbr as curved_surface_kernel does) and the walls
+struct GradFaces {
+    const int* nbr;
+    const int2* cnbr;
+    const int* boundary;      // curvilinear: the caller's index of sorted boundary k (wall data)
+    const int* wall_kind;
+    const double* wall;       // [3, l, B]
+    double gamma, inv_w_first, inv_w_last;
+};
+__device__ __forceinline__ void wall_value(double gamma, const double* ui, int kind, const double* w, double* uo);
+
+// FACES: the interface and boundary terms (BR1) as well, for a mesh whose every face has an interface or a boundary. They
+// take u alone, so the thread of a face node adds its own faces' lifts (the value u* of a face is the mean of both sides
+// or the wall's) before it stores the gradients: one launch instead of one per colour and boundary class, each of which
+// read and wrote the face nodes' gradients again (64 x 64 cavity, N = 4: five launches, 30 us, in one of 10).
+template <int N, bool CURVED = false, bool FACES = false>
 static __global__ void __launch_bounds__(VolCfg<N>::THREADS) grad_volume_kernel(const double* __restrict__ u,
                                                                               const double* __restrict__ inv_jac,
                                                                               int E, double* gx, double* gy,
-                                                                              const double* __restrict__ metrics = nullptr) {
+                                                                              const double* __restrict__ metrics = nullptr,
+                                                                              GradFaces gf = GradFaces{}) {
     using C = ParCfg<N>;
     constexpr int n = C::n, nn = C::nn, EB = C::EB;
     __shared__ double sU[NV * EB * nn];
     __shared__ double sDh[nn];
+    wait_for_previous();
+    dependents_may_start();
     for (int k = threadIdx.x; k < nn; k += blockDim.x) sDh[k] = c_tlw_Dhat[N][k];
     const int el = threadIdx.x / nn, node = threadIdx.x - (threadIdx.x / nn) * nn;
     const int i = node % n, j = node / n;
@@ -88,7 +111,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS) grad_volume_kernel(
     const bool active = el < EB && e < E;
     if (active) {
         double x[NV];
-        load4(u + ((size_t)e * nn + node) * NV, x);
+        load4w(u + ((size_t)e * nn + node) * NV, x);
 #pragma unroll
         for (int v = 0; v < NV; ++v) sU[(v * EB + el) * nn + node] = x[v];
     }
@@ -96,7 +119,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS) grad_volume_kernel(
     if (!active) return;
     const double ij = CURVED ? __ldg(inv_jac + (size_t)e * nn + node) : __ldg(inv_jac + e);
     double J[4] = {1.0, 0.0, 0.0, 1.0};
-    if (CURVED) load4(metrics + ((size_t)e * nn + node) * 4, J);
+    if (CURVED) load4w(metrics + ((size_t)e * nn + node) * 4, J);
     double ox[NV], oy[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
@@ -115,8 +138,47 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS) grad_volume_kernel(
             oy[v] = ij * sy;
         }
     }
-    store4(gx + ((size_t)e * nn + node) * NV, ox);
-    store4(gy + ((size_t)e * nn + node) * NV, oy);
+    if (FACES) {
+#pragma unroll
+        for (int d = 0; d < 2; ++d) {
+            const int a = d == 0 ? i : j, l = d == 0 ? j : i;
+            if (a != 0 && a != n - 1) continue;
+            const int f = 2 * d + (a == 0 ? 0 : 1);
+            const double sg = f & 1 ? 1.0 : -1.0, iw = f & 1 ? gf.inv_w_last : gf.inv_w_first;
+            double own[NV], us[NV];
+#pragma unroll
+            for (int v = 0; v < NV; ++v) own[v] = sU[(v * EB + el) * nn + node];
+            int other, node_there, boundary;
+            if (CURVED) {
+                const int2 nb = __ldg(gf.cnbr + 4 * (size_t)e + f);
+                other = nb.x;
+                node_there = face_node_index(n, nb.y & 3, (nb.y >> 2) & 1 ? n - 1 - l : l);
+                boundary = other < 0 ? __ldg(gf.boundary - other - 1) : 0;
+            } else {
+                other = __ldg(gf.nbr + 4 * (size_t)e + f);
+                node_there = face_node_index(n, f ^ 1, l);
+                boundary = -other - 1;
+            }
+            if (other >= 0) {
+                double x[NV];
+                load4w(u + ((size_t)other * nn + node_there) * NV, x);
+#pragma unroll
+                for (int v = 0; v < NV; ++v) us[v] = 0.5 * (own[v] + x[v]);
+            } else {
+                wall_value(gf.gamma, own, __ldg(gf.wall_kind + boundary), gf.wall + 3 * ((size_t)boundary * n + l), us);
+            }
+            const double c = iw * ij;
+            const double n0 = CURVED ? sg * (d == 0 ? J[0] : J[2]) * c : (d == 0 ? sg * c : 0.0);
+            const double n1 = CURVED ? sg * (d == 0 ? J[1] : J[3]) * c : (d == 0 ? 0.0 : sg * c);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                if (CURVED || d == 0) ox[v] = fma(n0, us[v], ox[v]);
+                if (CURVED || d == 1) oy[v] = fma(n1, us[v], oy[v]);
+            }
+        }
+    }
+    store4w(gx + ((size_t)e * nn + node) * NV, ox);
+    store4w(gy + ((size_t)e * nn + node) * NV, oy);
 }
 
 // gradient interface term (BR1): x-interfaces lift into gx, y-interfaces into gy (one launch for both)
@@ -158,6 +220,18 @@ static __global__ void __launch_bounds__(128) grad_interface_kernel(const double
     store4(pR, x);
 }
 
+// the wall value of boundary b at face node l (below)
+__device__ __forceinline__ void wall_value(double gamma, const double* ui, int kind, const double* w, double* uo) {
+    const double v1 = __ldg(w), v2 = __ldg(w + 1);
+    const double rho = ui[0];
+    const double p = kind == WALL_ADIABATIC ? (gamma - 1.0) * (ui[3] - 0.5 * (ui[1] * ui[1] + ui[2] * ui[2]) / rho)
+                                            : rho * __ldg(w + 2);
+    uo[0] = rho;
+    uo[1] = rho * v1;
+    uo[2] = rho * v2;
+    uo[3] = p / (gamma - 1.0) + 0.5 * rho * (v1 * v1 + v2 * v2);
+}
+
 // gradient boundary term (Trixi calc_boundary_flux_by_direction_gradient!): the wall value of
 // BoundaryConditionNavierStokesWall(NoSlip(v), Adiabatic | Isothermal) (compressible_navier_stokes_2d.jl:92-124),
 // prim2cons(rho_inner, v_wall, p) with p the inner pressure (adiabatic) or rho_inner T_wall (isothermal), is the
@@ -178,13 +252,8 @@ static __global__ void __launch_bounds__(128) grad_boundary_kernel(const double*
     const int node = dir == 1 ? n * l : dir == 2 ? (n - 1) + n * l : dir == 3 ? l : l + n * (n - 1);
     double ui[NV], x[NV];
     load4(u + ((size_t)e * nn + node) * NV, ui);
-    const double* w = wall + 3 * ((size_t)k * n + l);
-    const double v1 = __ldg(w), v2 = __ldg(w + 1);
-    const double rho = ui[0];
-    const double p = __ldg(wall_kind + k) == WALL_ADIABATIC
-                         ? (gamma - 1.0) * (ui[3] - 0.5 * (ui[1] * ui[1] + ui[2] * ui[2]) / rho)
-                         : rho * __ldg(w + 2);
-    const double uo[NV] = {rho, rho * v1, rho * v2, p / (gamma - 1.0) + 0.5 * rho * (v1 * v1 + v2 * v2)};
+    double uo[NV];
+    wall_value(gamma, ui, __ldg(wall_kind + k), wall + 3 * ((size_t)k * n + l), uo);
     double* g = (dir <= 2 ? gx : gy) + ((size_t)e * nn + node) * NV;
     const double c = (dir % 2 == 0 ? inv_w_last : -inv_w_first) * __ldg(inv_jac + e);
     load4_rw(g, x);
@@ -255,13 +324,8 @@ static __global__ void __launch_bounds__(128) curved_grad_boundary_kernel(
     const int node = face_node_index(n, f, l);
     double ui[NV];
     load4(u + ((size_t)e * nn + node) * NV, ui);
-    const double* w = wall + 3 * ((size_t)b * n + l);
-    const double v1 = __ldg(w), v2 = __ldg(w + 1);
-    const double rho = ui[0];
-    const double p = __ldg(wall_kind + b) == WALL_ADIABATIC
-                         ? (gamma - 1.0) * (ui[3] - 0.5 * (ui[1] * ui[1] + ui[2] * ui[2]) / rho)
-                         : rho * __ldg(w + 2);
-    const double uo[NV] = {rho, rho * v1, rho * v2, p / (gamma - 1.0) + 0.5 * rho * (v1 * v1 + v2 * v2)};
+    double uo[NV];
+    wall_value(gamma, ui, __ldg(wall_kind + b), wall + 3 * ((size_t)b * n + l), uo);
     curved_grad_lift(metrics, inv_jac, n, e, f, node, uo, (f & 1) ? inv_w_last : inv_w_first, gx, gy);
 }
 
@@ -304,7 +368,7 @@ struct ParLW {
 // the node's J^{-1} and its gradient J^{-1} (Ja^1_d D_xi d_m + Ja^2_d D_eta d_m) (src/solvers/dgsem_p4est/
 // dg_2d_parabolic.jl:51-104, 641-1787); the face traces are the contravariant fluxes along the face direction.
 template <int N, int MODE, bool CURVED = false>
-static __global__ void __launch_bounds__(ParCfg<N>::THREADS, 1) par_volume_kernel(ParArgs a) {
+static __global__ void __launch_bounds__(ParCfg<N>::THREADS, ParCfg<N>::MIN_BLOCKS) par_volume_kernel(ParArgs a) {
     using C = ParCfg<N>;
     using K = ParLW<C::DEPTH>;
     constexpr int n = C::n, nn = C::nn, EB = C::EB, DEPTH = C::DEPTH, TILE = C::TILE;
@@ -317,6 +381,8 @@ static __global__ void __launch_bounds__(ParCfg<N>::THREADS, 1) par_volume_kerne
     double* P = W + TILE;          // [q][v] planes: P + q * TILE
     double* GX = P + 4 * TILE;
     double* GY = GX + 4 * TILE;
+    wait_for_previous();
+    dependents_may_start();
     for (int k = threadIdx.x; k < nn; k += blockDim.x) {
         sD[k] = c_tlw_D[N][k];
         sDh[k] = c_tlw_Dhat[N][k];
@@ -349,12 +415,12 @@ static __global__ void __launch_bounds__(ParCfg<N>::THREADS, 1) par_volume_kerne
     double u[NV] = {1.0, 0.0, 0.0, 2.5}, gx[NV] = {0, 0, 0, 0}, gy[NV] = {0, 0, 0, 0};
     double ij = 1.0, J[4] = {1.0, 0.0, 0.0, 1.0};
     if (active) {
-        load4(a.u + ((size_t)e * nn + node) * NV, u);
-        load4(a.gx + ((size_t)e * nn + node) * NV, gx);
-        load4(a.gy + ((size_t)e * nn + node) * NV, gy);
+        load4w(a.u + ((size_t)e * nn + node) * NV, u);
+        load4w(a.gx + ((size_t)e * nn + node) * NV, gx);
+        load4w(a.gy + ((size_t)e * nn + node) * NV, gy);
         if (CURVED) {
             ij = __ldg(a.inv_jac + (size_t)e * nn + node);
-            load4(a.metrics + ((size_t)e * nn + node) * 4, J);
+            load4w(a.metrics + ((size_t)e * nn + node) * 4, J);
         } else {
             ij = __ldg(a.inv_jac + e);
         }
@@ -486,7 +552,7 @@ static __global__ void __launch_bounds__(ParCfg<N>::THREADS, 1) par_volume_kerne
 #pragma unroll
         for (int v = 0; v < NV; ++v) o[v] = fma(sc, acc[v], u[v]);
     }
-    store4(a.out + off, o);
+    store4w(a.out + off, o);
     if (CURVED) {
         // traces: the fluxes along the face's reference direction
 #pragma unroll
@@ -501,10 +567,15 @@ static __global__ void __launch_bounds__(ParCfg<N>::THREADS, 1) par_volume_kerne
         }
     }
     const size_t tb = (size_t)e * 4 * n * NV;
-    if (i == 0) { store4(a.tU + tb + (0 * n + j) * NV, U); store4(a.tF + tb + (0 * n + j) * NV, Fa); store4(a.tFv + tb + (0 * n + j) * NV, Fv); }
-    if (i == n - 1) { store4(a.tU + tb + (1 * n + j) * NV, U); store4(a.tF + tb + (1 * n + j) * NV, Fa); store4(a.tFv + tb + (1 * n + j) * NV, Fv); }
-    if (j == 0) { store4(a.tU + tb + (2 * n + i) * NV, U); store4(a.tF + tb + (2 * n + i) * NV, Ga); store4(a.tFv + tb + (2 * n + i) * NV, Gv); }
-    if (j == n - 1) { store4(a.tU + tb + (3 * n + i) * NV, U); store4(a.tF + tb + (3 * n + i) * NV, Ga); store4(a.tFv + tb + (3 * n + i) * NV, Gv); }
+    // (one store a direction, as store_traces)
+    if (i == 0 || i == n - 1) {
+        const size_t k = tb + ((i == 0 ? 0 : n) + j) * NV;
+        store4w(a.tU + k, U); store4w(a.tF + k, Fa); store4w(a.tFv + k, Fv);
+    }
+    if (j == 0 || j == n - 1) {
+        const size_t k = tb + ((j == 0 ? 2 * n : 3 * n) + i) * NV;
+        store4w(a.tU + k, U); store4w(a.tF + k, Ga); store4w(a.tFv + k, Gv);
+    }
 }
 
 // advective and viscous maxima for the parabolic dt: max_bits <- max_e J^{-1} (l1 + l2),
@@ -582,70 +653,62 @@ static __global__ void __launch_bounds__(MS_THREADS) curved_par_speed_kernel(con
     constexpr int n = N + 1, nn = n * n;
     constexpr int ELEMS = MsCfg<N>::ELEMS;
     __shared__ double c1s[ELEMS * nn], c2s[ELEMS * nn], l1s[ELEMS * nn], l2s[ELEMS * nn];
-    __shared__ double wmax[MS_THREADS / 32], wadv[MS_THREADS / 32], wvis[MS_THREADS / 32];
+    __shared__ double red[ELEMS], rad[ELEMS], wvis[MS_THREADS / 32];
+    wait_for_previous();
+    dependents_may_start();
     const int e0 = blockIdx.x * ELEMS;
     const int ne = min(ELEMS, E - e0);
-    const double gm1 = ns.gamma - 1.0;
     double vis = 0.0;
-    for (int k = threadIdx.x; k < ne * nn; k += MS_THREADS) {
-        const size_t node = (size_t)e0 * nn + k;
-        double x[NV], J[4];
-        load4w(u + node * NV, x);
-        load4w(metrics + node * 4, J);
-        const double ir = 1.0 / x[0];
-        const double v1 = x[1] * ir, v2 = x[2] * ir;
-        const double p = gm1 * (x[3] - 0.5 * (x[1] * v1 + x[2] * v2));
-        const double c = checked_sqrt(ns.gamma * p * ir, &s->status);
-        const double l1 = fabs(v1) + c, l2 = fabs(v2) + c;
-        const double ijn = fabs(__ldg(inv_jac + node));
-        c1s[k] = fabs(J[0] * l1 + J[1] * l2) * ijn;
-        c2s[k] = fabs(J[2] * l1 + J[3] * l2) * ijn;
+    auto one = [&](int k, const double* x, const double* J) {
+        double l1, l2;
+        node_speeds(ns.gamma, x, &s->status, l1, l2);
         l1s[k] = l1;
         l2s[k] = l2;
+        curved_speeds(J, __ldg(inv_jac + (size_t)e0 * nn + k), l1, l2);
+        c1s[k] = l1;
+        c2s[k] = l2;
         const double ij = __ldg(inv_jac + e0 + k / nn);
         vis = fmax(vis, ij * ij * fmax(4.0 * ns.mu / (3.0 * x[0]), ns.mu * ns.kappa / (x[0] * ns.Pr)));
-    }
-    __syncthreads();
-    double m = 0.0, ma = 0.0;
-    if (threadIdx.x < ne) {
-        double m1 = 0.0, m2 = 0.0, ml1 = 0.0, ml2 = 0.0;
-        for (int k = 0; k < nn; ++k) {
-            m1 = fmax(m1, c1s[threadIdx.x * nn + k]);
-            m2 = fmax(m2, c2s[threadIdx.x * nn + k]);
-            ml1 = fmax(ml1, l1s[threadIdx.x * nn + k]);
-            ml2 = fmax(ml2, l2s[threadIdx.x * nn + k]);
+    };
+    for_nodes(ne * nn, [&](int k, int k2, bool both) {
+        double x[NV], y[NV], J[4], J2[4];
+        load4w(u + ((size_t)e0 * nn + k) * NV, x);
+        load4w(metrics + ((size_t)e0 * nn + k) * 4, J);
+        if (both) {
+            load4w(u + ((size_t)e0 * nn + k2) * NV, y);
+            load4w(metrics + ((size_t)e0 * nn + k2) * 4, J2);
         }
-        m = m1 + m2;
-        ma = __ldg(inv_jac + e0 + threadIdx.x) * (ml1 + ml2);
-    }
+        one(k, x, J);
+        if (both) one(k2, y, J2);
+    });
+    __syncthreads();
+    const int el = threadIdx.x / MsCfg<N>::LANES;
+    const double m = element_max<N>(c1s, ne) + element_max<N>(c2s, ne);
+    const double ma = (element_max<N>(l1s, ne) + element_max<N>(l2s, ne)) * (el < ne ? __ldg(inv_jac + e0 + el) : 0.0);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-        ma = fmax(ma, __shfl_xor_sync(0xffffffffu, ma, o));
-        vis = fmax(vis, __shfl_xor_sync(0xffffffffu, vis, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        wmax[threadIdx.x >> 5] = m;
-        wadv[threadIdx.x >> 5] = ma;
-        wvis[threadIdx.x >> 5] = vis;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double b = wmax[0], ba = wadv[0], bv = wvis[0];
-        for (int w = 1; w < MS_THREADS / 32; ++w) {
-            b = fmax(b, wmax[w]);
-            ba = fmax(ba, wadv[w]);
-            bv = fmax(bv, wvis[w]);
+    for (int o = 16; o > 0; o >>= 1) vis = fmax(vis, __shfl_xor_sync(0xffffffffu, vis, o));
+    if ((threadIdx.x & 31) == 0) wvis[threadIdx.x >> 5] = vis;
+    if (threadIdx.x % MsCfg<N>::LANES == 0) rad[el] = el < ne ? ma : 0.0;
+    const double b = cta_max<N>(red, m, ne);   // (its barrier publishes rad and wvis too)
+    if (threadIdx.x < 32) {
+        double ba = threadIdx.x < ELEMS ? rad[threadIdx.x] : 0.0, bv = threadIdx.x < MS_THREADS / 32 ? wvis[threadIdx.x] : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            ba = fmax(ba, __shfl_xor_sync(0xffffffffu, ba, o));
+            bv = fmax(bv, __shfl_xor_sync(0xffffffffu, bv, o));
         }
-        if (b > 0.0) atomicMax(&s->max_bits, (unsigned long long)__double_as_longlong(b));
-        if (ba > 0.0) atomicMax(adv_bits, (unsigned long long)__double_as_longlong(ba));
-        if (bv > 0.0) atomicMax(visc_bits, (unsigned long long)__double_as_longlong(bv));
+        if (threadIdx.x == 0) {
+            if (b > 0.0) atomicMax(&s->max_bits, (unsigned long long)__double_as_longlong(b));
+            if (ba > 0.0) atomicMax(adv_bits, (unsigned long long)__double_as_longlong(ba));
+            if (bv > 0.0) atomicMax(visc_bits, (unsigned long long)__double_as_longlong(bv));
+        }
     }
 }
 
 // dt = min(cfl 2 / (n lam_a), cfl / ((lam_a' + 2 (2N + 1) lam_v) 2 (2N + 1))), then the set_dt! clamp;
 // lam_a' = lam_a on a TreeMesh, visc_bits[1] (the parabolic max_dt's own advective maximum) when curved
 static __global__ void par_finalize_dt_kernel(StepState* s, unsigned long long* visc_bits, int N, int curved = 0) {
+    wait_for_previous();
     const double tiny = 4.9406564584124654e-324;
     double la = __longlong_as_double((long long)s->max_bits);
     double lv = __longlong_as_double((long long)visc_bits[0]);

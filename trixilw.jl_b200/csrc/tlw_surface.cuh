@@ -146,6 +146,8 @@ __device__ __forceinline__ void interface_node_flux(const SurfArgs& a, int orien
 template <int N>
 static __global__ void __launch_bounds__(256) interface_kernel(SurfArgs a) {
     constexpr int n = N + 1;
+    wait_for_previous();
+    dependents_may_start();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int k = t / n;
     const int l = t - k * n;
@@ -283,6 +285,8 @@ __device__ __forceinline__ void boundary_node_flux(const BndArgs& a, int k, int 
 template <int N>
 static __global__ void __launch_bounds__(128) boundary_kernel(BndArgs a) {
     constexpr int n = N + 1;
+    wait_for_previous();
+    dependents_may_start();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int kk = t / n;
     const int l = t - kk * n;
@@ -333,6 +337,63 @@ template <int N> struct SurfCfg {
     static constexpr int MIN_BLOCKS = THREADS <= 128 ? TLW_SURF_MINB : 5;
 };
 
+// The maxima of l1 and l2 over the NB phase-2 threads of each element (thread el2 * NB + b), in threads b = 0 and 1;
+// sF: shared memory of at least 2 * EB * NB doubles that nobody reads any more. Every thread of the CTA calls it.
+template <int NB, int EB>
+__device__ __forceinline__ void element_maxima(double* sF, int tid, int el2, int b, bool has2, double& l1, double& l2) {
+    if constexpr (32 % NB == 0) {
+        // NB aligned consecutive lanes of one warp: by shuffles
+#pragma unroll
+        for (int o = NB / 2; o > 0; o >>= 1) {
+            l1 = fmax(l1, __shfl_xor_sync(0xffffffffu, l1, o));
+            l2 = fmax(l2, __shfl_xor_sync(0xffffffffu, l2, o));
+        }
+    } else {
+        __syncthreads();
+        if (has2) {
+            sF[tid] = l1;
+            sF[EB * NB + tid] = l2;
+        }
+        __syncthreads();
+        double m = 0.0;
+        if (has2 && b < 2) {
+            const double* p = sF + b * EB * NB + el2 * NB;
+#pragma unroll
+            for (int k = 0; k < NB; ++k) m = fmax(m, p[k]);
+        }
+        // threads 0 and 1 of an element are neighbouring lanes (NB is even): both get both maxima
+        const double other = __shfl_xor_sync(0xffffffffu, m, 1);
+        l1 = b == 0 ? m : other;
+        l2 = b == 0 ? other : m;
+    }
+}
+
+// The end of a step's last surface pass: the warp's largest m (bits of a non-negative double) into the partial maxima
+// of the next step, one atomic per warp; block 0 moves the step state's t and step count on (advance).
+__device__ __forceinline__ void keep_cfl_maximum(unsigned long long m, unsigned long long* cfl_max, StepState* advance,
+                                                 int tid) {
+    // the largest of the warp's 64-bit words: the largest upper half, then the largest lower half below it
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(m >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(m >> 32) == hi ? (unsigned)m : 0u);
+    if ((tid & 31) == 0 && (hi | lo))
+        atomicMax(cfl_max + (blockIdx.x % RING_WAYS) * RING_STRIDE, (unsigned long long)hi << 32 | lo);
+    if (advance && blockIdx.x == 0 && tid == 0) {
+        const double t = advance->t;
+        if (!run_finished(t, advance->t_end)) {
+            advance->t = t + advance->dt;
+            advance->steps += 1;
+        }
+    }
+}
+// phase-2 thread b of an element: its face node (bottom row, top row, left column, right column)
+template <int n>
+__device__ __forceinline__ void face_node_of_thread(int b, int& i, int& j) {
+    if (b < n) { i = b; j = 0; }
+    else if (b < 2 * n) { i = b - n; j = n - 1; }
+    else if (b < 3 * n - 2) { i = 0; j = b - 2 * n + 1; }
+    else { i = n - 1; j = b - 3 * n + 3; }
+}
+
 // nbr entry of a face on mortar m: NBR_MORTAR + (m << 2 | role), role 0 / 1: the element is the mortar's lower / upper
 // small one, 2: its large one (mortar and boundary ids stay below 2^27)
 constexpr int NBR_MORTAR = -(1 << 30), NBR_MORTAR_END = -(1 << 29);
@@ -369,10 +430,7 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, (BND || SC || MORT
     const int el2 = tid / NB, b = tid - el2 * NB, e2 = e0 + el2;
     const bool has2 = el2 < EB && e2 < a.E;
     int i2, j2;
-    if (b < n) { i2 = b; j2 = 0; }
-    else if (b < 2 * n) { i2 = b - n; j2 = n - 1; }
-    else if (b < 3 * n - 2) { i2 = 0; j2 = b - 2 * n + 1; }
-    else { i2 = n - 1; j2 = b - 3 * n + 3; }
+    face_node_of_thread<n>(b, i2, j2);
     double* o2 = a.out + ((size_t)e2 * n * n + i2 + n * j2) * NV;
     double x[NV];
     if (TLW_SURF_PREFETCH && has2) load4w_rw(o2, x);
@@ -440,32 +498,7 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, (BND || SC || MORT
         if (a.cfl_slots || a.cfl_max) node_speeds(a.gamma, x, a.status, l1, l2);
     }
     if (!a.cfl_slots && !a.cfl_max) return;
-    if constexpr (32 % NB == 0) {
-        // the element's NB phase-2 threads are NB aligned consecutive lanes of one warp: reduce by shuffles
-#pragma unroll
-        for (int o = NB / 2; o > 0; o >>= 1) {
-            l1 = fmax(l1, __shfl_xor_sync(0xffffffffu, l1, o));
-            l2 = fmax(l2, __shfl_xor_sync(0xffffffffu, l2, o));
-        }
-    } else {
-        // the element's face-node maxima through shared memory (NB consecutive threads per element)
-        __syncthreads();
-        if (has2) {
-            sF[tid] = l1;
-            sF[EB * NB + tid] = l2;
-        }
-        __syncthreads();
-        double m = 0.0;
-        if (has2 && b < 2) {
-            const double* p = sF + b * EB * NB + el2 * NB;
-#pragma unroll
-            for (int k = 0; k < NB; ++k) m = fmax(m, p[k]);
-        }
-        // threads 0 and 1 of an element are neighbouring lanes (NB is even): both get both maxima
-        const double other = __shfl_xor_sync(0xffffffffu, m, 1);
-        l1 = b == 0 ? m : other;
-        l2 = b == 0 ? other : m;
-    }
+    element_maxima<NB, EB>(sF, tid, el2, b, has2, l1, l2);
     if (a.cfl_slots) {
         if (has2 && b < 2)
             a.cfl_slots[(size_t)e2 * CFL_SLOTS + 2 + b] = (unsigned long long)__double_as_longlong(b ? l2 : l1);
@@ -474,19 +507,7 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, (BND || SC || MORT
     // the element's scaled speed with the interior maxima; one atomic per warp
     unsigned long long m = 0ull;
     if (has2 && b == 0) m = (unsigned long long)__double_as_longlong(ij * (fmax(l1, in.x) + fmax(l2, in.y)));
-    // the largest of the warp's 64-bit words: the largest upper half, then the largest lower half below it
-    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(m >> 32));
-    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(m >> 32) == hi ? (unsigned)m : 0u);
-    if ((tid & 31) == 0 && (hi | lo))
-        atomicMax(a.cfl_max + (blockIdx.x % RING_WAYS) * RING_STRIDE, (unsigned long long)hi << 32 | lo);
-    if (a.advance && blockIdx.x == 0 && tid == 0) {
-        StepState* s = a.advance;
-        const double t = s->t;
-        if (!run_finished(t, s->t_end)) {
-            s->t = t + s->dt;
-            s->steps += 1;
-        }
-    }
+    keep_cfl_maximum(m, a.cfl_max, a.advance, tid);
 }
 
 
@@ -498,7 +519,42 @@ template <int N>
 struct MsCfg {
     static constexpr int n = N + 1, nn = n * n;
     static constexpr int ELEMS = N >= 6 ? 16 : 32;   // elements per CTA (shared memory: 4 x ELEMS x nn doubles)
+    static constexpr int LANES = MS_THREADS / ELEMS;  // threads per element in the reduction over its nodes
 };
+
+// The passes over a state (CFL speeds, indicator, parabolic maxima): a CTA's threads take its nodes two at a time, so
+// that both nodes' records are in flight together, and LANES threads reduce each element. (With one node at a time and
+// one thread per element the pass of the 64 x 64 cavity, N = 4, took 9.4 us and the 256^2 Riemann one 26.5.)
+template <class F>
+__device__ __forceinline__ void for_nodes(int count, F&& two) {
+    for (int k = threadIdx.x; k < count; k += 2 * MS_THREADS) two(k, k + MS_THREADS, k + MS_THREADS < count);
+}
+// the maximum of x over an element's nodes, in all of its LANES threads
+template <int N>
+__device__ __forceinline__ double element_max(const double* x, int ne) {
+    using C = MsCfg<N>;
+    const int el = threadIdx.x / C::LANES, q = threadIdx.x % C::LANES;
+    double m = 0.0;
+    if (el < ne)
+        for (int k = q; k < C::nn; k += C::LANES) m = fmax(m, x[el * C::nn + k]);
+#pragma unroll
+    for (int o = C::LANES / 2; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    return m;
+}
+// the CTA's maximum of an element value (valid in the threads of element el < ne), in thread 0; red: ELEMS doubles
+template <int N>
+__device__ __forceinline__ double cta_max(double* red, double m, int ne) {
+    using C = MsCfg<N>;
+    const int el = threadIdx.x / C::LANES;
+    if (threadIdx.x % C::LANES == 0) red[el] = el < ne ? m : 0.0;
+    __syncthreads();
+    double r = threadIdx.x < C::ELEMS ? red[threadIdx.x] : 0.0;
+    if (threadIdx.x < 32) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_xor_sync(0xffffffffu, r, o));
+    }
+    return r;
+}
 
 struct IndicatorArgs {
     double* alpha_raw;       // [e] indicator before smoothing
@@ -534,36 +590,40 @@ static __global__ void __launch_bounds__(MS_THREADS) max_speed_kernel(const doub
     constexpr int ELEMS = MsCfg<N>::ELEMS;
     __shared__ double l1s[SPEED ? ELEMS * nn : 1], l2s[SPEED ? ELEMS * nn : 1];
     __shared__ double inds[IND ? ELEMS * nn : 1], tmps[IND ? ELEMS * nn : 1];
-    __shared__ double wmax[MS_THREADS / 32];
+    __shared__ double red[ELEMS];
+    wait_for_previous();
+    dependents_may_start();
     const int e0 = blockIdx.x * ELEMS;
     const int ne = min(ELEMS, E - e0);
     const double gm1 = gamma - 1.0;
-    for (int k = threadIdx.x; k < ne * nn; k += MS_THREADS) {
-        double x[NV];
-        load4w(u + ((size_t)e0 * nn + k) * NV, x);
-        if (SPEED && CSPEED) {
-            const size_t node = (size_t)e0 * nn + k;
-            double J[4], l1, l2;
-            load4w(ia.metrics + node * 4, J);
+    auto one = [&](int k, const double* x, const double* J) {
+        if (SPEED) {
+            double l1, l2;
             node_speeds(gamma, x, &s->status, l1, l2);
-            const double ij = fabs(__ldg(ia.inv_jac_node + node));
-            l1s[k] = fabs(J[0] * l1 + J[1] * l2) * ij;
-            l2s[k] = fabs(J[2] * l1 + J[3] * l2) * ij;
-        } else if (SPEED) {
-            node_speeds(gamma, x, &s->status, l1s[k], l2s[k]);
+            if (CSPEED) curved_speeds(J, __ldg(ia.inv_jac_node + (size_t)e0 * nn + k), l1, l2);
+            l1s[k] = l1;
+            l2s[k] = l2;
         }
         // indicator variable density_pressure = (gamma - 1)(rho rho_e - |rho v|^2 / 2)
         if (IND) inds[k] = gm1 * (x[0] * x[3] - 0.5 * (x[1] * x[1] + x[2] * x[2]));
-    }
+    };
+    for_nodes(ne * nn, [&](int k, int k2, bool both) {
+        double x[NV], y[NV], J[4], J2[4];
+        load4w(u + ((size_t)e0 * nn + k) * NV, x);
+        if (both) load4w(u + ((size_t)e0 * nn + k2) * NV, y);
+        if (SPEED && CSPEED) {
+            load4w(ia.metrics + ((size_t)e0 * nn + k) * 4, J);
+            if (both) load4w(ia.metrics + ((size_t)e0 * nn + k2) * 4, J2);
+        }
+        one(k, x, J);
+        if (both) one(k2, y, J2);
+    });
     __syncthreads();
     double m = 0.0;
-    if (SPEED && threadIdx.x < ne) {
-        double ml1 = 0.0, ml2 = 0.0;
-        for (int k = 0; k < nn; ++k) {
-            ml1 = fmax(ml1, l1s[threadIdx.x * nn + k]);
-            ml2 = fmax(ml2, l2s[threadIdx.x * nn + k]);
-        }
-        m = CSPEED ? ml1 + ml2 : __ldg(inv_jac + e0 + threadIdx.x) * (ml1 + ml2);
+    if (SPEED) {
+        m = element_max<N>(l1s, ne) + element_max<N>(l2s, ne);
+        const int el = threadIdx.x / MsCfg<N>::LANES;
+        if (!CSPEED && el < ne) m *= __ldg(inv_jac + e0 + el);
     }
     if (IND) {
         const int el = threadIdx.x >> 3, q = threadIdx.x & 7;
@@ -612,31 +672,28 @@ static __global__ void __launch_bounds__(MS_THREADS) max_speed_kernel(const doub
         }
     }
     if (SPEED && bs.inst) {
-        // batched: the (<= 32) element values sit in warp 0; one atomic per instance present
+        // batched: the (<= 32) element values in warp 0; one atomic per instance present
+        if (threadIdx.x % MsCfg<N>::LANES == 0) red[threadIdx.x / MsCfg<N>::LANES] = m;
+        __syncthreads();
         if (threadIdx.x < 32) {
             const int last = min(ne, 32) - 1;
             const int my = threadIdx.x <= last ? __ldg(bs.inst + e0 + threadIdx.x) : -1;
+            double r = threadIdx.x <= last ? red[threadIdx.x] : 0.0;
             const int first_inst = __shfl_sync(0xffffffffu, my, 0);
             const int last_inst = __shfl_sync(0xffffffffu, my, last);
             if (first_inst == last_inst) {
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-                if (threadIdx.x == 0 && m > 0.0)
-                    atomicMax(bs.inst_max + first_inst, (unsigned long long)__double_as_longlong(m));
-            } else if (threadIdx.x <= last && m > 0.0) {
-                atomicMax(bs.inst_max + my, (unsigned long long)__double_as_longlong(m));
+                for (int o = 16; o > 0; o >>= 1) r = fmax(r, __shfl_xor_sync(0xffffffffu, r, o));
+                if (threadIdx.x == 0 && r > 0.0)
+                    atomicMax(bs.inst_max + first_inst, (unsigned long long)__double_as_longlong(r));
+            } else if (threadIdx.x <= last && r > 0.0) {
+                atomicMax(bs.inst_max + my, (unsigned long long)__double_as_longlong(r));
             }
         }
     } else if (SPEED) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double b = wmax[0];
-            for (int w = 1; w < MS_THREADS / 32; ++w) b = fmax(b, wmax[w]);
-            if (b > 0.0) atomicMax(bs.target ? bs.target : &s->max_bits, (unsigned long long)__double_as_longlong(b));
-        }
+        const double b = cta_max<N>(red, m, ne);
+        if (threadIdx.x == 0 && b > 0.0)
+            atomicMax(bs.target ? bs.target : &s->max_bits, (unsigned long long)__double_as_longlong(b));
     }
 }
 
@@ -673,6 +730,8 @@ static __global__ void batch_finalize_dt_kernel(BatchTime b) {
 // independent of the order (max over non-negative doubles = max over their bit patterns)
 static __global__ void alpha_smooth_kernel(const int* __restrict__ left, const int* __restrict__ right, int count,
                                     const double* __restrict__ alpha_raw, double* alpha) {
+    wait_for_previous();
+    dependents_may_start();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const int l = __ldg(left + k), r = __ldg(right + k);
@@ -683,6 +742,7 @@ static __global__ void alpha_smooth_kernel(const int* __restrict__ left, const i
 
 // dt of the step from the CFL maximum in max_bits, and the time after it
 static __global__ void finalize_dt_kernel(StepState* s, int n) {
+    wait_for_previous();
     bool finished;
     const double dt = step_size(s, s->max_bits, n, finished);
     const double t = s->t;

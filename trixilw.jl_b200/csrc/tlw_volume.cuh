@@ -909,7 +909,7 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
 
     const int tid = threadIdx.x;
     wait_for_previous();
-    dependents_may_start();
+    if (!SC) dependents_may_start();
     prefetch_next<C>(a.u, 4, a.E, tid);
     if (CURVED) {
         prefetch_next<C>(a.metrics, 4, a.E, tid);
@@ -934,7 +934,7 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
     if constexpr (BEGIN) begin_step<C>(a, &s_dt, tid);
     else dt = a.inst ? a.dt[__ldg(a.inst + min(e, a.E - 1))] : *a.dt;
     // per-element maxima of the interior nodes' speeds for the next step's CFL (plain LW step only)
-    constexpr bool SLOTS = MODE == MODE_STEP && !SC && !CURVED;
+    constexpr bool SLOTS = MODE == MODE_STEP && !SC && !TE;
 
     // F[1..3] and G[2], G[3] are accumulated stage by stage; F[0], G[0] (the time averages of rho v1, rho v2) follow
     // from U, and G[1] = F[2]. The states carry gamma rho e as their last variable (see StencilSum).
@@ -1141,7 +1141,15 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
         }
         store_result<MODE>(a.out + ((size_t)e * nn + node) * NV, MODE == MODE_STEP ? s0 : -inverse_jacobian(), dt, acc, ub,
                            SRC ? Ssrc : nullptr, o);
-        if (SLOTS && a.cfl_slots && i > 0 && i < n - 1 && j > 0 && j < n - 1) node_speeds(a.gamma, o, a.status, l1, l2);
+        if (SLOTS && a.cfl_slots && i > 0 && i < n - 1 && j > 0 && j < n - 1) {
+            node_speeds(a.gamma, o, a.status, l1, l2);
+            if (CURVED) {
+                const size_t k = (size_t)e * nn + node;
+                double Jn[4];
+                load4w(a.metrics + k * 4, Jn);
+                curved_speeds(Jn, __ldg(a.inv_jac_node + k), l1, l2);
+            }
+        }
     }
     if (SLOTS && a.cfl_slots) write_interior_slots<N, C>(a, X, active, el, i, j, tid, l1, l2);
     if (TE) {
@@ -1237,7 +1245,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     double* UF = FVY + C::PLANES;      // curvilinear MUSCL: face values, 4 regions (left, right, down, up)
     const int tid = threadIdx.x;
     wait_for_previous();
-    dependents_may_start();
+    if (!SC) dependents_may_start();
     prefetch_next<C>(a.u, 4, a.E, tid);
     const int el = tid / nn;
     const int node = tid - el * nn;
@@ -1397,7 +1405,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     double* UF = FVY + C::PLANES;      // curvilinear MUSCL: face values, 4 regions (left, right, down, up)
     const int tid = threadIdx.x;
     wait_for_previous();
-    dependents_may_start();
+    if (!SC) dependents_may_start();
     prefetch_next<C>(a.u, 4, a.E, tid);
     if (COMPACT) {
         prefetch_next<C>(a.u_base, 4, a.E, tid);
@@ -1520,7 +1528,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     line_contract<N, C, true>(X, Y, tid);
     phase_sync<C>();
     // the step's final values: per-element CFL slots as the LW kernel writes them (plain TreeMesh MDRK step)
-    constexpr bool SLOTS = MODE == MODE_STEP && !SC && !CURVED;
+    constexpr bool SLOTS = MODE == MODE_STEP && !SC;
     double l1 = 0.0, l2 = 0.0;
     if (active) {
         double acc[NV];
@@ -1533,7 +1541,15 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
         if (MODE == MODE_STEP) load4w(a.u_base + ((size_t)e * nn + node) * NV, ub);
         store_result<MODE>(a.out + ((size_t)e * nn + node) * NV, MODE == MODE_STEP ? -dt * ij : -ij, dt, acc, ub,
                            SRC ? Ssrc : nullptr, o);
-        if (SLOTS && a.cfl_slots && i > 0 && i < n - 1 && j > 0 && j < n - 1) node_speeds(a.gamma, o, a.status, l1, l2);
+        if (SLOTS && a.cfl_slots && i > 0 && i < n - 1 && j > 0 && j < n - 1) {
+            node_speeds(a.gamma, o, a.status, l1, l2);
+            if (CURVED) {
+                const size_t k = (size_t)e * nn + node;
+                double Jn[4];
+                load4w(a.metrics + k * 4, Jn);
+                curved_speeds(Jn, __ldg(a.inv_jac_node + k), l1, l2);
+            }
+        }
     }
     if (SLOTS && a.cfl_slots) write_interior_slots<N, C>(a, X, active, el, i, j, tid, l1, l2);
 }
