@@ -86,3 +86,30 @@ def test_end_time_and_limiter_switch(oracle_mod, tl, td):
         _, t = o.steps(ref, 3, 0.2, t, 1e9, kind=0 if td == "lw" else 1, nthreads=NTH)
         assert integ.t == pytest.approx(t, rel=1e-13)
     assert np.all(rel_l2(integ.get_state(), ref) < 1e-12)
+
+
+@pytest.mark.parametrize("walls,N,td,cfl", [(True, 3, "lw", 2.5), (True, 4, "mdrk", 7.0), (False, 4, "lw", 3.5)])
+def test_run_that_ends_in_an_inadmissible_state(oracle_mod, tl, walls, N, td, cfl):
+    """A step far past the stability limit leaves negative pressures. Between walls the step itself is sound and the
+    next one, which has no wave speed, is not; a plain periodic mesh reports its new state at once; a recorded run
+    never steps from its last state and says nothing of it."""
+    mesh, semi = make(tl, 3, N, td, walls)
+    u = semi.compute_coefficients(0.0)
+    o = oracle_mod.Oracle(mesh, N)
+    if walls:
+        o.set_boundary_kinds(np.repeat(np.array([1, 1, 2, 2], dtype=np.int32), mesh.n_boundaries_per_direction))
+    ref = u.copy()
+    o.steps(ref, 1, cfl, 0.0, 1e9, kind=0 if td == "lw" else 1, nthreads=NTH)
+    q = ref.reshape(-1, 4)
+    pr = 0.4 * (q[:, 3] - 0.5 * (q[:, 1] ** 2 + q[:, 2] ** 2) / q[:, 0])
+    assert (pr * q[:, 0] < 0).any()
+    integ = tl.LWIntegrator(tl.semidiscretize(semi, semi.time_discretization, (0.0, 1e9)))
+    integ.set_state(u, 0.0)
+    integ.step(1, cfl)
+    if walls:
+        integ.sync_time()
+        integ.step(1, 0.2)
+    with pytest.raises(tl.DomainError):
+        integ.sync_time()
+    if not walls:
+        assert np.isfinite(tl.forward_record(semi, u, 1, cfl, 1)).all()

@@ -249,6 +249,12 @@ bool fused_cfl(const tlw_handle* h) {
     return h->d_slots && (use_surface_pass(h) || use_curved_pass(h)) && !h->sc && !h->parabolic && h->lim_count == 0;
 }
 
+// the status word of the speeds a fused step out of state buffer `from` keeps: a plain periodic mesh reports an
+// inadmissible new state with the step that wrote it, the others (where a run may end in one) with the next step
+unsigned* speed_status(tlw_handle* h, int from) {
+    return use_slots(h) ? &h->d_step->status : speed_status_of(ring_slot(h, 1 - from));
+}
+
 // Whether the volume kernel of a fused step forms dt itself: it costs each CTA about 1 % (512^2: N = 3 0.195 -> 0.200,
 // N = 4 0.430 -> 0.434, N = 5 0.699 -> 0.707 ms), a dt launch about 3 us, so up to 16 resident sets of CTAs (148 SMs x 5
 // CTAs of about 128 nodes). Not with source terms, whose kernels are not built that way.
@@ -373,6 +379,7 @@ void enqueue_curved_surfaces(tlw_handle* h, int mode, const double* u_jump, doub
             ca.cfl_interior = (const double*)h->d_slots;
             ca.cfl_max = ring_slot(h, 1 - ring);
             ca.advance = h->d_step;
+            ca.speed_status = speed_status(h, ring);
         }
         dispatch<CSrf>(h->N, h->stream, ca, cb);
         if (ev) {
@@ -542,6 +549,7 @@ void enqueue_rhs(tlw_handle* h, int stage, int mode, const double* u_flux, const
     va.cfl_stride = fused ? 2 : CFL_SLOTS;
     if (mode == MODE_STEP && stage != TLW_STAGE_MDRK1 && (fused || (use_slots(h) && !fused_cfl(h))) && !h->te_request)
         va.cfl_slots = h->d_slots;
+    va.speed_status = fused ? speed_status(h, ring) : &h->d_step->status;
     if (fused && stage != TLW_STAGE_MDRK2 && begin_in_volume(h)) {
         va.step = h->d_step;
         va.ring = ring_slot(h, ring);
@@ -610,6 +618,7 @@ void enqueue_rhs(tlw_handle* h, int stage, int mode, const double* u_flux, const
     sa.jac_first = h->jac_first;
     sa.w_first = h->h_basis.weights[0];
     sa.w_last = h->h_basis.weights[h->n - 1];
+    sa.speed_status = va.speed_status;
     if (!fused) {
         sa.cfl_slots = va.cfl_slots;
     } else if (stage != TLW_STAGE_MDRK1) {
@@ -685,7 +694,7 @@ void enqueue_step(tlw_handle* h, int from, cudaEvent_t after_dt = nullptr, const
     const bool fused = fused_cfl(h);
     if (fused) {
         if (!h->slots_valid) {   // the first step of a state: its CFL maximum by a pass over it
-            cudaMemsetAsync(ring_slot(h, from), 0, RING_WAYS * RING_STRIDE * sizeof(unsigned long long), h->stream);
+            cudaMemsetAsync(h->d_ring, 0, 2 * RING_WAYS * RING_STRIDE * sizeof(unsigned long long), h->stream);
             if (h->curved)
                 dispatch<CSpd>(h->N, h->stream, u, (const double*)h->d_Ja, (const double*)h->d_ijn, (int)h->E, h->opts.gamma,
                                h->d_step, ring_slot(h, from));
@@ -705,7 +714,7 @@ void enqueue_step(tlw_handle* h, int from, cudaEvent_t after_dt = nullptr, const
                        false, indicator_args(h));
     if (fused) {
         if (!begin_in_volume(h))
-            launch_dependent(h->stream, begin_step_kernel, 1, 1, 0, h->d_step, ring_slot(h, from), ring_slot(h, 1 - from), h->n);
+            launch_dependent(h->stream, begin_step_kernel, 1, 1, 0, h->d_step, ring_slot(h, from), ring_slot(h, 1 - from), h->n, nullptr);
     } else if (h->parabolic) launch_dependent(h->stream, par_finalize_dt_kernel, 1, 1, 0, h->d_step, h->d_visc, h->N, h->curved ? 1 : 0);
     else launch_dependent(h->stream, finalize_dt_kernel, 1, 1, 0, h->d_step, h->n);
     if (after_dt) cudaEventRecord(after_dt, h->stream);

@@ -121,6 +121,7 @@ struct CurvedSurfArgs {
     const double* cfl_interior;
     unsigned long long* cfl_max;
     StepState* advance;
+    unsigned* speed_status;
 };
 
 // fn_low slot of a face: load_fn_low! fills (bottom, right, top, left) (src/solvers/dgsem_tree/dg_2d.jl:236-249)
@@ -516,7 +517,7 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, TLW_CURVED_MINB)
         if (a.cfl_max) {
             double J[4];
             load4w(a.metrics + node * 4, J);
-            node_speeds(a.gamma, x, a.status, l1, l2);
+            node_speeds(a.gamma, x, a.speed_status, l1, l2);
             curved_speeds(J, ij, l1, l2);
         }
     }

@@ -210,6 +210,9 @@ __device__ __forceinline__ bool run_finished(double t, double te) {
     return fabs(t - te) <= 1.4901161193847656e-8 * fmax(fabs(t), fabs(te)) || t >= te;
 }
 
+// Where the status bits of the speeds kept in a ring wait for the step that takes its dt from them
+__host__ __device__ inline unsigned* speed_status_of(unsigned long long* ring) { return reinterpret_cast<unsigned*>(ring + 1); }
+
 // The time step of a state whose scaled maximum speed has the bits `bits`: cfl * 2 / (n * max), or the fixed dt,
 // clamped so that t + dt <= t_end (set_dt!, src/solvers/lwfr.jl:76-90); 0 for a finished run, whose remaining steps
 // are then exact no-ops on the state.
@@ -224,9 +227,12 @@ __device__ __forceinline__ double step_size(const StepState* s, unsigned long lo
 }
 
 // dt of a step that keeps its own CFL maximum, from the partial maxima at ring; `write`: into the step state, with the
-// partial maxima at ring_next cleared for this step's surface pass (which moves t on at the end)
-__device__ __forceinline__ double begin_step_dt(StepState* s, const unsigned long long* ring, unsigned long long* ring_next,
+// partial maxima at ring_next cleared for this step's surface pass (which moves t on at the end). The word after the
+// first maximum holds the status bits of these speeds where they count from this step on (speed_status).
+__device__ __forceinline__ double begin_step_dt(StepState* s, unsigned long long* ring, unsigned long long* ring_next,
                                                 int n, bool write) {
+    unsigned* late = speed_status_of(ring);
+    const unsigned late_bits = write ? *late : 0u;
     unsigned long long bits = 0ull;
 #pragma unroll
     for (int k = 0; k < RING_WAYS; ++k) bits = max(bits, __ldg(ring + k * RING_STRIDE));
@@ -237,6 +243,10 @@ __device__ __forceinline__ double begin_step_dt(StepState* s, const unsigned lon
         s->t_step = s->t;
 #pragma unroll
         for (int k = 0; k < RING_WAYS; ++k) ring_next[k * RING_STRIDE] = 0ull;
+        if (late_bits) {
+            atomicOr(&s->status, late_bits);
+            *late = 0u;
+        }
     }
     return dt;
 }

@@ -55,6 +55,7 @@ struct SurfArgs {
     const double* cfl_interior;
     unsigned long long* cfl_max;
     StepState* advance;
+    unsigned* speed_status;   // status word of the kept speeds
 };
 
 __device__ __forceinline__ bool admissible(double gm1, const double* u) {
@@ -495,7 +496,7 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, (BND || SC || MORT
             for (int v = 0; v < NV; ++v) x[v] = fma(s, p[v], x[v]);
         }
         store4w(o2, x);
-        if (a.cfl_slots || a.cfl_max) node_speeds(a.gamma, x, a.status, l1, l2);
+        if (a.cfl_slots || a.cfl_max) node_speeds(a.gamma, x, a.speed_status, l1, l2);
     }
     if (!a.cfl_slots && !a.cfl_max) return;
     element_maxima<NB, EB>(sF, tid, el2, b, has2, l1, l2);
@@ -754,9 +755,12 @@ static __global__ void finalize_dt_kernel(StepState* s, int n) {
 }
 
 // dt of a step that keeps its own CFL maximum, where its first kernel does not form it
-static __global__ void begin_step_kernel(StepState* s, const unsigned long long* ring, unsigned long long* ring_next, int n) {
+// (record: the dt also goes there)
+static __global__ void begin_step_kernel(StepState* s, unsigned long long* ring, unsigned long long* ring_next, int n,
+                                         double* record = nullptr) {
     wait_for_previous();
-    begin_step_dt(s, ring, ring_next, n, true);
+    const double dt = begin_step_dt(s, ring, ring_next, n, true);
+    if (record) *record = dt;
 }
 
 // the next step's CFL maximum from the per-element slots: max_e J^{-1} (max_s l1 + max_s l2)

@@ -97,7 +97,7 @@ enum VolMode { MODE_RHS = 0, MODE_STEP = 1 };
 
 struct VolArgs {
     const double* u;        // state the stage fluxes are evaluated at  [v,i,j,e]
-    const double* u_base;   // MODE_STEP: out = u_base + dt * du        [v,i,j,e]
+    const double* u_base;   // MODE_STEP, MDRK: out = u_base + dt * du  [v,i,j,e] (LW: u + dt * du)
     double* out;            // du (MODE_RHS) or the updated state (MODE_STEP)
     double* tU;             // face traces of U   [v, l, face, e]
     double* tF;             // face traces of F.n [v, l, face, e]
@@ -129,9 +129,10 @@ struct VolArgs {
     const double* inv_jac_node;
     unsigned long long* cfl_slots;   // plain step on a TreeMesh: per-element CFL slots (or null)
     int cfl_stride;                  // words per element there: CFL_SLOTS, or 2 (the interior maxima alone)
+    unsigned* speed_status;          // status word of these speeds
     // BEGIN kernels (begin_step); null selects the others, whose dt is final
     StepState* step;
-    const unsigned long long* ring;
+    unsigned long long* ring;
     unsigned long long* ring_next;
     // temporal error estimate of the Adaptive step control (lw_volume_kernel_4!'s u_np1 / u_np1_low tail)
     double* temporal_errors;          // [e]
@@ -1142,7 +1143,7 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
         store_result<MODE>(a.out + ((size_t)e * nn + node) * NV, MODE == MODE_STEP ? s0 : -inverse_jacobian(), dt, acc, ub,
                            SRC ? Ssrc : nullptr, o);
         if (SLOTS && a.cfl_slots && i > 0 && i < n - 1 && j > 0 && j < n - 1) {
-            node_speeds(a.gamma, o, a.status, l1, l2);
+            node_speeds(a.gamma, o, a.speed_status, l1, l2);
             if (CURVED) {
                 const size_t k = (size_t)e * nn + node;
                 double Jn[4];
@@ -1542,7 +1543,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
         store_result<MODE>(a.out + ((size_t)e * nn + node) * NV, MODE == MODE_STEP ? -dt * ij : -ij, dt, acc, ub,
                            SRC ? Ssrc : nullptr, o);
         if (SLOTS && a.cfl_slots && i > 0 && i < n - 1 && j > 0 && j < n - 1) {
-            node_speeds(a.gamma, o, a.status, l1, l2);
+            node_speeds(a.gamma, o, a.speed_status, l1, l2);
             if (CURVED) {
                 const size_t k = (size_t)e * nn + node;
                 double Jn[4];
