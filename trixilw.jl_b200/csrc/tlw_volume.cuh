@@ -72,9 +72,9 @@ struct VolCfg {
     static constexpr int NODES = EB * nn;              // node slots of the CTA
     // doubles a node of the compact MDRK stage 2 keeps for itself (slot k of the node of thread t at k*NODES + t)
     static constexpr int MDRK_KEEP = 9;
-    // regions: X (f / x-results), Y (g / y-results); shock capturing adds F0X, F0Y (fluxes at u), UU (u), VC (v1, v2,
-    // c), FVX, FVY (first-order subcell fluxes), and with MUSCL subcells four regions of face values
-    __host__ __device__ static constexpr size_t regions(bool sc, int rec) { return (size_t)(!sc ? 2 : rec ? 12 : 8) * PLANES; }
+    // regions: X (f / x-results), Y (g / y-results); shock capturing adds UU (u), VC (v1, v2, c, p),
+    // FVX, FVY (first-order subcell fluxes), and with MUSCL subcells four regions of face values
+    __host__ __device__ static constexpr size_t regions(bool sc, int rec) { return (size_t)(!sc ? 2 : rec ? 10 : 6) * PLANES; }
     static constexpr size_t lw_bytes(bool sc = false, int rec = 0) { return regions(sc, rec) * sizeof(double); }
     static constexpr size_t mdrk_bytes(bool sc = false, int rec = 0, bool compact = false) {
         return (regions(sc, rec) + (size_t)(compact ? MDRK_KEEP : 0) * NODES) * sizeof(double);
@@ -299,111 +299,108 @@ __device__ __forceinline__ void line_contract(double* X, double* Y, int tid) {
 }
 
 // ---- shock capturing helpers (src/solvers/dgsem_tree/dg_2d.jl:251-282, 1948-1991; Trixi calcflux_fv!) ----
-// stage 0: park u and (v1, v2, c) of the node for the first-order subcell fluxes of its neighbours
+// The subcell scheme works on the instantaneous u: each node parks u and (v1, v2, c, p), from which its right and upper
+// neighbours form the fluxes of their common subcell faces (the shared-memory pipe bounds these kernels: the flux pairs
+// at u parked as well, and both faces of a direction read back for the divergence, took 83 instead of 39 64-bit
+// accesses a node; Riemann 256^2, N = 4: 152 -> 133 us). A node keeps the fluxes of its own left and lower face over
+// the last contraction and reads the two others.
+// stage 0: park u and (v1, v2, c, p)
 template <int N, class C>
 __device__ __forceinline__ void sc_park(double* UU, double* VC, int el, int i, int j, const double* u, double gamma,
                                         unsigned* status) {
-    const double ir = 1.0 / u[0];
+    const double ir = nr_reciprocal(u[0]);
     const double v1 = u[1] * ir, v2 = u[2] * ir;
     const double p = (gamma - 1.0) * (u[3] - 0.5 * (u[1] * v1 + u[2] * v2));
     const double c = checked_sqrt(gamma * p * ir, status);
-    const double vc[NV] = {v1, v2, c, 0.0};
+    const double vc[NV] = {v1, v2, c, p};
     node_put<N, C>(UU, VC, el, i, j, u, vc);
 }
-
-// Rusanov (Trixi flux_lax_friedrichs, 4 arguments) between node L and node R of one element, from the
-// parked states, fluxes (fx: x-fluxes if orientation 1, else y-fluxes) and speeds
-template <int N, class C>
-__device__ __forceinline__ void sc_face_flux(const double* UU, const double* VC, const double* FL, int el, int iL,
-                                             int jL, int iR, int jR, int orientation, int speed_kind, double* out) {
-    const int aL = el * C::P + iL + C::R * jL, aR = el * C::P + iR + C::R * jR;
-    constexpr int PV = C::PV;   // stride between variable planes
-    const double vL = VC[(orientation == 1 ? 0 : PV) + aL], vR = VC[(orientation == 1 ? 0 : PV) + aR];
-    const double cL = VC[2 * PV + aL], cR = VC[2 * PV + aR];
-    const double lambda = speed_kind == 0 ? fmax(fabs(vL), fabs(vR)) + fmax(cL, cR)
-                                          : fmax(fabs(vL) + cL, fabs(vR) + cR);
+// what a subcell face needs of a node: the state, its velocity, sound speed and pressure
+struct ScNode {
+    double u[NV], v1, v2, c, p;
+};
+template <class C>
+__device__ __forceinline__ ScNode sc_node(const double* UU, const double* VC, int at) {
+    constexpr int PV = C::PV;
+    return ScNode{{UU[at], UU[PV + at], UU[2 * PV + at], UU[3 * PV + at]}, VC[at], VC[PV + at], VC[2 * PV + at], VC[3 * PV + at]};
+}
+template <class C>
+__device__ __forceinline__ ScNode sc_node(const double* u, const double* VC, int at, bool) {
+    constexpr int PV = C::PV;
+    return ScNode{{u[0], u[1], u[2], u[3]}, VC[at], VC[PV + at], VC[2 * PV + at], VC[3 * PV + at]};
+}
+// Rusanov (Trixi flux_lax_friedrichs, 4 arguments) across an x (D = 0) or y (D = 1) face
+template <int D>
+__device__ __forceinline__ void sc_face_flux(const ScNode& L, const ScNode& R, int speed_kind, double* out) {
+    const double vL = D == 0 ? L.v1 : L.v2, vR = D == 0 ? R.v1 : R.v2;
+    const double lambda = speed_kind == 0 ? fmax(fabs(vL), fabs(vR)) + fmax(L.c, R.c)
+                                          : fmax(fabs(vL) + L.c, fabs(vR) + R.c);
+    const double h = -0.5 * lambda;
+    const double fL[NV] = {L.u[1 + D], fma(L.u[1], vL, D == 0 ? L.p : 0.0), fma(L.u[2], vL, D == 1 ? L.p : 0.0), (L.u[3] + L.p) * vL};
+    const double fR[NV] = {R.u[1 + D], fma(R.u[1], vR, D == 0 ? R.p : 0.0), fma(R.u[2], vR, D == 1 ? R.p : 0.0), (R.u[3] + R.p) * vR};
 #pragma unroll
-    for (int v = 0; v < NV; ++v)
-        out[v] = 0.5 * (FL[v * PV + aL] + FL[v * PV + aR]) + (-0.5 * lambda * (UU[v * PV + aR] - UU[v * PV + aL]));
+    for (int v = 0; v < NV; ++v) out[v] = 0.5 * (fL[v] + fR[v]) + h * (R.u[v] - L.u[v]);
 }
 
-// final stage: each node computes the subcell flux on its left (x) and lower (y) subcell face
+// last contraction's input: each node computes the subcell flux on its left (fx) and lower (fy) subcell face. On
+// elements that blend nothing in only those next to the element's faces, which the surface takes (fn_low [v, l, face, e]:
+// faces -x, +x use the subcell faces between nodes 0|1 and n-2|n-1 of row j).
 template <int N, class C>
-__device__ __forceinline__ void sc_faces(const double* UU, const double* VC, const double* F0X, const double* F0Y,
-                                         double* FVX, double* FVY, int el, int i, int j, int speed_kind) {
-    constexpr int PV = C::PV;
-    const int a = el * C::P + i + C::R * j;
-    double f[NV];
-    if (i >= 1) {
-        sc_face_flux<N, C>(UU, VC, F0X, el, i - 1, j, i, j, 1, speed_kind, f);
+__device__ __forceinline__ void sc_faces(const VolArgs& a, const double* UU, const double* VC, double* FVX, double* FVY,
+                                         int el, int e, int i, int j, const double* u, bool blended, double* fx, double* fy) {
+    constexpr int n = C::n, PV = C::PV;
+    const int at = el * C::P + i + C::R * j;
+    const bool edge_x = i == 1 || i == n - 1, edge_y = j == 1 || j == n - 1;
+    const ScNode own = sc_node<C>(u, VC, at, true);
+    const size_t tb = (size_t)e * 4 * n * NV;
+    if (i >= 1 && (blended || edge_x)) {
+        sc_face_flux<0>(sc_node<C>(UU, VC, at - 1), own, a.speed_kind, fx);
+        if (edge_x) store4w(a.tFn + tb + ((i == 1 ? 0 : n) + j) * NV, fx);
+        if (n == 2 && i == 1) store4w(a.tFn + tb + (n + j) * NV, fx);
 #pragma unroll
-        for (int v = 0; v < NV; ++v) FVX[v * PV + a] = f[v];
+        for (int v = 0; v < NV; ++v) FVX[v * PV + at] = fx[v];
     }
-    if (j >= 1) {
-        sc_face_flux<N, C>(UU, VC, F0Y, el, i, j - 1, i, j, 2, speed_kind, f);
+    if (j >= 1 && (blended || edge_y)) {
+        sc_face_flux<1>(sc_node<C>(UU, VC, at - C::R), own, a.speed_kind, fy);
+        if (edge_y) store4w(a.tFn + tb + ((j == 1 ? 2 * n : 3 * n) + i) * NV, fy);
+        if (n == 2 && j == 1) store4w(a.tFn + tb + (3 * n + i) * NV, fy);
 #pragma unroll
-        for (int v = 0; v < NV; ++v) FVY[v * PV + a] = f[v];
+        for (int v = 0; v < NV; ++v) FVY[v * PV + at] = fy[v];
     }
 }
 
-// epilogue: fv = w_i^-1 (f*_{i+1/2} - f*_{i-1/2}) + w_j^-1 (g*_{j+1/2} - g*_{j-1/2}) (element-boundary
-// subcell fluxes are zero); acc <- (1 - alpha) acc + alpha fv; fn_low traces of the four faces
+// epilogue of a node with the weight alpha: fv = w_i^-1 (f*_{i+1/2} - f*_{i-1/2}) + w_j^-1 (g*_{j+1/2} - g*_{j-1/2})
+// (element-boundary subcell fluxes are zero); acc <- (1 - alpha) acc + alpha fv
 template <int N, class C>
-__device__ __forceinline__ void sc_blend(const VolArgs& a, const double* FVX, const double* FVY, int el, int e, int i,
-                                         int j, double alpha, double* acc) {
-    constexpr int n = C::n;
-    constexpr int PV = C::PV;
-    const int base = el * C::P;
+__device__ __forceinline__ void sc_blend(const double* FVX, const double* FVY, int el, int i, int j, double alpha,
+                                         const double* fx, const double* fy, double* acc) {
+    constexpr int n = C::n, PV = C::PV;
+    const int at = el * C::P + i + C::R * j;
     const double iwi = 1.0 / c_tlw_w[N][i], iwj = 1.0 / c_tlw_w[N][j];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-        const double xr = i + 1 < n ? FVX[v * PV + base + (i + 1) + C::R * j] : 0.0;
-        const double xl = i >= 1 ? FVX[v * PV + base + i + C::R * j] : 0.0;
-        const double yt = j + 1 < n ? FVY[v * PV + base + i + C::R * (j + 1)] : 0.0;
-        const double yb = j >= 1 ? FVY[v * PV + base + i + C::R * j] : 0.0;
-        const double fv = iwi * (xr - xl) + iwj * (yt - yb);
+        const double xr = i + 1 < n ? FVX[v * PV + at + 1] : 0.0;
+        const double yt = j + 1 < n ? FVY[v * PV + at + C::R] : 0.0;
+        const double fv = iwi * (xr - (i >= 1 ? fx[v] : 0.0)) + iwj * (yt - (j >= 1 ? fy[v] : 0.0));
         acc[v] = (1.0 - alpha) * acc[v] + alpha * fv;
-    }
-    // fn_low [v, l, face, e]: faces -x, +x use the subcell faces between nodes 0|1 and n-2|n-1 of row j
-    const size_t tb = (size_t)e * 4 * n * NV;
-    double f[NV];
-    if (i == 1) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) f[v] = FVX[v * PV + base + 1 + C::R * j];
-        store4(a.tFn + tb + (0 * n + j) * NV, f);
-    }
-    if (i == n - 1) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) f[v] = FVX[v * PV + base + (n - 1) + C::R * j];
-        store4(a.tFn + tb + (1 * n + j) * NV, f);
-    }
-    if (j == 1) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) f[v] = FVY[v * PV + base + i + C::R * 1];
-        store4(a.tFn + tb + (2 * n + i) * NV, f);
-    }
-    if (j == n - 1) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) f[v] = FVY[v * PV + base + i + C::R * (n - 1)];
-        store4(a.tFn + tb + (3 * n + i) * NV, f);
     }
 }
 
 // ---- shock capturing on curvilinear meshes, the reference's P4estMesh{2} path (src/solvers/dgsem_tree/
 // dg_2d.jl:236-365, src/solvers/dgsem_structured/dg_2d.jl:75-311; Trixi calcflux_fv! for curved meshes) ----
-// flux_lax_friedrichs(uL, uR, nrm) from the states, their physical fluxes, normal velocities and sound speeds
-__device__ __forceinline__ void sc_normal_flux(int speed_kind, const double* uL, const double* fL, const double* gL,
-                                               double vnL, double cL, const double* uR, const double* fR,
-                                               const double* gR, double vnR, double cR, const double* nrm,
-                                               double* out) {
+// flux_lax_friedrichs(uL, uR, nrm)
+__device__ __forceinline__ void sc_normal_flux(int speed_kind, const ScNode& L, const ScNode& R, const double* nrm, double* out) {
     const double nn = sqrt(nrm[0] * nrm[0] + nrm[1] * nrm[1]);
-    const double lambda = speed_kind == 0 ? fmax(fabs(vnL), fabs(vnR)) + fmax(cL, cR) * nn
-                                          : fmax(fabs(vnL) + cL * nn, fabs(vnR) + cR * nn);
+    const double vL = L.v1 * nrm[0] + L.v2 * nrm[1], vR = R.v1 * nrm[0] + R.v2 * nrm[1];
+    const double lambda = speed_kind == 0 ? fmax(fabs(vL), fabs(vR)) + fmax(L.c, R.c) * nn
+                                          : fmax(fabs(vL) + L.c * nn, fabs(vR) + R.c * nn);
+    const double h = -0.5 * lambda;
+    const double fL[NV] = {L.u[1] * nrm[0] + L.u[2] * nrm[1], fma(L.u[1], vL, L.p * nrm[0]), fma(L.u[2], vL, L.p * nrm[1]),
+                           (L.u[3] + L.p) * vL};
+    const double fR[NV] = {R.u[1] * nrm[0] + R.u[2] * nrm[1], fma(R.u[1], vR, R.p * nrm[0]), fma(R.u[2], vR, R.p * nrm[1]),
+                           (R.u[3] + R.p) * vR};
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        const double fnL = fL[v] * nrm[0] + gL[v] * nrm[1], fnR = fR[v] * nrm[0] + gR[v] * nrm[1];
-        out[v] = 0.5 * (fnL + fnR) + (-0.5 * lambda * (uR[v] - uL[v]));
-    }
+    for (int v = 0; v < NV; ++v) out[v] = 0.5 * (fL[v] + fR[v]) + h * (R.u[v] - L.u[v]);
 }
 
 // Julia sign
@@ -557,16 +554,17 @@ __device__ __forceinline__ void sc_muscl_faces(const VolArgs& a, const double* U
         for (int v = 0; v < NV; ++v) UF[k * C::PLANES + v * PV + o] = fv[k][v];
 }
 
-// final stage on a curvilinear mesh: the subcell flux on the node's left (xi) and lower (eta) face along the
-// subcell normal; pure DG elements only need faces 1 and n-1, the latter with the reference's calc_fn_low!
-// normal; MUSCL elements take the reconstructed face values (their fluxes and speeds computed here)
+// last contraction's input on a curvilinear mesh: the subcell flux on the node's left (xi) and lower (eta) face along
+// the subcell normal; pure DG elements only need faces 1 and n-1, the latter with the reference's calc_fn_low! normal;
+// MUSCL elements take the reconstructed face values. fn_low of the four faces in load_fn_low!'s P4estMesh order (slot 0
+// bottom, 1 right, 2 top, 3 left).
 template <int N, class C, int REC>
-__device__ __forceinline__ void sc_faces_curved(const VolArgs& a, const double* UU, const double* VC, const double* F0X,
-                                                const double* F0Y, const double* UF, double* FVX, double* FVY, int el,
-                                                int e, int i, int j, bool blended, bool muscl) {
+__device__ __forceinline__ void sc_faces_curved(const VolArgs& a, const double* UU, const double* VC, const double* UF,
+                                                double* FVX, double* FVY, int el, int e, int i, int j, const double* u,
+                                                bool blended, bool muscl, double* fx, double* fy) {
     constexpr int n = C::n;
     constexpr int PV = C::PV;
-    const double gm1 = a.gamma - 1.0;
+    const size_t tb = (size_t)e * 4 * n * NV;
 #pragma unroll
     for (int d = 0; d < 2; ++d) {
         const int f = d == 0 ? i : j, line = d == 0 ? j : i;
@@ -575,76 +573,43 @@ __device__ __forceinline__ void sc_faces_curved(const VolArgs& a, const double* 
                                ? a.subq + (((size_t)e * 2 + d) * n + line) * 2
                                : a.subn + ((((size_t)e * 2 + d) * n + line) * (n - 1) + (f - 1)) * 2;
         const double nrm[2] = {__ldg(np), __ldg(np + 1)};
-        const int aL = el * C::P + (d == 0 ? i - 1 : i) + C::R * (d == 0 ? j : j - 1);
-        const int aR = el * C::P + i + C::R * j;
-        double uL[NV], uR[NV], fL[NV], gL[NV], fR[NV], gR[NV], vnL, vnR, cL, cR, out[NV];
+        const int aR = el * C::P + i + C::R * j, aL = aR - (d == 0 ? 1 : C::R);
+        ScNode L, R;
         if (REC >= 1 && muscl) {
             // the right (up) face value of the node before the face, the left (down) one of the node after it
             const double* PL = UF + (d == 0 ? 1 : 3) * C::PLANES;
             const double* PR = UF + (d == 0 ? 0 : 2) * C::PLANES;
 #pragma unroll
-            for (int v = 0; v < NV; ++v) { uL[v] = PL[v * PV + aL]; uR[v] = PR[v * PV + aR]; }
-            euler_fluxes(gm1, uL[0], uL[1], uL[2], uL[3], fL, gL);
-            euler_fluxes(gm1, uR[0], uR[1], uR[2], uR[3], fR, gR);
-            const double irL = 1.0 / uL[0], irR = 1.0 / uR[0];
-            const double v1L = uL[1] * irL, v2L = uL[2] * irL, v1R = uR[1] * irR, v2R = uR[2] * irR;
-            cL = checked_sqrt(a.gamma * (gm1 * (uL[3] - 0.5 * (uL[1] * v1L + uL[2] * v2L))) * irL, a.status);
-            cR = checked_sqrt(a.gamma * (gm1 * (uR[3] - 0.5 * (uR[1] * v1R + uR[2] * v2R))) * irR, a.status);
-            vnL = v1L * nrm[0] + v2L * nrm[1];
-            vnR = v1R * nrm[0] + v2R * nrm[1];
-        } else {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                uL[v] = UU[v * PV + aL]; uR[v] = UU[v * PV + aR];
-                fL[v] = F0X[v * PV + aL]; gL[v] = F0Y[v * PV + aL];
-                fR[v] = F0X[v * PV + aR]; gR[v] = F0Y[v * PV + aR];
+            for (int v = 0; v < NV; ++v) { L.u[v] = PL[v * PV + aL]; R.u[v] = PR[v * PV + aR]; }
+            for (ScNode* q : {&L, &R}) {
+                const double ir = 1.0 / q->u[0];
+                q->v1 = q->u[1] * ir;
+                q->v2 = q->u[2] * ir;
+                q->p = a.gm1 * (q->u[3] - 0.5 * (q->u[1] * q->v1 + q->u[2] * q->v2));
+                q->c = checked_sqrt(a.gamma * q->p * ir, a.status);
             }
-            vnL = VC[aL] * nrm[0] + VC[PV + aL] * nrm[1];
-            vnR = VC[aR] * nrm[0] + VC[PV + aR] * nrm[1];
-            cL = VC[2 * PV + aL];
-            cR = VC[2 * PV + aR];
+        } else {
+            L = sc_node<C>(UU, VC, aL);
+            R = sc_node<C>(u, VC, aR, true);
         }
-        sc_normal_flux(a.speed_kind, uL, fL, gL, vnL, cL, uR, fR, gR, vnR, cR, nrm, out);
+        double* out = d == 0 ? fx : fy;
+        sc_normal_flux(a.speed_kind, L, R, nrm, out);
+        if (f == 1 || f == n - 1) store4w(a.tFn + tb + ((d == 0 ? (i == 1 ? 3 : 1) : (j == 1 ? 0 : 2)) * n + line) * NV, out);
         double* dst = d == 0 ? FVX : FVY;
 #pragma unroll
         for (int v = 0; v < NV; ++v) dst[v * PV + aR] = out[v];
     }
 }
 
-// epilogue on a curvilinear mesh: acc <- (1 - alpha) acc (+ alpha fv on blended elements); fn_low of the four
-// faces in load_fn_low!'s P4estMesh order (slot 0 bottom, 1 right, 2 top, 3 left)
+// epilogue on a curvilinear mesh: acc <- (1 - alpha) acc (+ alpha fv on blended elements)
 template <int N, class C>
-__device__ __forceinline__ void sc_blend_curved(const VolArgs& a, const double* FVX, const double* FVY, int el, int e,
-                                                int i, int j, double alpha, bool blended, double* acc) {
-    constexpr int n = C::n;
-    constexpr int PV = C::PV;
-    const int base = el * C::P;
+__device__ __forceinline__ void sc_blend_curved(const double* FVX, const double* FVY, int el, int i, int j, double alpha,
+                                                bool blended, const double* fx, const double* fy, double* acc) {
     if (blended) {
-        const double iwi = 1.0 / c_tlw_w[N][i], iwj = 1.0 / c_tlw_w[N][j];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            const double xr = i + 1 < n ? FVX[v * PV + base + (i + 1) + C::R * j] : 0.0;
-            const double xl = i >= 1 ? FVX[v * PV + base + i + C::R * j] : 0.0;
-            const double yt = j + 1 < n ? FVY[v * PV + base + i + C::R * (j + 1)] : 0.0;
-            const double yb = j >= 1 ? FVY[v * PV + base + i + C::R * j] : 0.0;
-            const double fv = iwi * (xr - xl) + iwj * (yt - yb);
-            acc[v] = (1.0 - alpha) * acc[v] + alpha * fv;
-        }
+        sc_blend<N, C>(FVX, FVY, el, i, j, alpha, fx, fy, acc);
     } else {
 #pragma unroll
         for (int v = 0; v < NV; ++v) acc[v] = (1.0 - alpha) * acc[v];
-    }
-    const size_t tb = (size_t)e * 4 * n * NV;
-    double f[NV];
-    if (i == 1 || i == n - 1) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) f[v] = FVX[v * PV + base + i + C::R * j];
-        store4(a.tFn + tb + ((i == 1 ? 3 : 1) * n + j) * NV, f);
-    }
-    if (j == 1 || j == n - 1) {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) f[v] = FVY[v * PV + base + i + C::R * j];
-        store4(a.tFn + tb + ((j == 1 ? 0 : 2) * n + i) * NV, f);
     }
 }
 
@@ -900,9 +865,7 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
     extern __shared__ double smem_d[];
     double* X = smem_d;
     double* Y = X + C::PLANES;
-    double* F0X = Y + C::PLANES;       // shock capturing only
-    double* F0Y = F0X + C::PLANES;
-    double* UU = F0Y + C::PLANES;
+    double* UU = Y + C::PLANES;        // shock capturing only: u, (v1, v2, c, p), subcell fluxes
     double* VC = UU + C::PLANES;
     double* FVX = VC + C::PLANES;
     double* FVY = FVX + C::PLANES;
@@ -921,14 +884,14 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
     const int i = node % n, j = node / n;
     const int e = blockIdx.x * EB + el;
     const bool active = el < EB && e < a.E;
-    // curvilinear shock capturing: pure_and_blended_element_ids! (DG only where alpha is within 1e-12 of 0);
-    // MUSCL subcells on blended elements without a boundary face
-    double alpha_e = 0.0;
+    // shock capturing: DG only where alpha is 0 (curvilinear: within 1e-12 of it, pure_and_blended_element_ids!); MUSCL
+    // subcells on blended elements without a boundary face
+    double alpha_e = 0.0, fx[NV], fy[NV];
     bool blended = false, muscl = false;
-    if (SC && CURVED && active) {
+    if (SC && active) {
         alpha_e = __ldg(a.alpha + e);
-        blended = !(fabs(alpha_e) <= 1e-12);
-        muscl = REC >= 1 && blended && !__ldg(a.atb + e);
+        blended = CURVED ? !(fabs(alpha_e) <= 1e-12) : alpha_e != 0.0;
+        muscl = CURVED && REC >= 1 && blended && !__ldg(a.atb + e);
     }
     double dt = 0.0;
     __shared__ double s_dt;
@@ -976,7 +939,6 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
         }
         flux_base(a.gm1, uu, f, g);
         put(f, g);
-        if (SC) node_put<N, C>(F0X, F0Y, el, i, j, f, g);
         if (SC) sc_park<N, C>(UU, VC, el, i, j, uu, a.gamma, a.status);
         uu[3] *= a.gamma;
 #pragma unroll
@@ -1125,8 +1087,8 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
         store_traces<n>(a, e, i, j, U, F, G);
         line_put<N, C>(X, Y, el, i, j, F, G);
         if (SC) {
-            if constexpr (CURVED) sc_faces_curved<N, C, REC>(a, UU, VC, F0X, F0Y, UF, FVX, FVY, el, e, i, j, blended, muscl);
-            else sc_faces<N, C>(UU, VC, F0X, F0Y, FVX, FVY, el, i, j, a.speed_kind);
+            if constexpr (CURVED) sc_faces_curved<N, C, REC>(a, UU, VC, UF, FVX, FVY, el, e, i, j, ub, blended, muscl, fx, fy);
+            else sc_faces<N, C>(a, UU, VC, FVX, FVY, el, e, i, j, ub, blended, fx, fy);
         }
     }
     phase_sync<C>();
@@ -1137,8 +1099,8 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
         double acc[NV], o[NV];
         node_sum<N, C>(X, Y, el, i, j, acc);
         if (SC) {
-            if constexpr (CURVED) sc_blend_curved<N, C>(a, FVX, FVY, el, e, i, j, alpha_e, blended, acc);
-            else sc_blend<N, C>(a, FVX, FVY, el, e, i, j, __ldg(a.alpha + e), acc);
+            if constexpr (CURVED) sc_blend_curved<N, C>(FVX, FVY, el, i, j, alpha_e, blended, fx, fy, acc);
+            else if (blended) sc_blend<N, C>(FVX, FVY, el, i, j, alpha_e, fx, fy, acc);
         }
         store_result<MODE>(a.out + ((size_t)e * nn + node) * NV, MODE == MODE_STEP ? s0 : -inverse_jacobian(), dt, acc, ub,
                            SRC ? Ssrc : nullptr, o);
@@ -1237,9 +1199,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     extern __shared__ double smem_d[];
     double* X = smem_d;
     double* Y = X + C::PLANES;
-    double* F0X = Y + C::PLANES;       // shock capturing only: fluxes, u, speeds at u^n, subcell fluxes
-    double* F0Y = F0X + C::PLANES;
-    double* UU = F0Y + C::PLANES;
+    double* UU = Y + C::PLANES;        // shock capturing only: u, (v1, v2, c, p), subcell fluxes
     double* VC = UU + C::PLANES;
     double* FVX = VC + C::PLANES;
     double* FVY = FVX + C::PLANES;
@@ -1253,12 +1213,12 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     const int i = node % n, j = node / n;
     const int e = blockIdx.x * EB + el;
     const bool active = el < EB && e < a.E;
-    double alpha_e = 0.0;
+    double alpha_e = 0.0, fx[NV], fy[NV];
     bool blended = false, muscl = false;
-    if (SC && CURVED && active) {
+    if (SC && active) {
         alpha_e = __ldg(a.alpha + e);
-        blended = !(fabs(alpha_e) <= 1e-12);
-        muscl = REC >= 1 && blended && !__ldg(a.atb + e);
+        blended = CURVED ? !(fabs(alpha_e) <= 1e-12) : alpha_e != 0.0;
+        muscl = CURVED && REC >= 1 && blended && !__ldg(a.atb + e);
     }
     double dt = 0.0;
     __shared__ double s_dt;
@@ -1287,7 +1247,6 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
         put(f0, g0);
         if (SC) {
             // the subcell FV part uses the instantaneous u^n (multi_derivative_2d.jl:205)
-            node_put<N, C>(F0X, F0Y, el, i, j, f0, g0);
             sc_park<N, C>(UU, VC, el, i, j, uu, a.gamma, a.status);
         }
     }
@@ -1355,8 +1314,8 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
         store_traces<n>(a, e, i, j, U, F, G);
         line_put<N, C>(X, Y, el, i, j, F, G);
         if (SC) {
-            if constexpr (CURVED) sc_faces_curved<N, C, REC>(a, UU, VC, F0X, F0Y, UF, FVX, FVY, el, e, i, j, blended, muscl);
-            else sc_faces<N, C>(UU, VC, F0X, F0Y, FVX, FVY, el, i, j, a.speed_kind);
+            if constexpr (CURVED) sc_faces_curved<N, C, REC>(a, UU, VC, UF, FVX, FVY, el, e, i, j, uu, blended, muscl, fx, fy);
+            else sc_faces<N, C>(a, UU, VC, FVX, FVY, el, e, i, j, uu, blended, fx, fy);
         }
     }
     phase_sync<C>();
@@ -1366,8 +1325,8 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
         double acc[NV];
         node_sum<N, C>(X, Y, el, i, j, acc);
         if (SC) {
-            if constexpr (CURVED) sc_blend_curved<N, C>(a, FVX, FVY, el, e, i, j, alpha_e, blended, acc);
-            else sc_blend<N, C>(a, FVX, FVY, el, e, i, j, __ldg(a.alpha + e), acc);
+            if constexpr (CURVED) sc_blend_curved<N, C>(FVX, FVY, el, i, j, alpha_e, blended, fx, fy, acc);
+            else if (blended) sc_blend<N, C>(FVX, FVY, el, i, j, alpha_e, fx, fy, acc);
         }
         double o[NV], ub[NV];
         if (MODE == MODE_STEP) load4w(a.u_base + ((size_t)e * nn + node) * NV, ub);
@@ -1397,9 +1356,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     extern __shared__ double smem_d[];
     double* X = smem_d;
     double* Y = X + C::PLANES;
-    double* F0X = Y + C::PLANES;       // shock capturing only: fluxes, u, speeds at u^n, subcell fluxes
-    double* F0Y = F0X + C::PLANES;
-    double* UU = F0Y + C::PLANES;
+    double* UU = Y + C::PLANES;        // shock capturing only: u, (v1, v2, c, p), subcell fluxes
     double* VC = UU + C::PLANES;
     double* FVX = VC + C::PLANES;
     double* FVY = FVX + C::PLANES;
@@ -1417,12 +1374,12 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     const int i = node % n, j = node / n;
     const int e = blockIdx.x * EB + el;
     const bool active = el < EB && e < a.E;
-    double alpha_e = 0.0;
+    double alpha_e = 0.0, fx[NV], fy[NV];
     bool blended = false, muscl = false;
-    if (SC && CURVED && active) {
+    if (SC && active) {
         alpha_e = __ldg(a.alpha + e);
-        blended = !(fabs(alpha_e) <= 1e-12);
-        muscl = REC >= 1 && blended && !__ldg(a.atb + e);
+        blended = CURVED ? !(fabs(alpha_e) <= 1e-12) : alpha_e != 0.0;
+        muscl = CURVED && REC >= 1 && blended && !__ldg(a.atb + e);
     }
     // dt of this element's instance (batched form) or the single dt
     const double dt = a.inst ? a.dt[__ldg(a.inst + min(e, a.E - 1))] : *a.dt;
@@ -1460,10 +1417,8 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
         }
         if (SC) {
             // the subcell FV part uses the instantaneous u^n, not u* (multi_derivative_2d.jl:257)
-            double un[NV], fn0[NV], gn0[NV];
+            double un[NV];
             load4w(a.u_base + ((size_t)e * nn + node) * NV, un);
-            euler_fluxes(a.gm1, un[0], un[1], un[2], un[3], fn0, gn0);
-            node_put<N, C>(F0X, F0Y, el, i, j, fn0, gn0);
             sc_park<N, C>(UU, VC, el, i, j, un, a.gamma, a.status);
         }
     }
@@ -1521,8 +1476,10 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
         store_traces<n>(a, e, i, j, U, F, G);
         line_put<N, C>(X, Y, el, i, j, F, G);
         if (SC) {
-            if constexpr (CURVED) sc_faces_curved<N, C, REC>(a, UU, VC, F0X, F0Y, UF, FVX, FVY, el, e, i, j, blended, muscl);
-            else sc_faces<N, C>(UU, VC, F0X, F0Y, FVX, FVY, el, i, j, a.speed_kind);
+            double un[NV];
+            load4w(a.u_base + ((size_t)e * nn + node) * NV, un);
+            if constexpr (CURVED) sc_faces_curved<N, C, REC>(a, UU, VC, UF, FVX, FVY, el, e, i, j, un, blended, muscl, fx, fy);
+            else sc_faces<N, C>(a, UU, VC, FVX, FVY, el, e, i, j, un, blended, fx, fy);
         }
     }
     phase_sync<C>();
@@ -1535,8 +1492,8 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
         double acc[NV];
         node_sum<N, C>(X, Y, el, i, j, acc);
         if (SC) {
-            if constexpr (CURVED) sc_blend_curved<N, C>(a, FVX, FVY, el, e, i, j, alpha_e, blended, acc);
-            else sc_blend<N, C>(a, FVX, FVY, el, e, i, j, __ldg(a.alpha + e), acc);
+            if constexpr (CURVED) sc_blend_curved<N, C>(FVX, FVY, el, i, j, alpha_e, blended, fx, fy, acc);
+            else if (blended) sc_blend<N, C>(FVX, FVY, el, i, j, alpha_e, fx, fy, acc);
         }
         double o[NV], ub[NV];
         if (MODE == MODE_STEP) load4w(a.u_base + ((size_t)e * nn + node) * NV, ub);
