@@ -225,14 +225,13 @@ bool use_slots(const tlw_handle* h) {
 #ifndef TLW_MDRK_COMPACT
 #define TLW_MDRK_COMPACT 1
 #endif
-// (not with shock capturing: on the 512^2 Riemann problem the blended variant's steps took 1.099 ms at 142
-// registers (one CTA per SM's worth) and 1.029 ms capped at 96 registers, against 0.993 ms with the sweeps)
-#ifndef TLW_SURFACE_PASS_SC
-#define TLW_SURFACE_PASS_SC 0
-#endif
+// (shock capturing: meshes of up to 4 million nodes without mortars. Both sides of a face evaluate the blended flux, so
+// the pass pays as long as the traces of U, F and fn_low stay near the caches: Riemann problem, us a step with the sweeps
+// and boundary launches against the pass: 16^2 N = 4 31 / 22.5, 64^2 N = 4 38 / 34, 256^2 N = 3 144 / 135, N = 4 240 / 222,
+// N = 5 332 / 316, N = 6 (3.2 million nodes) 469 / 465; 512^2 N = 3 (4.2 million) 472 / 482, N = 5 1179 / 1186)
 bool use_surface_pass(const tlw_handle* h) {
-    return TLW_SURFACE_PASS && h->d_nbr && !h->curved && (!h->sc || TLW_SURFACE_PASS_SC) && h->nh == 0 &&
-           (h->nmx + h->nmy == 0 || h->nbr_mortars);
+    if (h->sc && (h->nmx + h->nmy > 0 || (int64_t)h->E * h->nn > 4000000)) return false;
+    return TLW_SURFACE_PASS && h->d_nbr && !h->curved && h->nh == 0 && (h->nmx + h->nmy == 0 || h->nbr_mortars);
 }
 
 // one element-centric pass for all faces of a curvilinear mesh instead of a launch per colour and boundary class (not
@@ -291,8 +290,6 @@ HaloArgs halo_args(tlw_handle* h, int cls, int mode, const double* u_jump, doubl
         a.alpha = h->d_alpha;
         a.tFn = h->d_tFn;
         a.jac_first = h->jac_first;
-        a.w_first = h->h_basis.weights[0];
-        a.w_last = h->h_basis.weights[h->n - 1];
     }
     return a;
 }
@@ -337,8 +334,6 @@ void enqueue_curved_surfaces(tlw_handle* h, int mode, const double* u_jump, doub
     if (h->sc) {
         ca.alpha = h->d_alpha;
         ca.tFn = h->d_tFn;
-        ca.w_first = h->h_basis.weights[0];
-        ca.w_last = h->h_basis.weights[h->n - 1];
     }
     if (h->unstructured) {
         ca.tG = h->d_tG;
@@ -616,8 +611,6 @@ void enqueue_rhs(tlw_handle* h, int stage, int mode, const double* u_flux, const
     sa.alpha = h->d_alpha;
     sa.tFn = h->d_tFn;
     sa.jac_first = h->jac_first;
-    sa.w_first = h->h_basis.weights[0];
-    sa.w_last = h->h_basis.weights[h->n - 1];
     sa.speed_status = va.speed_status;
     if (!fused) {
         sa.cfl_slots = va.cfl_slots;

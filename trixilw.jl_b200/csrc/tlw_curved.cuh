@@ -30,16 +30,16 @@ namespace tlw {
 __device__ __forceinline__ double max_abs_speed_normal(double gamma, const double* ul, const double* ur,
                                                        const double* nrm, int kind, unsigned* status) {
     const double gm1 = gamma - 1.0;
-    const double irl = 1.0 / ul[0], irr = 1.0 / ur[0];
+    const double irl = nr_reciprocal(ul[0]), irr = nr_reciprocal(ur[0]);
     const double v1l = ul[1] * irl, v2l = ul[2] * irl, v1r = ur[1] * irr, v2r = ur[2] * irr;
     const double pl = gm1 * (ul[3] - 0.5 * (ul[1] * v1l + ul[2] * v2l));
     const double pr = gm1 * (ur[3] - 0.5 * (ur[1] * v1r + ur[2] * v2r));
     const double vl = v1l * nrm[0] + v2l * nrm[1];
     const double vr = v1r * nrm[0] + v2r * nrm[1];
+    const double nn = sqrt(nrm[0] * nrm[0] + nrm[1] * nrm[1]);
+    if (kind == 0) return fmax(fabs(vl), fabs(vr)) + checked_sqrt_max(gamma * pl * irl, gamma * pr * irr, status) * nn;
     const double cl = checked_sqrt(gamma * pl * irl, status);
     const double cr = checked_sqrt(gamma * pr * irr, status);
-    const double nn = sqrt(nrm[0] * nrm[0] + nrm[1] * nrm[1]);
-    if (kind == 0) return fmax(fabs(vl), fabs(vr)) + fmax(cl, cr) * nn;
     return fmax(fabs(vl) + cl * nn, fabs(vr) + cr * nn);
 }
 
@@ -48,7 +48,7 @@ __device__ __forceinline__ void min_max_speed_normal(double gamma, const double*
                                                      const double* nrm, double* lmin, double* lmax,
                                                      unsigned* status) {
     const double gm1 = gamma - 1.0;
-    const double irl = 1.0 / ul[0], irr = 1.0 / ur[0];
+    const double irl = nr_reciprocal(ul[0]), irr = nr_reciprocal(ur[0]);
     const double v1l = ul[1] * irl, v2l = ul[2] * irl, v1r = ur[1] * irr, v2r = ur[2] * irr;
     const double pl = gm1 * (ul[3] - 0.5 * (ul[1] * v1l + ul[2] * v2l));
     const double pr = gm1 * (ur[3] - 0.5 * (ur[1] * v1r + ur[2] * v2r));
@@ -110,7 +110,6 @@ struct CurvedSurfArgs {
     // shock capturing (or null): blending factors [e] and the face-adjacent subcell fluxes fn_low [v, l, slot, e]
     const double* alpha;
     const double* tFn;
-    double w_first, w_last;
     // UnstructuredMesh2D (or null): physical flux traces tF <- F, tG <- G, and the caller's outward normals
     // [2, l, face, e]
     const double* tG;
@@ -176,14 +175,14 @@ __device__ __forceinline__ void blend_curved_flux(const CurvedSurfArgs& a, int p
     const double dt = *a.dt;
     const double J = __ldg(a.inv_jac + (size_t)pe * nn + np);
     double test[NV], low[NV];
-    const double cl = dt * J / (a.w_last * 0.5);
+    const double cl = dt * J * (2.0 * a.inv_w_last);
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         test[v] = uP[v] - cl * (Fn[v] - fil[v]);
         low[v] = uP[v] - cl * (fn[v] - fil[v]);
     }
     if (!admissible(gm1, test)) zhang_shu_flux_fix(gm1, uP, low, Fn, fil, fn, cl);
-    const double cr = -dt * J / (a.w_first * 0.5);
+    const double cr = -dt * J * (2.0 * a.inv_w_first);
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         test[v] = uS[v] - cr * (Fn[v] - fir[v]);
@@ -220,12 +219,12 @@ __device__ __forceinline__ void blend_unstructured_flux(const CurvedSurfArgs& a,
 #pragma unroll
     for (int v = 0; v < NV; ++v) Fb[v] = (1.0 - alp) * Fn[v] + alp * fn[v];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) low[v] = UP[v] - dt * J / (a.w_last * 0.5) * (Fb[v] - fil[v]);
+    for (int v = 0; v < NV; ++v) low[v] = UP[v] - dt * J * (2.0 * a.inv_w_last) * (Fb[v] - fil[v]);
     if (!admissible(gm1, low)) {
         alp = 1.0;
     } else {
 #pragma unroll
-        for (int v = 0; v < NV; ++v) low[v] = US[v] - dt * J / (a.w_first * 0.5) * (fir[v] - Fb[v]);
+        for (int v = 0; v < NV; ++v) low[v] = US[v] - dt * J * (2.0 * a.inv_w_first) * (fir[v] - Fb[v]);
         if (!admissible(gm1, low)) alp = 1.0;
     }
 #pragma unroll

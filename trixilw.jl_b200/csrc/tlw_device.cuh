@@ -159,6 +159,12 @@ __device__ __forceinline__ double checked_sqrt(double x, unsigned* status) {
     return sqrt(x);
 }
 
+// max(sqrt a, sqrt b), each argument checked: the larger argument's root (the correctly rounded root is monotone)
+__device__ __forceinline__ double checked_sqrt_max(double a, double b, unsigned* status) {
+    if (!(a >= 0.0 && b >= 0.0)) atomicOr(status, STATUS_NONADMISSIBLE);
+    return sqrt(fmax(a, b));
+}
+
 // Trixi max_abs_speeds: |v1| + c and |v2| + c of a state, computed the same way by every CFL pass
 __device__ __forceinline__ void node_speeds(double gamma, const double* x, unsigned* status, double& l1, double& l2) {
     const double ir = nr_reciprocal(x[0]);
@@ -255,15 +261,15 @@ __device__ __forceinline__ double begin_step_dt(StepState* s, unsigned long long
 __device__ __forceinline__ double max_abs_speed(double gamma, const double* ul, const double* ur, int orientation,
                                                 int kind, unsigned* status) {
     const double gm1 = gamma - 1.0;
-    const double irl = 1.0 / ul[0], irr = 1.0 / ur[0];
+    const double irl = nr_reciprocal(ul[0]), irr = nr_reciprocal(ur[0]);
     const double v1l = ul[1] * irl, v2l = ul[2] * irl, v1r = ur[1] * irr, v2r = ur[2] * irr;
     const double pl = gm1 * (ul[3] - 0.5 * (ul[1] * v1l + ul[2] * v2l));
     const double pr = gm1 * (ur[3] - 0.5 * (ur[1] * v1r + ur[2] * v2r));
     const double vl = orientation == 1 ? v1l : v2l;
     const double vr = orientation == 1 ? v1r : v2r;
+    if (kind == 0) return fmax(fabs(vl), fabs(vr)) + checked_sqrt_max(gamma * pl * irl, gamma * pr * irr, status);
     const double cl = checked_sqrt(gamma * pl * irl, status);
     const double cr = checked_sqrt(gamma * pr * irr, status);
-    if (kind == 0) return fmax(fabs(vl), fabs(vr)) + fmax(cl, cr);
     return fmax(fabs(vl) + cl, fabs(vr) + cr);
 }
 
@@ -271,7 +277,7 @@ __device__ __forceinline__ double max_abs_speed(double gamma, const double* ul, 
 __device__ __forceinline__ void min_max_speed(double gamma, const double* ul, const double* ur, int orientation,
                                               double* lmin, double* lmax, unsigned* status) {
     const double gm1 = gamma - 1.0;
-    const double irl = 1.0 / ul[0], irr = 1.0 / ur[0];
+    const double irl = nr_reciprocal(ul[0]), irr = nr_reciprocal(ur[0]);
     const double v1l = ul[1] * irl, v2l = ul[2] * irl, v1r = ur[1] * irr, v2r = ur[2] * irr;
     const double pl = gm1 * (ul[3] - 0.5 * (ul[1] * v1l + ul[2] * v2l));
     const double pr = gm1 * (ur[3] - 0.5 * (ur[1] * v1r + ur[2] * v2r));

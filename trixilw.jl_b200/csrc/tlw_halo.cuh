@@ -53,7 +53,7 @@ struct HaloArgs {
     // (element 1's: on a conforming TreeMesh every element's) and the GLL end weights
     const double* alpha;      // or null
     const double* tFn;
-    double jac_first, w_first, w_last;
+    double jac_first;
 };
 
 __device__ __forceinline__ int halo_face_node(int n, int f, int l) {
@@ -113,10 +113,10 @@ static __global__ void __launch_bounds__(128) halo_face_kernel(HaloArgs a) {
         load4(r + 3 * NV, fr);
         const double al = __ldg(a.alpha + e), ar = r[4 * NV];
         if (local_left)
-            blend_flux_values(a.gamma, a.speed_kind, a.status, a.jac_first, a.w_first, a.w_last, a.orientation, ul,
+            blend_flux_values(a.gamma, a.speed_kind, a.status, a.jac_first, a.inv_w_first, a.inv_w_last, a.orientation, ul,
                               ur, al, ar, fl, fr, *a.dt, Fn);
         else
-            blend_flux_values(a.gamma, a.speed_kind, a.status, a.jac_first, a.w_first, a.w_last, a.orientation, ur,
+            blend_flux_values(a.gamma, a.speed_kind, a.status, a.jac_first, a.inv_w_first, a.inv_w_last, a.orientation, ur,
                               ul, ar, al, fr, fl, *a.dt, Fn);
     }
     const double dts = a.step_mode ? *a.dt : 1.0;

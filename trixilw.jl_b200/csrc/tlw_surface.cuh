@@ -42,7 +42,6 @@ struct SurfArgs {
     const double* alpha;     // [e]
     const double* tFn;       // first-order subcell flux next to each face [v, l, face, e]
     double jac_first;        // J^{-1} used by the admissibility test (element 1's on TreeMesh)
-    double w_first, w_last;  // GLL weights w_1, w_n
     const int* inst;         // batched form: instance of each element (dt indexed by it); null otherwise
     const double* tFv;      // compressible Navier-Stokes: viscous normal flux traces (null otherwise)
     unsigned long long* cfl_slots;   // plain LW step: per-element CFL slots of the nodes finalised here
@@ -60,7 +59,8 @@ struct SurfArgs {
 
 __device__ __forceinline__ bool admissible(double gm1, const double* u) {
     // is_admissible (src/equations/compressible_euler_2d.jl:4-7): rho > 0 and p > 0
-    const double v1 = u[1] / u[0], v2 = u[2] / u[0];
+    const double ir = nr_reciprocal(u[0]);
+    const double v1 = u[1] * ir, v2 = u[2] * ir;
     const double p = gm1 * (u[3] - 0.5 * (u[1] * v1 + u[2] * v2));
     return u[0] > 0.0 && p > 0.0;
 }
@@ -68,9 +68,9 @@ __device__ __forceinline__ bool admissible(double gm1, const double* u) {
 // Fn <- alp fn + (1 - alp) Fn with compute_alp (dg_2d.jl:1879-1901, 1929-1937): fn is the first-order
 // flux at the instantaneous u, alp = (alpha_L + alpha_R)/2, or 1 when the low-order update of either face
 // subcell (subcell flux next to the face, fil / fir, lambda = 1/2) is not admissible. jac is the J^{-1} the
-// reference takes for the test (element 1's on TreeMesh), wf / wl the GLL weights w_1 / w_n.
+// reference takes for the test (element 1's on TreeMesh), iwf / iwl the inverse GLL weights 1 / w_1, 1 / w_n.
 __device__ __forceinline__ void blend_flux_values(double gamma, int speed_kind, unsigned* status, double jac,
-                                                  double wf, double wl, int orientation, const double* uL,
+                                                  double iwf, double iwl, int orientation, const double* uL,
                                                   const double* uR, double alphaL, double alphaR, const double* fil,
                                                   const double* fir, double dt, double* Fn) {
     const double gm1 = gamma - 1.0;
@@ -84,14 +84,14 @@ __device__ __forceinline__ void blend_flux_values(double gamma, int speed_kind, 
     double Fb[NV], low[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) Fb[v] = (1.0 - alp) * Fn[v] + alp * fn[v];
-    const double lamx = 0.5;
+    const double cl = dt * jac * (2.0 * iwl), cr = dt * jac * (2.0 * iwf);   // dt J^{-1} / (w lambda)
 #pragma unroll
-    for (int v = 0; v < NV; ++v) low[v] = uL[v] - dt * jac / (wl * lamx) * (Fb[v] - fil[v]);
+    for (int v = 0; v < NV; ++v) low[v] = uL[v] - cl * (Fb[v] - fil[v]);
     if (!admissible(gm1, low)) {
         alp = 1.0;
     } else {
 #pragma unroll
-        for (int v = 0; v < NV; ++v) low[v] = uR[v] - dt * jac / (wf * lamx) * (fir[v] - Fb[v]);
+        for (int v = 0; v < NV; ++v) low[v] = uR[v] - cr * (fir[v] - Fb[v]);
         if (!admissible(gm1, low)) alp = 1.0;
     }
 #pragma unroll
@@ -106,7 +106,7 @@ __device__ __forceinline__ void blend_interface_flux(const SurfArgs& a, int orie
     double fil[NV], fir[NV];
     load4(a.tFn + (((size_t)le * 4 + faceL) * n + l) * NV, fil);
     load4(a.tFn + (((size_t)re * 4 + faceR) * n + l) * NV, fir);
-    blend_flux_values(a.gamma, a.speed_kind, a.status, a.jac_first, a.w_first, a.w_last, orientation, uL, uR,
+    blend_flux_values(a.gamma, a.speed_kind, a.status, a.jac_first, a.inv_w_first, a.inv_w_last, orientation, uL, uR,
                       __ldg(a.alpha + le), __ldg(a.alpha + re), fil, fir, dt, Fn);
 }
 
@@ -336,6 +336,9 @@ template <int N> struct SurfCfg {
     // whole warps (the face-node maxima are reduced by warp shuffles over full masks)
     static constexpr int THREADS = (EB * 4 * n + 31) / 32 * 32;
     static constexpr int MIN_BLOCKS = THREADS <= 128 ? TLW_SURF_MINB : 5;
+    // the blended flux: 142 registers uncapped; Riemann 256^2, N = 4, a pass of 8 steps: 1.790 ms with 5 CTAs an SM, 1.779
+    // with 6 (80 registers), 1.783 with 7; 2.00 ms uncapped or with 4, when the flux still divided
+    static constexpr int SC_MIN_BLOCKS = THREADS <= 128 ? 6 : 4;
 };
 
 // The maxima of l1 and l2 over the NB phase-2 threads of each element (thread el2 * NB + b), in threads b = 0 and 1;
@@ -403,17 +406,15 @@ constexpr int NBR_MORTAR = -(1 << 30), NBR_MORTAR_END = -(1 << 29);
 // (MORTAR) a side of an L2 mortar: nbr[4e + f] (f = -x, +x, -y, +y) is the element across face f, -(k + 1) for boundary
 // k of the boundary arguments, or a mortar side. The nodes of a mortar's large face evaluate both halves' fluxes and
 // project them, so a mesh after AMR steps in the same two launches as a conforming one (64^2 refined once in the
-// middle, N = 4: 42.4 -> 29.3 us a step, the four launches of sweeps and mortars in one). Phase 1: one thread per (element, face, node) evaluates that face's flux exactly as
-// interface_kernel / boundary_kernel do (an interface with its own (left, right) arguments, so both elements get
+// middle, N = 4: 42.4 -> 29.3 us a step, the four launches of sweeps and mortars in one).
+// Phase 1: one thread per (element, face, node) evaluates that face's flux exactly as interface_kernel / boundary_kernel do (an interface with its own (left, right) arguments, so both elements get
 // the same bits) into shared memory. Phase 2: one thread per face node of the element applies the x face's lift
 // and then the y face's (the order of the x and y launches), with the Jacobian and dt, and reduces the element's
 // face-node CFL speeds. Each interface is evaluated twice and each element's face nodes are read and written once:
 // no strided x sweep, no atomics.
-#ifndef TLW_SURF_MINB_SC
-#define TLW_SURF_MINB_SC 1
-#endif
+// With boundaries or mortars the register count is left to the compiler; the blended flux is capped (see SurfCfg).
 template <int N, bool BND, bool SC, bool MORTAR = false>
-static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, (BND || SC || MORTAR) ? TLW_SURF_MINB_SC : SurfCfg<N>::MIN_BLOCKS)
+static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, SC ? SurfCfg<N>::SC_MIN_BLOCKS : (BND || MORTAR) ? 1 : SurfCfg<N>::MIN_BLOCKS)
     surface_kernel(SurfArgs a, BndArgs bnd, MortarArgs mo) {
     using C = SurfCfg<N>;
     constexpr int n = N + 1, EB = C::EB, NB = 4 * (n - 1);
