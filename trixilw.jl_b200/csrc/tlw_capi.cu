@@ -1949,9 +1949,9 @@ int tlw_rhs(tlw_handle* h, int32_t stage, double* du, const double* u, const dou
         return fail(h, TLW_E_STATE, "MDRK stages need a handle created with TLW_MDRK");
     TLW_CUDA(h, cudaSetDevice(h->device));
     const size_t bytes = state_doubles(h) * sizeof(double);
-    const double tdt[2] = {dt, t};   // dt_call, then (after t_step) t_call: the source terms' time
-    TLW_CUDA(h, cudaMemcpyAsync(&h->d_step->dt_call, &tdt[0], sizeof(double), cudaMemcpyHostToDevice, h->stream));
-    TLW_CUDA(h, cudaMemcpyAsync(&h->d_step->t_call, &tdt[1], sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    TLW_CUDA(h, cudaMemcpyAsync(&h->d_step->dt_call, &dt, sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    if (h->source)   // the source terms' time
+        TLW_CUDA(h, cudaMemcpyAsync(&h->d_step->t_call, &t, sizeof(double), cudaMemcpyHostToDevice, h->stream));
     const double *du_in = u, *dus = us;
     double* dout = du;
     // host arrays, and device arrays whose node records are not 32-byte aligned (the surface pass reads and writes
