@@ -592,7 +592,7 @@ static __global__ void __launch_bounds__(MS_THREADS) max_speed_kernel(const doub
     constexpr int ELEMS = MsCfg<N>::ELEMS;
     __shared__ double l1s[SPEED ? ELEMS * nn : 1], l2s[SPEED ? ELEMS * nn : 1];
     __shared__ double inds[IND ? ELEMS * nn : 1], tmps[IND ? ELEMS * nn : 1];
-    __shared__ double red[ELEMS];
+    __shared__ double red[ELEMS], sums[IND ? 3 * ELEMS : 1];
     wait_for_previous();
     dependents_may_start();
     const int e0 = blockIdx.x * ELEMS;
@@ -661,7 +661,17 @@ static __global__ void __launch_bounds__(MS_THREADS) max_speed_kernel(const doub
             c1 += __shfl_xor_sync(0xffffffffu, c1, o);
             c2 += __shfl_xor_sync(0xffffffffu, c2, o);
         }
+        // the blending factor, one thread per element: on the eight lanes of an element its exponential and divisions
+        // took as many instructions as the rest of the kernel (Riemann 256^2, N = 4: 22.0 -> 20.3 us)
         if (el < ne && q == 0) {
+            sums[el] = tot;
+            sums[ELEMS + el] = c1;
+            sums[2 * ELEMS + el] = c2;
+        }
+        __syncthreads();
+        if (threadIdx.x < ne) {
+            const int el = threadIdx.x;
+            const double tot = sums[el], c1 = sums[ELEMS + el], c2 = sums[2 * ELEMS + el];
             const double f1 = tot != 0.0 ? (tot - c1) / tot : 0.0;
             const double f2 = c1 != 0.0 ? (c1 - c2) / c1 : 0.0;
             const double energy = fmax(f1, f2);
