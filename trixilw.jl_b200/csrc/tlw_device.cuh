@@ -182,8 +182,8 @@ __device__ __forceinline__ void curved_speeds(const double* J, double inv_jac, d
     l2 = fabs(J[2] * a + J[3] * b) * ij;
 }
 
-// Per-element CFL slots written by the kernels that produce the final values of a step (plain LW on a
-// periodic conforming TreeMesh): slot s of element e holds the bits of max(|v1| + c) and max(|v2| + c) over
+// Per-element CFL slots written by the kernels that produce the final values of a step that does not reduce its
+// CFL maximum itself (a periodic conforming TreeMesh with the positivity limiter, or without the surface pass): slot s of element e holds the bits of max(|v1| + c) and max(|v2| + c) over
 // the nodes finalised there: 0 interior (volume kernel); 1 all face nodes (the element-centric surface pass),
 // or with the interface sweeps 1 / 2 the -x / +x face without corners (x interfaces), 3 / 4 the -y / +y face
 // with corners (y interfaces). The next step reduces them instead of reading the whole state again.
