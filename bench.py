@@ -121,7 +121,7 @@ def mdrk_volume_flops_per_node(N: int) -> float:
 def surface_pass_bytes_per_element(N: int) -> float:
     """Algorithmic (unique) bytes of one element-centric surface launch per element: read the element's own U
     and F.n face traces (2 x 4 faces x n x nv), read its 4(n - 1) face nodes of u for the jumps, read-modify-write
-    the same face nodes of the output, write two CFL slots. The neighbours' traces and face nodes are the
+    the same face nodes of the output, read the interior maxima (two words). The neighbours' traces and face nodes are the
     neighbours' own bytes, counted once there."""
     n, nv = N + 1, 4
     nb = 4 * (n - 1)
@@ -655,9 +655,9 @@ def run_ours(args):
                     {"achieved": None, "peak": fp64_peak, "unit": "TFLOP/s",
                      "note": "no algorithmic flop model for the Navier-Stokes or the shock-capturing kernels"})
         binding = fp64_rec if fp64_bound else hbm_rec
-        # a TreeMesh whose every face is an interface or a boundary runs one element-centric surface launch per
-        # stage (surface_kernel); other meshes run the x and y sweeps
-        surf_pass = not curved and not ns and getattr(semi.mesh, "n_mortars", 0) == 0
+        # a TreeMesh runs one element-centric surface launch per stage (surface_kernel); with shock capturing above
+        # 4 M nodes the x and y sweeps
+        surf_pass = not curved and not ns and not sc
         stages = 2 if td == "mdrk" else 1
         surf_ms = (phase[2] + phase[3]) / args.steps
         phases_rec = {"cfl_dt": phase[0] / args.steps, "volume": phase[1] / args.steps, "surfaces": surf_ms,
@@ -701,9 +701,11 @@ def run_ours(args):
                          "phase_ms_per_step": phases_rec,
                          **({"surface": surf_rec} if surf_rec else {})},
             "clocks": clocks,
-            "gpu_launches": args.steps * ((8 + 2 * int(L.tlw_curved_colors(semi.handle))) if ns else
-                                          (5 + int(L.tlw_curved_colors(semi.handle))) if icname == "blast" else
-                                          (2 + 2 * stages + (1 if icname == "riemann" else 0))),
+            # Navier-Stokes: maxima, dt, gradients, volume, surfaces; blast: CFL and indicator, smoothing, dt, volume, a
+            # launch per colour; riemann (above 4 M nodes): those four, x / y interfaces and boundaries; else dt and per
+            # stage volume and surfaces
+            "gpu_launches": args.steps * (5 if ns else (4 + int(L.tlw_curved_colors(semi.handle))) if icname == "blast" else
+                                          8 if icname == "riemann" else 1 + 2 * stages),
         }
         if world == 1 and not args.no_cpu_baseline:
             rate, threads, nsteps, el = cpu_oracle_rate(level, N, td, icname, steps_hint=args.steps)
@@ -1034,7 +1036,7 @@ def run_batched(args, emit=True):
                          "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else "fallback",
                          "alg_bytes_per_step": step_alg},
             "clocks": clocks,
-            "gpu_launches": K * (1 + 4 * len(E_by_N)),
+            "gpu_launches": K * (1 + 3 * len(E_by_N)),   # dt; per degree the CFL pass, volume and surfaces
         }
         if world == 1 and not args.no_cpu_baseline:
             sys.path.insert(0, os.path.join(ROOT, "oracle"))
@@ -1191,10 +1193,10 @@ def run_adjoint(args, emit=True):
             "e2e": {"value": ndofs * nsteps / e2e_s, "unit": UNIT, "h2d_bytes_per_step": 8 * 5 * ndofs / nsteps,
                     "d2h_bytes_per_step": 8 * 8 * ndofs / nsteps, "seconds": e2e_s},
             "clocks": clocks,
-            # per gradient: record 5 a step (speed, dt, volume, 2 interface sweeps), objective 2, recompute 3 a
+            # per gradient: record 3 a step (dt, volume, surfaces) and one speed pass, objective 2, recompute 2 a
             # step (the last segment comes from the record, each segment's last step is a volume launch only),
             # adjoint 2 a step
-            "gpu_launches": reps * (5 * nsteps + 2 + 3 * (nsteps - ck) - 2 * ((nsteps - 1) // ck) + 2 * nsteps),
+            "gpu_launches": reps * (3 * nsteps + 1 + 2 + 2 * (nsteps - ck) - (nsteps - 1) // ck + 2 * nsteps),
         }
         if not emit:
             return out
