@@ -164,7 +164,9 @@ int tlw_set_parabolic_walls(tlw_handle* h, const int32_t* kinds, const double* w
  *   mortar_large_sides  [n_mortars]     1: large element on the -side, 2: on the +side   Trixi mortars.large_sides
  *   mortar_orientations [n_mortars]     1 = x, 2 = y                                     Trixi mortars.orientations
  * The LW traces are carried over the mortar as prolong2mortars! / calc_mortar_flux! do
- * (src/solvers/dgsem_tree/dg_2d.jl:1456-1646), with Trixi's L2 mortar operators. Not with shock capturing. */
+ * (src/solvers/dgsem_tree/dg_2d.jl:1456-1646), with Trixi's L2 mortar operators; with shock capturing they keep the
+ * plain LW flux and the blending factors are smoothed across them. Not with Navier-Stokes: refused here after
+ * tlw_set_parabolic, and there once the mesh has mortars. */
 int tlw_set_tree_mortars(tlw_handle* h, int64_t n_mortars, const int64_t* mortar_neighbor_ids,
                          const int64_t* mortar_large_sides, const int64_t* mortar_orientations);
 

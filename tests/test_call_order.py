@@ -1,0 +1,43 @@
+"""Orders of calls on a handle that the library refuses, or that it has to keep consistent."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def make(tl, N, td="lw", periodic=True):
+    tdo = tl.LW() if td == "lw" else tl.MDRK()
+    mesh = tl.TreeMesh((-10.0, -10.0), (10.0, 10.0), 3, periodicity=periodic)
+    solver = tl.DGSEM(N, tl.flux_lax_friedrichs, tl.VolumeIntegralFR(tdo))
+    more = {}
+    if not periodic:
+        more["boundary_conditions"] = {"x_neg": tl.boundary_condition_slip_wall_vertical,
+                                       "x_pos": tl.boundary_condition_slip_wall_vertical,
+                                       "y_neg": tl.boundary_condition_slip_wall_horizontal,
+                                       "y_pos": tl.boundary_condition_slip_wall_horizontal}
+    ic = tl.IsentropicVortex(5.0, velocity=(1.0, 1.0) if periodic else (0.0, 0.0))
+    return tl.SemidiscretizationHyperbolic(mesh, tdo, tl.CompressibleEulerEquations2D(1.4), ic, solver, **more)
+
+
+def test_mortars_after_navier_stokes_are_refused(tl):
+    """Nothing is launched: the mesh upload, the Navier-Stokes terms and then the mortars, whose sides no Navier-Stokes
+    kernel takes."""
+    from trixilw import _lib
+    L = _lib.lib()
+    semi = make(tl, 3)
+    m = tl.RefinedTreeMesh((-10.0, -10.0), (10.0, 10.0), 2, ((0.0, 0.0), (4.0, 4.0)))
+    h = semi.handle
+    ij = np.ascontiguousarray(m.inverse_jacobian)
+    dp = lambda a: a.ctypes.data_as(_lib.ctypes.POINTER(_lib.ctypes.c_double))
+    ip = lambda a: a.ctypes.data_as(_lib.ctypes.POINTER(_lib.ctypes.c_int64))
+    upload = lambda: _lib.check(h, L.tlw_set_tree_mesh(h, m.n_elements, dp(ij), m.n_interfaces, ip(m.interface_neighbor_ids),
+                                                       ip(m.interface_orientations), 0, None, None, None, None))
+    mortars = lambda count: L.tlw_set_tree_mortars(h, count, ip(m.mortar_neighbor_ids), ip(m.mortar_large_sides),
+                                                   ip(m.mortar_orientations))
+    upload()
+    _lib.check(h, L.tlw_set_parabolic(h, 1e-3, 0.72))
+    assert mortars(m.n_mortars) == _lib.TLW_E_UNSUPPORTED
+    assert mortars(0) == _lib.TLW_OK
+    upload()                                  # a new mesh has no Navier-Stokes terms
+    assert mortars(m.n_mortars) == _lib.TLW_OK
+    assert L.tlw_set_parabolic(h, 1e-3, 0.72) == _lib.TLW_E_UNSUPPORTED

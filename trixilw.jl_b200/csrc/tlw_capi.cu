@@ -1207,6 +1207,9 @@ int tlw_set_tree_mortars(tlw_handle* h, int64_t n_mortars, const int64_t* mortar
                          const int64_t* mortar_large_sides, const int64_t* mortar_orientations) {
     if (!h) return TLW_E_ARG;
     if (!h->have_mesh || h->curved) return fail(h, TLW_E_STATE, "mortars follow tlw_set_tree_mesh");
+    // (as tlw_set_parabolic refuses a mesh that has mortars; the Navier-Stokes kernels would take the mortar sides in
+    // d_nbr for boundaries)
+    if (h->parabolic && n_mortars > 0) return fail(h, TLW_E_UNSUPPORTED, "Navier-Stokes: conforming mesh");
     if (n_mortars < 0 || (n_mortars > 0 && (!mortar_neighbor_ids || !mortar_large_sides || !mortar_orientations)))
         return fail(h, TLW_E_ARG, "mortars");
     std::vector<int> ml[2], mu[2], mg[2], ms[2];
