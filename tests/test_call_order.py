@@ -41,3 +41,40 @@ def test_mortars_after_navier_stokes_are_refused(tl):
     upload()                                  # a new mesh has no Navier-Stokes terms
     assert mortars(m.n_mortars) == _lib.TLW_OK
     assert L.tlw_set_parabolic(h, 1e-3, 0.72) == _lib.TLW_E_UNSUPPORTED
+
+
+@pytest.mark.parametrize("N,td,periodic,limiter", [(3, "lw", True, False), (4, "mdrk", True, False), (4, "lw", False, False),
+                                                   (3, "lw", True, True)])
+def test_split_steps_between_steps(oracle_mod, tl, N, td, periodic, limiter):
+    """On a mesh without halo faces the split step may stand between runs of plain steps, which then take the time step
+    of the state it left. dt of every step and the state against the oracle, at the bars of the multi-step tests."""
+    from trixilw import _lib
+    L = _lib.lib()
+    semi = make(tl, N, td, periodic)
+    if limiter:   # (leaves the vortex as it is; the steps keep per-element maxima)
+        from trixilw.limiters import install
+        install(semi, (tl.PositivityPreservingLimiterZhangShu((5e-6,), (tl.density,)),))
+    o = oracle_mod.Oracle(semi.mesh, N)
+    if not periodic:
+        o.set_boundary_kinds(np.repeat(np.array([1, 1, 2, 2], dtype=np.int32), semi.mesh.n_boundaries_per_direction))
+    u = semi.compute_coefficients(0.0)
+    integ = tl.LWIntegrator(tl.semidiscretize(semi, semi.time_discretization, (0.0, 1e9)))
+    integ.set_state(u, 0.0)
+    h = semi.handle
+
+    def split(count):
+        for _ in range(count):
+            _lib.check(h, L.tlw_dd_begin(h, 0.2, 0.0, 1e9))
+            for _stage in range(L.tlw_dd_stages(h)):
+                _lib.check(h, L.tlw_dd_volume(h))
+                _lib.check(h, L.tlw_dd_finish(h))
+
+    ref, t = u.copy(), 0.0
+    for run, count in ((lambda c: integ.step(c, 0.2), 3), (split, 3), (lambda c: integ.step(c, 0.2), 2), (split, 2),
+                       (lambda c: integ.step(c, 0.2, use_graph=False), 1)):
+        run(count)
+        integ.sync_time()
+        _, t = o.steps(ref, count, 0.2, t, 1e9, kind=0 if td == "lw" else 1)
+        assert integ.t == pytest.approx(t, rel=1e-13)
+    a, b = integ.get_state().reshape(-1, 4), ref.reshape(-1, 4)
+    assert np.all(np.linalg.norm(a - b, axis=0) < 1e-12 * np.linalg.norm(b, axis=0))

@@ -1500,6 +1500,7 @@ int tlw_dd_finish(tlw_handle* h) {
     }
     TLW_CUDA(h, cudaGetLastError());
     h->cur ^= 1;
+    h->slots_valid = false;   // (an unpartitioned mesh may go on with tlw_step: these steps keep no CFL maximum)
     return TLW_OK;
 }
 
