@@ -39,13 +39,14 @@ using namespace tlw;
 namespace {
 
 // The adjoint kernels read and write the library's own arrays (segment states and traces, the adjoint states, the
-// face-trace adjoints), whose node records are 32-byte aligned: one 256-bit access per record.
+// face-trace adjoints), whose node records are 32-byte aligned: one 256-bit access per record. They are launched the
+// ordinary way, after everything in front of them has ended, so they may read it through the non-coherent path.
 #ifndef TLW_ADJ_WIDE
 #define TLW_ADJ_WIDE 1
 #endif
 __device__ __forceinline__ void aload4(const double* p, double* x) {
-    if (TLW_ADJ_WIDE) load4w(p, x);
-    else load4(p, x);
+    if (TLW_ADJ_WIDE) load4w_const(p, x);
+    else load4_const(p, x);
 }
 __device__ __forceinline__ void astore4(double* p, const double* x) {
     if (TLW_ADJ_WIDE) store4w(p, x);

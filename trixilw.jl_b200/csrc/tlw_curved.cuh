@@ -169,7 +169,7 @@ __device__ __forceinline__ void blend_curved_flux(const CurvedSurfArgs& a, int p
         fn[v] = 0.5 * ((fP[v] * nrm[0] + gP[v] * nrm[1]) + (fS[v] * nrm[0] + gS[v] * nrm[1])) + (-0.5 * lam * (uS[v] - uP[v]));
     load4(a.tFn + (((size_t)pe * 4 + pf) * n + l) * NV, fil);
     load4(a.tFn + (((size_t)se * 4 + sf) * n + l) * NV, fir);
-    const double alp = 0.5 * (__ldg(a.alpha + pe) + __ldg(a.alpha + se));
+    const double alp = 0.5 * (a.alpha[pe] + a.alpha[se]);
 #pragma unroll
     for (int v = 0; v < NV; ++v) Fn[v] = (1.0 - alp) * Fn[v] + alp * fn[v];
     const double dt = *a.dt;
@@ -212,7 +212,7 @@ __device__ __forceinline__ void blend_unstructured_flux(const CurvedSurfArgs& a,
         fn[v] = 0.5 * ((fP[v] * nrm[0] + gP[v] * nrm[1]) + (fS[v] * nrm[0] + gS[v] * nrm[1])) + (-0.5 * lam * (uS[v] - uP[v]));
     load4(a.tFn + (((size_t)pe * 4 + fn_low_slot(pf)) * n + l) * NV, fil);
     load4(a.tFn + (((size_t)se * 4 + fn_low_slot(sf)) * n + ls) * NV, fir);
-    double alp = 0.5 * (__ldg(a.alpha + pe) + __ldg(a.alpha + se));
+    double alp = 0.5 * (a.alpha[pe] + a.alpha[se]);
     const double dt = *a.dt;
     const double J = __ldg(a.inv_jac + (size_t)pe * nn + np);
     double Fb[NV], low[NV];
@@ -279,7 +279,7 @@ __device__ __forceinline__ void curved_interface_flux(const CurvedSurfArgs& a, i
     } else {
         load4w(a.tF + tp, FP);
         load4w(a.tF + ts, FS);
-        load4w(a.metrics + ((size_t)pe * nn + np) * 4, J);
+        load4w_const(a.metrics + ((size_t)pe * nn + np) * 4, J);
         const double nrm[2] = {sgP * (pf < 2 ? J[0] : J[2]), sgP * (pf < 2 ? J[1] : J[3])};
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
@@ -323,11 +323,11 @@ static __global__ void __launch_bounds__(128) curved_interface_kernel(CurvedSurf
     double* oP = a.out + ((size_t)pe * nn + np) * NV;
     double* oS = a.out + ((size_t)se * nn + ns) * NV;
     double x[NV];
-    load4w_rw(oP, x);
+    load4w(oP, x);
 #pragma unroll
     for (int v = 0; v < NV; ++v) x[v] = fma(cP, Fn[v], x[v]);
     store4w(oP, x);
-    load4w_rw(oS, x);
+    load4w(oS, x);
 #pragma unroll
     for (int v = 0; v < NV; ++v) x[v] = fma(cS, Fn[v], x[v]);
     store4w(oS, x);
@@ -380,7 +380,7 @@ __device__ __forceinline__ void curved_boundary_flux(const CurvedBndArgs& a, int
     const size_t tb = (((size_t)e * 4 + f) * n + l) * NV;
     load4w(a.tU + tb, Ui);
     load4w(a.tF + tb, Fi);
-    load4w(a.metrics + ((size_t)e * nn + node) * 4, J);
+    load4w_const(a.metrics + ((size_t)e * nn + node) * 4, J);
     const double nrm[2] = {sg * (f < 2 ? J[0] : J[2]), sg * (f < 2 ? J[1] : J[3])};
 #pragma unroll
     for (int v = 0; v < NV; ++v) Fi[v] *= sg;
@@ -393,7 +393,7 @@ __device__ __forceinline__ void curved_boundary_flux(const CurvedBndArgs& a, int
         for (int v = 0; v < NV; ++v) Uo[v] = Fo[v] = 0.0;
         for (int q = 0; q < n; ++q) {
             double ub[NV], fx[NV], gy[NV];
-            load4(a.levels + (((size_t)b * n + l) * n + q) * NV, ub);
+            load4_const(a.levels + (((size_t)b * n + l) * n + q) * NV, ub);
             euler_fluxes(gm1, ub[0], ub[1], ub[2], ub[3], fx, gy);
             const double w = a.scaling_factor * a.weights[q] / 2.0;
 #pragma unroll
@@ -440,7 +440,7 @@ static __global__ void __launch_bounds__(128) curved_boundary_kernel(CurvedBndAr
     const double c = -dts * __ldg(a.inv_jac + (size_t)e * nn + node) * ((f & 1) ? a.inv_w_last : a.inv_w_first);
     double* o = a.out + ((size_t)e * nn + node) * NV;
     double x[NV];
-    load4_rw(o, x);
+    load4(o, x);
 #pragma unroll
     for (int v = 0; v < NV; ++v) x[v] = fma(c, Fn[v], x[v]);
     store4(o, x);
@@ -495,8 +495,8 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, TLW_CURVED_MINB)
         face_node_of_thread<n>(b, i2, j2);
         const size_t node = (size_t)e2 * nn + i2 + n * j2;
         double x[NV];
-        load4w_rw(a.out + node * NV, x);
-        if (a.cfl_max && b == 0) in = __ldg(reinterpret_cast<const double2*>(a.cfl_interior) + e2);
+        load4w(a.out + node * NV, x);
+        if (a.cfl_max && b == 0) in = reinterpret_cast<const double2*>(a.cfl_interior)[e2];
         const double ij = __ldg(a.inv_jac + node);
         const double c = -(a.step_mode ? *a.dt : 1.0) * ij;
         const double* F = sF + el2 * 4 * n * NV;
@@ -515,7 +515,7 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, TLW_CURVED_MINB)
         store4w(a.out + node * NV, x);
         if (a.cfl_max) {
             double J[4];
-            load4w(a.metrics + node * 4, J);
+            load4w_const(a.metrics + node * 4, J);
             node_speeds(a.gamma, x, a.speed_status, l1, l2);
             curved_speeds(J, ij, l1, l2);
         }
@@ -531,7 +531,7 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, TLW_CURVED_MINB)
 // max_nodes |Ja^2 . (l1, l2)| |J^{-1}|, l_d = |v_d| + c. A CTA takes MsCfg<N>::ELEMS elements: a coalesced pass
 // over their nodes into shared memory, then one thread per element reduces its nodes.
 template <int N>
-static __global__ void __launch_bounds__(MS_THREADS) curved_max_speed_kernel(const double* __restrict__ u,
+static __global__ void __launch_bounds__(MS_THREADS) curved_max_speed_kernel(const double* u,
                                                                              const double* __restrict__ metrics,
                                                                              const double* __restrict__ inv_jac,
                                                                              int E, double gamma, StepState* s,
@@ -554,10 +554,10 @@ static __global__ void __launch_bounds__(MS_THREADS) curved_max_speed_kernel(con
     for_nodes(ne * nn, [&](int k, int k2, bool both) {
         double x[NV], y[NV], J[4], J2[4];
         load4w(u + ((size_t)e0 * nn + k) * NV, x);
-        load4w(metrics + ((size_t)e0 * nn + k) * 4, J);
+        load4w_const(metrics + ((size_t)e0 * nn + k) * 4, J);
         if (both) {
             load4w(u + ((size_t)e0 * nn + k2) * NV, y);
-            load4w(metrics + ((size_t)e0 * nn + k2) * 4, J2);
+            load4w_const(metrics + ((size_t)e0 * nn + k2) * 4, J2);
         }
         one(k, x, J);
         if (both) one(k2, y, J2);

@@ -83,7 +83,7 @@ static __global__ void __launch_bounds__(128) curved_mortar_kernel(CurvedMortarA
         load4(a.tF + ts, Fs);
 #pragma unroll
         for (int v = 0; v < NV; ++v) Fs[v] *= sgS;   // F_S . n_S
-        load4(a.metrics + ((size_t)se * nn + ns) * 4, J);
+        load4_const(a.metrics + ((size_t)se * nn + ns) * 4, J);
         const double nrm[2] = {sgS * (sf < 2 ? J[0] : J[2]), sgS * (sf < 2 ? J[1] : J[3])};
         const double* fwd = c_tlw_mortar[N][h ? 0 : 1];
         double fir[NV] = {0, 0, 0, 0};
@@ -94,7 +94,7 @@ static __global__ void __launch_bounds__(128) curved_mortar_kernel(CurvedMortarA
             double x[NV], y[NV], z[NV], JL[4];
             load4(a.u + ((size_t)lg * nn + nl) * NV, x);
             load4(a.tU + (((size_t)lg * 4 + lf) * n + li) * NV, y);
-            load4(a.metrics + ((size_t)lg * nn + nl) * 4, JL);
+            load4_const(a.metrics + ((size_t)lg * nn + nl) * 4, JL);
             const double nL[2] = {-0.5 * (sgL * (lf < 2 ? JL[0] : JL[2])), -0.5 * (sgL * (lf < 2 ? JL[1] : JL[3]))};
             euler_flux_normal(gm1, x, nL, z);
             const double c = fwd[l * n + i];
@@ -122,7 +122,7 @@ static __global__ void __launch_bounds__(128) curved_mortar_kernel(CurvedMortarA
                 fn[v] = 0.5 * ((fS[v] * nrm[0] + gS[v] * nrm[1]) + (fL[v] * nrm[0] + gL[v] * nrm[1])) +
                         (-0.5 * lam * (ul[v] - us[v]));
             load4(a.tFn + ts, fil);
-            const double alp = 0.5 * (__ldg(a.alpha + se) + __ldg(a.alpha + lg));
+            const double alp = 0.5 * (a.alpha[se] + a.alpha[lg]);
 #pragma unroll
             for (int v = 0; v < NV; ++v) fstar[v] = (1.0 - alp) * fstar[v] + alp * fn[v];
             const double dt = *a.dt;
@@ -146,7 +146,7 @@ static __global__ void __launch_bounds__(128) curved_mortar_kernel(CurvedMortarA
         const double cs = -dts * __ldg(a.inv_jac + (size_t)se * nn + ns) * ((sf & 1) ? a.inv_w_last : a.inv_w_first);
         double* os = a.out + ((size_t)se * nn + ns) * NV;
         double x[NV];
-        load4_rw(os, x);
+        load4(os, x);
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
             x[v] = fma(cs, fstar[v], x[v]);
@@ -168,7 +168,7 @@ static __global__ void __launch_bounds__(128) curved_mortar_kernel(CurvedMortarA
         const double cl = -dts * __ldg(a.inv_jac + (size_t)lg * nn + nl) * ((lf & 1) ? a.inv_w_last : a.inv_w_first);
         double* ol = a.out + ((size_t)lg * nn + nl) * NV;
         double x[NV];
-        load4_rw(ol, x);
+        load4(ol, x);
 #pragma unroll
         for (int v = 0; v < NV; ++v) x[v] = fma(cl, -2.0 * p[v], x[v]);
         store4(ol, x);

@@ -241,7 +241,7 @@ __device__ __forceinline__ double begin_step_dt(StepState* s, unsigned long long
     const unsigned late_bits = write ? *late : 0u;
     unsigned long long bits = 0ull;
 #pragma unroll
-    for (int k = 0; k < RING_WAYS; ++k) bits = max(bits, __ldg(ring + k * RING_STRIDE));
+    for (int k = 0; k < RING_WAYS; ++k) bits = max(bits, ring[k * RING_STRIDE]);
     bool finished;
     const double dt = step_size(s, bits, n, finished);
     if (write) {
@@ -332,14 +332,21 @@ inline cudaError_t zero_on(cudaStream_t s, void* dst, size_t bytes) {
     return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
 }
 
-__device__ __forceinline__ void load4(const double* __restrict__ p, double* x) {
-    const double2 a = __ldg(reinterpret_cast<const double2*>(p));
-    const double2 b = __ldg(reinterpret_cast<const double2*>(p) + 1);
-    x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
-}
-__device__ __forceinline__ void load4_rw(const double* p, double* x) {
+// What a kernel of the same chain wrote (states, traces, gradients, blending factors, CFL maxima) is read by load4,
+// load4w and plain loads: coherent, and ordered after wait_for_previous, which clobbers memory (load4w is a volatile
+// asm that does too). load4_const, load4w_const and __ldg read through the non-coherent path, whose data must not
+// change while the kernel lives, and which a compiler may move above the wait: for what the host uploaded (metrics,
+// Jacobians, connectivity, boundary data) and for kernels that are only launched the ordinary way. The coherent loads
+// cost nothing, a pass with .nc loads against one without: 512^2, N = 4, 8 steps 5071 / 5071 us, MDRK 256^2 1837 / 1838,
+// warped 201 x 167 878 / 878, Riemann 256^2 1763 / 1764, cavity 64^2 836 / 835.
+__device__ __forceinline__ void load4(const double* p, double* x) {
     const double2 a = *reinterpret_cast<const double2*>(p);
     const double2 b = *(reinterpret_cast<const double2*>(p) + 1);
+    x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+}
+__device__ __forceinline__ void load4_const(const double* p, double* x) {
+    const double2 a = __ldg(reinterpret_cast<const double2*>(p));
+    const double2 b = __ldg(reinterpret_cast<const double2*>(p) + 1);
     x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
 }
 __device__ __forceinline__ void store4(double* p, const double* x) {
@@ -349,14 +356,14 @@ __device__ __forceinline__ void store4(double* p, const double* x) {
 // One 256-bit access per 4-double node record (global memory only; the record 32-byte aligned): the surface
 // pass, the interface sweeps, the curvilinear interfaces, the CFL / indicator passes and the adjoint kernels,
 // whose arrays are the library's own or were checked (or copied) by the entry point.
-__device__ __forceinline__ void load4w(const double* __restrict__ p, double* x) {
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3]) : "l"(p));
-}
-__device__ __forceinline__ void load4w_rw(const double* p, double* x) {
+__device__ __forceinline__ void load4w(const double* p, double* x) {
     asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
                  : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3])
                  : "l"(p)
                  : "memory");
+}
+__device__ __forceinline__ void load4w_const(const double* p, double* x) {
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(x[0]), "=d"(x[1]), "=d"(x[2]), "=d"(x[3]) : "l"(p));
 }
 __device__ __forceinline__ void store4w(double* p, const double* x) {
     asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(x[0]), "d"(x[1]), "d"(x[2]), "d"(x[3])

@@ -80,7 +80,7 @@ static __global__ void __launch_bounds__(128) halo_pack_kernel(HaloArgs a) {
     if (a.alpha) {
         load4(a.tFn + tb, x);
         store4(s + 3 * NV, x);
-        s[4 * NV] = __ldg(a.alpha + e);
+        s[4 * NV] = a.alpha[e];
     }
 }
 
@@ -111,7 +111,7 @@ static __global__ void __launch_bounds__(128) halo_face_kernel(HaloArgs a) {
         double fl[NV], fr[NV];
         load4(a.tFn + tb, fl);
         load4(r + 3 * NV, fr);
-        const double al = __ldg(a.alpha + e), ar = r[4 * NV];
+        const double al = a.alpha[e], ar = r[4 * NV];
         if (local_left)
             blend_flux_values(a.gamma, a.speed_kind, a.status, a.jac_first, a.inv_w_first, a.inv_w_last, a.orientation, ul,
                               ur, al, ar, fl, fr, *a.dt, Fn);
@@ -125,7 +125,7 @@ static __global__ void __launch_bounds__(128) halo_face_kernel(HaloArgs a) {
     const double c = local_left ? -ij * a.inv_w_last * dts : ij * a.inv_w_first * dts;
     double* o = a.out + ((size_t)e * nn + node) * NV;
     double x[NV];
-    load4_rw(o, x);
+    load4(o, x);
 #pragma unroll
     for (int v = 0; v < NV; ++v) x[v] = fma(c, Fn[v], x[v]);
     store4(o, x);
@@ -135,7 +135,7 @@ static __global__ void __launch_bounds__(128) halo_face_kernel(HaloArgs a) {
 static __global__ void halo_alpha_pack_kernel(const int* __restrict__ elem, const int* __restrict__ slot, int count,
                                               const double* __restrict__ alpha_raw, double* __restrict__ send) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < count) send[__ldg(slot + k)] = __ldg(alpha_raw + __ldg(elem + k));
+    if (k < count) send[__ldg(slot + k)] = alpha_raw[__ldg(elem + k)];
 }
 
 // alpha_e = max(alpha_e, alpha_raw_remote / 2) across the cut faces (the smoothing of alpha_smooth_kernel)
@@ -144,7 +144,7 @@ static __global__ void halo_alpha_smooth_kernel(const int* __restrict__ elem, co
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     unsigned long long* ab = reinterpret_cast<unsigned long long*>(alpha);
-    atomicMax(ab + __ldg(elem + k), (unsigned long long)__double_as_longlong(0.5 * __ldg(recv + __ldg(slot + k))));
+    atomicMax(ab + __ldg(elem + k), (unsigned long long)__double_as_longlong(0.5 * recv[__ldg(slot + k)]));
 }
 
 }  // namespace tlw

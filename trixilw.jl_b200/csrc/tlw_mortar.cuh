@@ -134,7 +134,7 @@ static __global__ void __launch_bounds__(128) mortar_kernel(MortarArgs a) {
         const double cs = left ? dts * __ldg(a.inv_jac + se) * a.inv_w_first : -dts * __ldg(a.inv_jac + se) * a.inv_w_last;
         double* os = a.out + ((size_t)se * nn + ns) * NV;
         double x[NV];
-        load4_rw(os, x);
+        load4(os, x);
 #pragma unroll
         for (int v = 0; v < NV; ++v) {
             x[v] = fma(cs, fstar[v], x[v]);
@@ -149,7 +149,7 @@ static __global__ void __launch_bounds__(128) mortar_kernel(MortarArgs a) {
         const double cl = left ? -dts * __ldg(a.inv_jac + lg) * a.inv_w_last : dts * __ldg(a.inv_jac + lg) * a.inv_w_first;
         double* ol = a.out + ((size_t)lg * nn + tree_face_node(n, large_face, l)) * NV;
         double x[NV];
-        load4_rw(ol, x);
+        load4(ol, x);
 #pragma unroll
         for (int v = 0; v < NV; ++v) x[v] = fma(cl, p[v], x[v]);
         store4(ol, x);

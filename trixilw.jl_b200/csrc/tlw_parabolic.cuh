@@ -93,7 +93,7 @@ __device__ __forceinline__ void wall_value(double gamma, const double* ui, int k
 // or the wall's) before it stores the gradients: one launch instead of one per colour and boundary class, each of which
 // read and wrote the face nodes' gradients again (64 x 64 cavity, N = 4: five launches, 30 us, in one of 10).
 template <int N, bool CURVED = false, bool FACES = false>
-static __global__ void __launch_bounds__(VolCfg<N>::THREADS) grad_volume_kernel(const double* __restrict__ u,
+static __global__ void __launch_bounds__(VolCfg<N>::THREADS) grad_volume_kernel(const double* u,
                                                                               const double* __restrict__ inv_jac,
                                                                               int E, double* gx, double* gy,
                                                                               const double* __restrict__ metrics = nullptr,
@@ -119,7 +119,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS) grad_volume_kernel(
     if (!active) return;
     const double ij = CURVED ? __ldg(inv_jac + (size_t)e * nn + node) : __ldg(inv_jac + e);
     double J[4] = {1.0, 0.0, 0.0, 1.0};
-    if (CURVED) load4w(metrics + ((size_t)e * nn + node) * 4, J);
+    if (CURVED) load4w_const(metrics + ((size_t)e * nn + node) * 4, J);
     double ox[NV], oy[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
@@ -210,11 +210,11 @@ static __global__ void __launch_bounds__(128) grad_interface_kernel(const double
     const double cL = __ldg(inv_jac + le) * inv_w_last, cR = -__ldg(inv_jac + re) * inv_w_first;
     double* pL = g + ((size_t)le * nn + nL) * NV;
     double* pR = g + ((size_t)re * nn + nR) * NV;
-    load4_rw(pL, x);
+    load4(pL, x);
 #pragma unroll
     for (int v = 0; v < NV; ++v) x[v] = fma(cL, 0.5 * (uL[v] + uR[v]), x[v]);
     store4(pL, x);
-    load4_rw(pR, x);
+    load4(pR, x);
 #pragma unroll
     for (int v = 0; v < NV; ++v) x[v] = fma(cR, 0.5 * (uL[v] + uR[v]), x[v]);
     store4(pR, x);
@@ -256,7 +256,7 @@ static __global__ void __launch_bounds__(128) grad_boundary_kernel(const double*
     wall_value(gamma, ui, __ldg(wall_kind + k), wall + 3 * ((size_t)k * n + l), uo);
     double* g = (dir <= 2 ? gx : gy) + ((size_t)e * nn + node) * NV;
     const double c = (dir % 2 == 0 ? inv_w_last : -inv_w_first) * __ldg(inv_jac + e);
-    load4_rw(g, x);
+    load4(g, x);
 #pragma unroll
     for (int v = 0; v < NV; ++v) x[v] = fma(c, uo[v], x[v]);
     store4(g, x);
@@ -270,14 +270,14 @@ __device__ __forceinline__ void curved_grad_lift(const double* __restrict__ metr
                                                  double* gx, double* gy) {
     const int nn = n * n;
     double J[4], x[NV], y[NV];
-    load4(metrics + ((size_t)e * nn + node) * 4, J);
+    load4_const(metrics + ((size_t)e * nn + node) * 4, J);
     const double sg = (f & 1) ? 1.0 : -1.0;
     const double c = iw * __ldg(inv_jac + (size_t)e * nn + node);
     const double n0 = sg * (f < 2 ? J[0] : J[2]) * c, n1 = sg * (f < 2 ? J[1] : J[3]) * c;
     double* px = gx + ((size_t)e * nn + node) * NV;
     double* py = gy + ((size_t)e * nn + node) * NV;
-    load4_rw(px, x);
-    load4_rw(py, y);
+    load4(px, x);
+    load4(py, y);
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         x[v] = fma(n0, us[v], x[v]);
@@ -420,7 +420,7 @@ static __global__ void __launch_bounds__(ParCfg<N>::THREADS, ParCfg<N>::MIN_BLOC
         load4w(a.gy + ((size_t)e * nn + node) * NV, gy);
         if (CURVED) {
             ij = __ldg(a.inv_jac + (size_t)e * nn + node);
-            load4w(a.metrics + ((size_t)e * nn + node) * 4, J);
+            load4w_const(a.metrics + ((size_t)e * nn + node) * 4, J);
         } else {
             ij = __ldg(a.inv_jac + e);
         }
@@ -644,7 +644,7 @@ static __global__ void __launch_bounds__(MS_THREADS) par_speed_kernel(const doub
 // parabolic maxima (adv_bits, visc_bits; inv_jac_lin read by the element-linear index, as that kernel reads it)
 // in one pass over u, with the same operations for each.
 template <int N>
-static __global__ void __launch_bounds__(MS_THREADS) curved_par_speed_kernel(const double* __restrict__ u,
+static __global__ void __launch_bounds__(MS_THREADS) curved_par_speed_kernel(const double* u,
                                                                              const double* __restrict__ metrics,
                                                                              const double* __restrict__ inv_jac,
                                                                              int E, NSParams ns, StepState* s,
@@ -673,10 +673,10 @@ static __global__ void __launch_bounds__(MS_THREADS) curved_par_speed_kernel(con
     for_nodes(ne * nn, [&](int k, int k2, bool both) {
         double x[NV], y[NV], J[4], J2[4];
         load4w(u + ((size_t)e0 * nn + k) * NV, x);
-        load4w(metrics + ((size_t)e0 * nn + k) * 4, J);
+        load4w_const(metrics + ((size_t)e0 * nn + k) * 4, J);
         if (both) {
             load4w(u + ((size_t)e0 * nn + k2) * NV, y);
-            load4w(metrics + ((size_t)e0 * nn + k2) * 4, J2);
+            load4w_const(metrics + ((size_t)e0 * nn + k2) * 4, J2);
         }
         one(k, x, J);
         if (both) one(k2, y, J2);

@@ -107,7 +107,7 @@ __device__ __forceinline__ void blend_interface_flux(const SurfArgs& a, int orie
     load4(a.tFn + (((size_t)le * 4 + faceL) * n + l) * NV, fil);
     load4(a.tFn + (((size_t)re * 4 + faceR) * n + l) * NV, fir);
     blend_flux_values(a.gamma, a.speed_kind, a.status, a.jac_first, a.inv_w_first, a.inv_w_last, orientation, uL, uR,
-                      __ldg(a.alpha + le), __ldg(a.alpha + re), fil, fir, dt, Fn);
+                      a.alpha[le], a.alpha[re], fil, fir, dt, Fn);
 }
 
 // The LW flux at node l of the interface (le, re) of one orientation, with the blending and the viscous
@@ -168,7 +168,7 @@ static __global__ void __launch_bounds__(256) interface_kernel(SurfArgs a) {
     const bool slots = a.cfl_slots && (a.orientation == 2 || (l > 0 && l < n - 1));
     const int sL_slot = a.orientation == 1 ? 2 : 4, sR_slot = a.orientation == 1 ? 1 : 3;
     double x[NV], l1, l2;
-    load4w_rw(oL, x);
+    load4w(oL, x);
 #pragma unroll
     for (int v = 0; v < NV; ++v) x[v] = fma(sL, Fn[v], x[v]);
     store4w(oL, x);
@@ -177,7 +177,7 @@ static __global__ void __launch_bounds__(256) interface_kernel(SurfArgs a) {
         atomicMax(a.cfl_slots + (size_t)le * CFL_SLOTS + 2 * sL_slot, (unsigned long long)__double_as_longlong(l1));
         atomicMax(a.cfl_slots + (size_t)le * CFL_SLOTS + 2 * sL_slot + 1, (unsigned long long)__double_as_longlong(l2));
     }
-    load4w_rw(oR, x);
+    load4w(oR, x);
 #pragma unroll
     for (int v = 0; v < NV; ++v) x[v] = fma(sR, Fn[v], x[v]);
     store4w(oR, x);
@@ -252,7 +252,7 @@ __device__ __forceinline__ void boundary_node_flux(const BndArgs& a, int k, int 
     if (kind == BC_DIRICHLET) {
         for (int q = 0; q < n; ++q) {
             double ub[NV], fb[NV];
-            load4(a.levels + (((size_t)k * n + l) * n + q) * NV, ub);
+            load4_const(a.levels + (((size_t)k * n + l) * n + q) * NV, ub);
             euler_flux_dir(gm1, ub, orientation, fb);
             const double w = 0.5 * a.scaling_factor;
 #pragma unroll
@@ -261,7 +261,7 @@ __device__ __forceinline__ void boundary_node_flux(const BndArgs& a, int k, int 
                 Fo[v] += w * fb[v] * a.weights[q];
             }
         }
-        load4(a.now + ((size_t)k * n + l) * NV, uo);
+        load4_const(a.now + ((size_t)k * n + l) * NV, uo);
     } else {
         slip_wall_exterior(kind, Fi, Ui, ui, Fo, Uo, uo);
     }
@@ -303,7 +303,7 @@ static __global__ void __launch_bounds__(128) boundary_kernel(BndArgs a) {
     const double s = (dir % 2 == 0) ? -ij * a.inv_w_last * dts : ij * a.inv_w_first * dts;
     double* o = a.out + ((size_t)e * n * n + node) * NV;
     double x[NV];
-    load4_rw(o, x);
+    load4(o, x);
 #pragma unroll
     for (int v = 0; v < NV; ++v) x[v] = fma(s, Fn[v], x[v]);
     store4(o, x);
@@ -435,7 +435,7 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, SC ? SurfCfg<N>::S
     face_node_of_thread<n>(b, i2, j2);
     double* o2 = a.out + ((size_t)e2 * n * n + i2 + n * j2) * NV;
     double x[NV];
-    if (TLW_SURF_PREFETCH && has2) load4w_rw(o2, x);
+    if (TLW_SURF_PREFETCH && has2) load4w(o2, x);
     {
         const int el = tid / (4 * n), r = tid - el * 4 * n, f = r / n, l = r - f * n, e = e0 + el;
         if (el < EB && e < a.E) {
@@ -475,9 +475,9 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, SC ? SurfCfg<N>::S
     double l1 = 0.0, l2 = 0.0, ij = 0.0;
     double2 in = make_double2(0.0, 0.0);
     if (has2) {
-        if (!TLW_SURF_PREFETCH) load4w_rw(o2, x);
+        if (!TLW_SURF_PREFETCH) load4w(o2, x);
         // (with the face node, not where it is needed: the CTA's end would wait for it)
-        if (a.cfl_max && b == 0) in = __ldg(reinterpret_cast<const double2*>(a.cfl_interior) + e2);
+        if (a.cfl_max && b == 0) in = reinterpret_cast<const double2*>(a.cfl_interior)[e2];
         const double dt = a.inst ? a.dt[__ldg(a.inst + e2)] : *a.dt;
         const double dts = a.step_mode ? dt : 1.0;
         ij = __ldg(a.inv_jac + e2);
@@ -583,7 +583,7 @@ struct BatchSpeedArgs {
 // CSPEED (curvilinear meshes): the speeds of curved_max_speed_kernel, |Ja^d . (l1, l2)| |J^{-1}| per node, and the
 // element's value max l1 + max l2 without the element J^{-1}
 template <int N, bool SPEED, bool IND, bool CSPEED = false>
-static __global__ void __launch_bounds__(MS_THREADS) max_speed_kernel(const double* __restrict__ u,
+static __global__ void __launch_bounds__(MS_THREADS) max_speed_kernel(const double* u,
                                                                const double* __restrict__ inv_jac, int E,
                                                                double gamma, StepState* s, IndicatorArgs ia,
                                                                BatchSpeedArgs bs) {
@@ -614,8 +614,8 @@ static __global__ void __launch_bounds__(MS_THREADS) max_speed_kernel(const doub
         load4w(u + ((size_t)e0 * nn + k) * NV, x);
         if (both) load4w(u + ((size_t)e0 * nn + k2) * NV, y);
         if (SPEED && CSPEED) {
-            load4w(ia.metrics + ((size_t)e0 * nn + k) * 4, J);
-            if (both) load4w(ia.metrics + ((size_t)e0 * nn + k2) * 4, J2);
+            load4w_const(ia.metrics + ((size_t)e0 * nn + k) * 4, J);
+            if (both) load4w_const(ia.metrics + ((size_t)e0 * nn + k2) * 4, J2);
         }
         one(k, x, J);
         if (both) one(k2, y, J2);
@@ -741,15 +741,15 @@ static __global__ void batch_finalize_dt_kernel(BatchTime b) {
 // Trixi apply_smoothing! (TreeMesh{2}): alpha_e = max(alpha_e, alpha_raw_nb / 2) over the interfaces,
 // independent of the order (max over non-negative doubles = max over their bit patterns)
 static __global__ void alpha_smooth_kernel(const int* __restrict__ left, const int* __restrict__ right, int count,
-                                    const double* __restrict__ alpha_raw, double* alpha) {
+                                    const double* alpha_raw, double* alpha) {
     wait_for_previous();
     dependents_may_start();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const int l = __ldg(left + k), r = __ldg(right + k);
     unsigned long long* ab = reinterpret_cast<unsigned long long*>(alpha);
-    atomicMax(ab + l, (unsigned long long)__double_as_longlong(0.5 * __ldg(alpha_raw + r)));
-    atomicMax(ab + r, (unsigned long long)__double_as_longlong(0.5 * __ldg(alpha_raw + l)));
+    atomicMax(ab + l, (unsigned long long)__double_as_longlong(0.5 * alpha_raw[r]));
+    atomicMax(ab + r, (unsigned long long)__double_as_longlong(0.5 * alpha_raw[l]));
 }
 
 // dt of the step from the CFL maximum in max_bits, and the time after it
@@ -785,8 +785,8 @@ static __global__ void __launch_bounds__(256) cfl_slots_reduce_kernel(const unsi
         unsigned long long b1 = 0ull, b2 = 0ull;
 #pragma unroll
         for (int k = 0; k < CFL_SLOTS / 2; ++k) {
-            b1 = max(b1, __ldg(sl + 2 * k));
-            b2 = max(b2, __ldg(sl + 2 * k + 1));
+            b1 = max(b1, sl[2 * k]);
+            b2 = max(b2, sl[2 * k + 1]);
         }
         m = fmax(m, __ldg(inv_jac + e) * (__longlong_as_double((long long)b1) + __longlong_as_double((long long)b2)));
     }

@@ -889,7 +889,7 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
     double alpha_e = 0.0, fx[NV], fy[NV];
     bool blended = false, muscl = false;
     if (SC && active) {
-        alpha_e = __ldg(a.alpha + e);
+        alpha_e = a.alpha[e];
         blended = CURVED ? !(fabs(alpha_e) <= 1e-12) : alpha_e != 0.0;
         muscl = CURVED && REC >= 1 && blended && !__ldg(a.atb + e);
     }
@@ -916,7 +916,7 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
     auto put = [&](const double* f, const double* g) {
         if (CURVED) {
             double ft[NV], gt[NV], Ja[4];
-            load4w(a.metrics + ((size_t)e * nn + node) * 4, Ja);
+            load4w_const(a.metrics + ((size_t)e * nn + node) * 4, Ja);
             contravariant(Ja, f, g, ft, gt);
             line_put<N, C>(X, Y, el, i, j, ft, gt);
         } else {
@@ -1074,7 +1074,7 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
             // the surface needs the normal fluxes: keep the contravariant time averages F~, G~ (their face
             // values are F . Ja^1 and F . Ja^2)
             double ft[NV], gt[NV], Ja[4];
-            load4w(a.metrics + ((size_t)e * nn + node) * 4, Ja);
+            load4w_const(a.metrics + ((size_t)e * nn + node) * 4, Ja);
             contravariant(Ja, F, G, ft, gt);
 #pragma unroll
             for (int v = 0; v < NV; ++v) { F[v] = ft[v]; G[v] = gt[v]; }
@@ -1109,7 +1109,7 @@ static __global__ void __launch_bounds__(VolCfg<N, EBX>::THREADS, (SC && CURVED)
             if (CURVED) {
                 const size_t k = (size_t)e * nn + node;
                 double Jn[4];
-                load4w(a.metrics + k * 4, Jn);
+                load4w_const(a.metrics + k * 4, Jn);
                 curved_speeds(Jn, __ldg(a.inv_jac_node + k), l1, l2);
             }
         }
@@ -1216,7 +1216,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     double alpha_e = 0.0, fx[NV], fy[NV];
     bool blended = false, muscl = false;
     if (SC && active) {
-        alpha_e = __ldg(a.alpha + e);
+        alpha_e = a.alpha[e];
         blended = CURVED ? !(fabs(alpha_e) <= 1e-12) : alpha_e != 0.0;
         muscl = CURVED && REC >= 1 && blended && !__ldg(a.atb + e);
     }
@@ -1238,7 +1238,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     if (active) {
         load4w(a.u + ((size_t)e * nn + node) * NV, uu);
         if (CURVED) {
-            load4w(a.metrics + ((size_t)e * nn + node) * 4, Ja);
+            load4w_const(a.metrics + ((size_t)e * nn + node) * 4, Ja);
             ij = __ldg(a.inv_jac_node + (size_t)e * nn + node);
         } else {
             ij = __ldg(a.inv_jac + e);
@@ -1377,7 +1377,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
     double alpha_e = 0.0, fx[NV], fy[NV];
     bool blended = false, muscl = false;
     if (SC && active) {
-        alpha_e = __ldg(a.alpha + e);
+        alpha_e = a.alpha[e];
         blended = CURVED ? !(fabs(alpha_e) <= 1e-12) : alpha_e != 0.0;
         muscl = CURVED && REC >= 1 && blended && !__ldg(a.atb + e);
     }
@@ -1390,7 +1390,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
         double f[NV], g[NV];
         load4w(a.u + ((size_t)e * nn + node) * NV, us);
         if (CURVED) {
-            load4w(a.metrics + ((size_t)e * nn + node) * 4, Ja);
+            load4w_const(a.metrics + ((size_t)e * nn + node) * 4, Ja);
             ij = __ldg(a.inv_jac_node + (size_t)e * nn + node);
         } else {
             ij = __ldg(a.inv_jac + e);
@@ -1504,7 +1504,7 @@ static __global__ void __launch_bounds__(VolCfg<N>::THREADS, (SC && CURVED) ? Vo
             if (CURVED) {
                 const size_t k = (size_t)e * nn + node;
                 double Jn[4];
-                load4w(a.metrics + k * 4, Jn);
+                load4w_const(a.metrics + k * 4, Jn);
                 curved_speeds(Jn, __ldg(a.inv_jac_node + k), l1, l2);
             }
         }
