@@ -2202,31 +2202,33 @@ int tlw_step(tlw_handle* h, int32_t nsteps, double cfl, double fixed_dt, double 
         if (e2 != cudaSuccess) { exec = nullptr; return fail(h, TLW_E_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e2)); }
         return TLW_OK;
     };
-    // capture every variant on first use, so that no capture/instantiation lands inside a later call
+    // the graphs of one and two steps on first use, so that no capture of theirs falls into a later call
     if ((rc = capture(0, 1, h->g_one[0])) || (rc = capture(1, 1, h->g_one[1])) || (rc = capture(0, 2, h->g_two[0])))
         return rc;
     int left = nsteps;
-    h->replayed += left;
+    auto replay = [&](cudaGraphExec_t exec, int count) -> int {
+        TLW_CUDA(h, cudaGraphLaunch(exec, h->stream));
+        left -= count;
+        h->replayed += count;
+        return TLW_OK;
+    };
     if (h->cur == 1) {
-        if ((rc = capture(1, 1, h->g_one[1]))) return rc;
-        TLW_CUDA(h, cudaGraphLaunch(h->g_one[1], h->stream));
+        if ((rc = replay(h->g_one[1], 1))) return rc;
         h->cur = 0;
-        --left;
     }
-    // long runs in graphs of many steps (the gap between two graphs falls between fewer steps), once the steps replayed
-    // have paid for their capture
+    // long runs in graphs of many steps (the gap between two graphs falls between fewer steps), captured once this call has
+    // enough steps in front of the capture to hide it, or the handle has replayed enough to have earned it
     constexpr int many = tlw_handle::MANY_STEPS;
-    if (left >= many && h->replayed >= tlw_handle::MANY_AFTER) {
-        if ((rc = capture(0, many, h->g_many))) return rc;
-        for (; left >= many; left -= many) TLW_CUDA(h, cudaGraphLaunch(h->g_many, h->stream));
-    }
-    if (left >= 2) {
-        if ((rc = capture(0, 2, h->g_two[0]))) return rc;
-        for (; left >= 2; left -= 2) TLW_CUDA(h, cudaGraphLaunch(h->g_two[0], h->stream));
+    while (left >= 2) {
+        const bool long_run = h->g_many || nsteps - left >= tlw_handle::MANY_QUEUED || h->replayed >= tlw_handle::MANY_AFTER;
+        if (left >= many && long_run) {
+            if ((rc = capture(0, many, h->g_many)) || (rc = replay(h->g_many, many))) return rc;
+        } else if ((rc = replay(h->g_two[0], 2))) {
+            return rc;
+        }
     }
     if (left == 1) {
-        if ((rc = capture(0, 1, h->g_one[0]))) return rc;
-        TLW_CUDA(h, cudaGraphLaunch(h->g_one[0], h->stream));
+        if ((rc = replay(h->g_one[0], 1))) return rc;
         h->cur = 1;
     }
     return TLW_OK;
