@@ -77,10 +77,10 @@ static __global__ void __launch_bounds__(128) curved_mortar_kernel(CurvedMortarA
         const int ns = face_node_index(n, sf, l);
         const double sgS = (sf & 1) ? 1.0 : -1.0, sgL = (lf & 1) ? 1.0 : -1.0;
         double us[NV], Us[NV], Fs[NV], ul[NV] = {0, 0, 0, 0}, Ul[NV] = {0, 0, 0, 0}, Fl[NV] = {0, 0, 0, 0}, J[4];
-        load4(a.u + ((size_t)se * nn + ns) * NV, us);
+        load4_const(a.u + ((size_t)se * nn + ns) * NV, us);
         const size_t ts = (((size_t)se * 4 + sf) * n + l) * NV;
-        load4(a.tU + ts, Us);
-        load4(a.tF + ts, Fs);
+        load4_const(a.tU + ts, Us);
+        load4_const(a.tF + ts, Fs);
 #pragma unroll
         for (int v = 0; v < NV; ++v) Fs[v] *= sgS;   // F_S . n_S
         load4_const(a.metrics + ((size_t)se * nn + ns) * 4, J);
@@ -92,8 +92,8 @@ static __global__ void __launch_bounds__(128) curved_mortar_kernel(CurvedMortarA
             const int li = rev ? n - 1 - i : i;
             const int nl = face_node_index(n, lf, li);
             double x[NV], y[NV], z[NV], JL[4];
-            load4(a.u + ((size_t)lg * nn + nl) * NV, x);
-            load4(a.tU + (((size_t)lg * 4 + lf) * n + li) * NV, y);
+            load4_const(a.u + ((size_t)lg * nn + nl) * NV, x);
+            load4_const(a.tU + (((size_t)lg * 4 + lf) * n + li) * NV, y);
             load4_const(a.metrics + ((size_t)lg * nn + nl) * 4, JL);
             const double nL[2] = {-0.5 * (sgL * (lf < 2 ? JL[0] : JL[2])), -0.5 * (sgL * (lf < 2 ? JL[1] : JL[3]))};
             euler_flux_normal(gm1, x, nL, z);
@@ -105,7 +105,7 @@ static __global__ void __launch_bounds__(128) curved_mortar_kernel(CurvedMortarA
                 Fl[v] = fma(c, z[v], Fl[v]);
             }
             if (a.alpha) {
-                load4(a.tFn + (((size_t)lg * 4 + lf) * n + i) * NV, x);
+                load4_const(a.tFn + (((size_t)lg * 4 + lf) * n + i) * NV, x);
 #pragma unroll
                 for (int v = 0; v < NV; ++v) fir[v] = fma(c, x[v], fir[v]);
             }
@@ -121,8 +121,8 @@ static __global__ void __launch_bounds__(128) curved_mortar_kernel(CurvedMortarA
             for (int v = 0; v < NV; ++v)
                 fn[v] = 0.5 * ((fS[v] * nrm[0] + gS[v] * nrm[1]) + (fL[v] * nrm[0] + gL[v] * nrm[1])) +
                         (-0.5 * lam * (ul[v] - us[v]));
-            load4(a.tFn + ts, fil);
-            const double alp = 0.5 * (a.alpha[se] + a.alpha[lg]);
+            load4_const(a.tFn + ts, fil);
+            const double alp = 0.5 * (__ldg(a.alpha + se) + __ldg(a.alpha + lg));
 #pragma unroll
             for (int v = 0; v < NV; ++v) fstar[v] = (1.0 - alp) * fstar[v] + alp * fn[v];
             const double dt = *a.dt;

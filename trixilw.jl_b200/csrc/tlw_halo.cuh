@@ -69,18 +69,18 @@ static __global__ void __launch_bounds__(128) halo_pack_kernel(HaloArgs a) {
     const int e = __ldg(a.elem + k), f = __ldg(a.face + k);
     const int node = halo_face_node(n, f, l);
     double x[NV], y[NV], z[NV];
-    load4(a.u + ((size_t)e * nn + node) * NV, x);
+    load4_const(a.u + ((size_t)e * nn + node) * NV, x);
     const size_t tb = (((size_t)e * 4 + f) * n + l) * NV;
-    load4(a.tU + tb, y);
-    load4(a.tF + tb, z);
+    load4_const(a.tU + tb, y);
+    load4_const(a.tF + tb, z);
     double* s = a.send + ((size_t)__ldg(a.slot + k) * n + l) * a.values;
     store4(s, x);
     store4(s + NV, y);
     store4(s + 2 * NV, z);
     if (a.alpha) {
-        load4(a.tFn + tb, x);
+        load4_const(a.tFn + tb, x);
         store4(s + 3 * NV, x);
-        s[4 * NV] = a.alpha[e];
+        s[4 * NV] = __ldg(a.alpha + e);
     }
 }
 
@@ -93,14 +93,14 @@ static __global__ void __launch_bounds__(128) halo_face_kernel(HaloArgs a) {
     const int e = __ldg(a.elem + k), f = __ldg(a.face + k);
     const int node = halo_face_node(n, f, l);
     double ul[NV], Ul[NV], Fl[NV], ur[NV], Ur[NV], Fr[NV], Fn[NV];
-    load4(a.u + ((size_t)e * nn + node) * NV, ul);
+    load4_const(a.u + ((size_t)e * nn + node) * NV, ul);
     const size_t tb = (((size_t)e * 4 + f) * n + l) * NV;
-    load4(a.tU + tb, Ul);
-    load4(a.tF + tb, Fl);
+    load4_const(a.tU + tb, Ul);
+    load4_const(a.tF + tb, Fl);
     const double* r = a.recv + ((size_t)__ldg(a.slot + k) * n + l) * a.values;
-    load4(r, ur);
-    load4(r + NV, Ur);
-    load4(r + 2 * NV, Fr);
+    load4_const(r, ur);
+    load4_const(r + NV, Ur);
+    load4_const(r + 2 * NV, Fr);
     const bool local_left = f & 1;   // +x / +y face: the local element is the interface's left side
     if (local_left)
         lw_surface_flux(a.gamma, a.flux_kind, a.speed_kind, Fl, Fr, Ul, Ur, ul, ur, a.orientation, Fn, a.status);
@@ -109,9 +109,9 @@ static __global__ void __launch_bounds__(128) halo_face_kernel(HaloArgs a) {
     if (a.alpha) {
         // the interface kernel's blend with the remote side's alpha and fn_low (compute_alp, dg_2d.jl:1879-1901)
         double fl[NV], fr[NV];
-        load4(a.tFn + tb, fl);
-        load4(r + 3 * NV, fr);
-        const double al = a.alpha[e], ar = r[4 * NV];
+        load4_const(a.tFn + tb, fl);
+        load4_const(r + 3 * NV, fr);
+        const double al = __ldg(a.alpha + e), ar = r[4 * NV];
         if (local_left)
             blend_flux_values(a.gamma, a.speed_kind, a.status, a.jac_first, a.inv_w_first, a.inv_w_last, a.orientation, ul,
                               ur, al, ar, fl, fr, *a.dt, Fn);
@@ -135,7 +135,7 @@ static __global__ void __launch_bounds__(128) halo_face_kernel(HaloArgs a) {
 static __global__ void halo_alpha_pack_kernel(const int* __restrict__ elem, const int* __restrict__ slot, int count,
                                               const double* __restrict__ alpha_raw, double* __restrict__ send) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < count) send[__ldg(slot + k)] = alpha_raw[__ldg(elem + k)];
+    if (k < count) send[__ldg(slot + k)] = __ldg(alpha_raw + __ldg(elem + k));
 }
 
 // alpha_e = max(alpha_e, alpha_raw_remote / 2) across the cut faces (the smoothing of alpha_smooth_kernel)
@@ -144,7 +144,7 @@ static __global__ void halo_alpha_smooth_kernel(const int* __restrict__ elem, co
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= count) return;
     unsigned long long* ab = reinterpret_cast<unsigned long long*>(alpha);
-    atomicMax(ab + __ldg(elem + k), (unsigned long long)__double_as_longlong(0.5 * recv[__ldg(slot + k)]));
+    atomicMax(ab + __ldg(elem + k), (unsigned long long)__double_as_longlong(0.5 * __ldg(recv + __ldg(slot + k))));
 }
 
 }  // namespace tlw

@@ -599,7 +599,7 @@ static __global__ void __launch_bounds__(MS_THREADS) par_speed_kernel(const doub
     double vis = 0.0;
     for (int k = threadIdx.x; k < ne * nn; k += MS_THREADS) {
         double x[NV];
-        load4(u + ((size_t)e0 * nn + k) * NV, x);
+        load4_const(u + ((size_t)e0 * nn + k) * NV, x);
         const double ir = 1.0 / x[0];
         const double v1 = x[1] * ir, v2 = x[2] * ir;
         const double p = gm1 * (x[3] - 0.5 * (x[1] * v1 + x[2] * v2));

@@ -785,8 +785,8 @@ static __global__ void __launch_bounds__(256) cfl_slots_reduce_kernel(const unsi
         unsigned long long b1 = 0ull, b2 = 0ull;
 #pragma unroll
         for (int k = 0; k < CFL_SLOTS / 2; ++k) {
-            b1 = max(b1, sl[2 * k]);
-            b2 = max(b2, sl[2 * k + 1]);
+            b1 = max(b1, __ldg(sl + 2 * k));
+            b2 = max(b2, __ldg(sl + 2 * k + 1));
         }
         m = fmax(m, __ldg(inv_jac + e) * (__longlong_as_double((long long)b1) + __longlong_as_double((long long)b2)));
     }
