@@ -22,10 +22,6 @@
 
 namespace tlw {
 
-#ifndef TLW_CURVED_MINB
-#define TLW_CURVED_MINB 4
-#endif
-
 // Trixi max_abs_speed_naive (kind 0) / max_abs_speed (kind 1) with a normal direction
 __device__ __forceinline__ double max_abs_speed_normal(double gamma, const double* ul, const double* ur,
                                                        const double* nrm, int kind, unsigned* status) {
@@ -453,9 +449,10 @@ static __global__ void __launch_bounds__(128) curved_boundary_kernel(CurvedBndAr
 // phase 2, one thread per face node, lifts the xi face's and then the eta face's flux and reduces the element's CFL
 // speeds. It replaces a launch per colour and two for the boundaries, each of which read and wrote the face nodes:
 // 201 x 167, N = 4: two colours of 19.8 us and a CFL pass of 16.8 become one pass of 34.8, 126 -> 110 us a step; the 64 x 64
-// cavity: four launches, 28 us, become one of 13.
+// cavity: four launches, 28 us, become one of 13. (4 CTAs an SM: 1, 3 and 5 take the same time within 0.3 %, 16^2 to
+// 160^2, N = 3, 4, 5, 7.)
 template <int N, bool PLAIN>
-static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, TLW_CURVED_MINB)
+static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, 4)
     curved_surface_kernel(CurvedSurfArgs a, CurvedBndArgs bnd) {
     using C = SurfCfg<N>;
     constexpr int n = N + 1, nn = n * n, EB = C::EB, NB = 4 * (n - 1);

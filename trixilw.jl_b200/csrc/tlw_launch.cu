@@ -285,11 +285,11 @@ struct LaunchImpl {
             if (h->curved) {
                 pa.inv_jac = h->d_ijn;
                 pa.metrics = h->d_Ja;
-                if (mode == MODE_RHS) launch_dependent(s, par_volume_kernel<N, MODE_RHS, true>, grid, P::THREADS, P::smem_bytes(), pa);
-                else launch_dependent(s, par_volume_kernel<N, MODE_STEP, true>, grid, P::THREADS, P::smem_bytes(), pa);
+                if (mode == MODE_RHS) launch_dependent(s, par_volume_kernel<N, MODE_RHS, true>, grid, P::THREADS, P::launch_bytes(grid), pa);
+                else launch_dependent(s, par_volume_kernel<N, MODE_STEP, true>, grid, P::THREADS, P::launch_bytes(grid), pa);
             } else {
-                if (mode == MODE_RHS) launch_dependent(s, par_volume_kernel<N, MODE_RHS>, grid, P::THREADS, P::smem_bytes(), pa);
-                else launch_dependent(s, par_volume_kernel<N, MODE_STEP>, grid, P::THREADS, P::smem_bytes(), pa);
+                if (mode == MODE_RHS) launch_dependent(s, par_volume_kernel<N, MODE_RHS>, grid, P::THREADS, P::launch_bytes(grid), pa);
+                else launch_dependent(s, par_volume_kernel<N, MODE_STEP>, grid, P::THREADS, P::launch_bytes(grid), pa);
             }
         }
     }
@@ -310,13 +310,13 @@ struct LaunchImpl {
     static void par_attributes() {
         if constexpr (N >= 3) {
             cudaFuncSetAttribute(par_volume_kernel<N, MODE_RHS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ParCfg<N>::smem_bytes());
+                                 (int)ParCfg<N>::max_bytes());
             cudaFuncSetAttribute(par_volume_kernel<N, MODE_STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ParCfg<N>::smem_bytes());
+                                 (int)ParCfg<N>::max_bytes());
             cudaFuncSetAttribute(par_volume_kernel<N, MODE_RHS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ParCfg<N>::smem_bytes());
+                                 (int)ParCfg<N>::max_bytes());
             cudaFuncSetAttribute(par_volume_kernel<N, MODE_STEP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ParCfg<N>::smem_bytes());
+                                 (int)ParCfg<N>::max_bytes());
         }
     }
     static void mortars(cudaStream_t s, const MortarArgs& a) {

@@ -63,13 +63,28 @@ struct ParCfg {
     static constexpr int EB = VolCfg<N>::EB;
     static constexpr int THREADS = VolCfg<N>::THREADS;
     static constexpr int DEPTH = N >= 4 ? 4 : 3;
-#ifndef TLW_PAR_MB
-#define TLW_PAR_MB 3
-#endif
-    static constexpr int MIN_BLOCKS = THREADS <= 128 ? TLW_PAR_MB : 1;
+    // CTAs an SM the registers must allow (3: 168; uncapped 218-226, two CTAs). Us a step with 2, 3, 4: TreeMesh 128^2
+    // N = 3 64.1 / 62.9 / 65.0, N = 4 137.2 / 136.1 / 155.6, N = 5 213.8 / 207.3 / 245.9; curvilinear 64^2 N = 4
+    // 48.4 / 47.7 / 53.2
+    static constexpr int MIN_BLOCKS = THREADS <= 128 ? 3 : 1;
     static constexpr int TILE = NV * EB * nn;   // 4 values per node of the CTA
     // D, Dhat; contraction tiles X, Y, W; perturbed states P (4) and their gradients GX, GY (4 + 4)
     static constexpr size_t smem_bytes() { return (size_t)(2 * nn + 15 * TILE) * sizeof(double); }
+    // Shared memory of a launch of `grid` CTAs. As a programmatic dependent launch it is placed while the CTAs in front
+    // run out, onto the SMs that come free first, up to MIN_BLOCKS on one, and a grid smaller than the device then waits
+    // for those SMs: so up to one CTA an SM asks for so much that one fits, up to two an SM that two do (228 KB an SM,
+    // 1 KB of it taken by each CTA). Us a step, N = 3, 4, without and with: 32^2 TreeMesh 21.8 / 17.5, 28.8 / 24.8;
+    // 24^2 curvilinear 16.9 / 16.9, 29.3 / 22.8; 36^2 22.7 / 20.2, 30.3 / 25.9; the launch the ordinary way 17.1, 24.3;
+    // 17.4, 22.0; 20.0, 25.9.
+    static constexpr size_t ONE_PER_SM = 114 * 1024, TWO_PER_SM = 76 * 1024;
+    static constexpr int SMS = 148;
+    static constexpr size_t launch_bytes(int grid) {
+        const size_t least = grid <= SMS ? ONE_PER_SM : grid <= 2 * SMS ? TWO_PER_SM : 0;
+        return least > smem_bytes() ? least : smem_bytes();
+    }
+    static constexpr size_t max_bytes() { return launch_bytes(1); }
+    static_assert(2 * (ONE_PER_SM + 1024) > 228 * 1024 && 3 * (TWO_PER_SM + 1024) > 228 * 1024 &&
+                  2 * (TWO_PER_SM + 1024) <= 228 * 1024, "spread of small grids");
 };
 
 // gradient volume term: gx = J^{-1} Dhat u (along i), gy = J^{-1} Dhat u (along j); on a curvilinear mesh
