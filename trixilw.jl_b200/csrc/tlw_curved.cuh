@@ -263,7 +263,7 @@ __device__ __forceinline__ void curved_interface_flux(const CurvedSurfArgs& a, i
     constexpr int nn = n * n;
     const int np = face_node_index(n, pf, l), ns = face_node_index(n, sf, ls);
     const double sgP = (pf & 1) ? 1.0 : -1.0, sgS = (sf & 1) ? 1.0 : -1.0;
-    double uP[NV], uS[NV], UP[NV], US[NV], FP[NV], FS[NV], J[4];
+    double uP[NV], uS[NV], UP[NV], US[NV], FP[NV], FS[NV], vP[NV], vS[NV], J[4];
     // (node records, traces and metrics move as one 256-bit access each)
     load4w(a.u + ((size_t)pe * nn + np) * NV, uP);
     load4w(a.u + ((size_t)se * nn + ns) * NV, uS);
@@ -282,15 +282,18 @@ __device__ __forceinline__ void curved_interface_flux(const CurvedSurfArgs& a, i
             FP[v] *= sgP;     // F_P . n_P
             FS[v] *= -sgS;    // F_S . (-n_S)
         }
+        // (in front of the flux, whose check may write the status word: loads do not move across that. 128^2, us a
+        // step behind / in front of it: N = 4 149.0 / 147.9, N = 5 225.9 / 223.8)
+        if (!PLAIN && a.tFv) {
+            load4w(a.tFv + tp, vP);
+            load4w(a.tFv + ts, vS);
+        }
         lw_surface_flux_normal(a.gamma, a.flux_kind, a.speed_kind, FP, FS, uP, uS, UP, US, nrm, Fn, a.status);
         if (!PLAIN && a.alpha) blend_curved_flux<N>(a, pe, se, pf, sf, l, np, uP, uS, nrm, Fn);
     }
     if (!PLAIN && a.tFv) {
         // minus the mean of both sides' viscous normal fluxes (calc_interface_flux_hyperbolic_parabolic!,
         // src/solvers/dgsem_p4est/dg_2d_parabolic.jl:1878-1958)
-        double vP[NV], vS[NV];
-        load4w(a.tFv + tp, vP);
-        load4w(a.tFv + ts, vS);
 #pragma unroll
         for (int v = 0; v < NV; ++v) Fn[v] -= 0.5 * (sgP * vP[v] + (-sgS) * vS[v]);
     }
