@@ -215,11 +215,12 @@ struct tlw_handle {
     cudaGraphExec_t g_one[2] = {nullptr, nullptr};
     cudaGraphExec_t g_two[2] = {nullptr, nullptr};
     cudaGraphExec_t g_many = nullptr;       // MANY_STEPS steps from buffer 0
-    // Its capture takes the host 65 (256^2) to 185 us (16^2, shock capturing). In a call of 64 steps it gains 1.4 us a
-    // step (16^2, N = 4: 618 -> 522 us a call), and behind MANY_QUEUED steps of the call (190 us at 16^2) the device does
-    // not wait for the capture: a new handle's first 64 steps take 785 us, 865 with the capture in front of them. In
-    // calls of 16 steps it gains 0.3 (16^2) to 0.8 us (256^2) a step, so shorter calls earn it after MANY_AFTER steps.
-    static constexpr int MANY_STEPS = 8, MANY_QUEUED = 24, MANY_AFTER = 400;
+    // Its capture takes the host 65 (256^2) to 205 us (16^2, MDRK). In a call of 64 steps it gains 1.4 us a step (16^2,
+    // N = 4: 618 -> 522 us a call), and behind MANY_QUEUED steps of the call (190 us at 16^2) the device does not wait
+    // for the capture: a new handle's first 64 steps take 785 us, 865 with the capture in front of them. In calls of 8
+    // to 16 steps it gains 0.3 (16^2, LW), 0.8 (256^2), 1.6 us a step (16^2, Navier-Stokes), so shorter calls have
+    // earned it after MANY_AFTER steps.
+    static constexpr int MANY_STEPS = 8, MANY_QUEUED = 24, MANY_AFTER = 200;
     long long replayed = 0;                 // steps launched from these graphs
     // discrete adjoint
     tlw::AdjointBuffers adj;
