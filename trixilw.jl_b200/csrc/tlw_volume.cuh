@@ -747,45 +747,47 @@ __device__ __forceinline__ void write_interior_slots(const VolArgs& a, double* X
 }
 
 // Flux pairs and their stencils. The stencils of the time derivatives of f and g are sums over the perturbed states
-// of products, of which five differ: rho v1^2, rho |v|^2, rho v1 v2, H v1 and H v2 (H = rho e + p); what is linear in
+// of products, of which five differ: rho v1^2, rho v2^2, rho v1 v2, H v1 and H v2 (H = rho e + p); what is linear in
 // the state (rho v1, rho v2 and the rho e part of p) has a stencil of L times the current derivative d of the state,
-// L the stencil's moment, so it is not summed at all: f = (L d_2, a + P, b, x), g = (L d_3, b, (s - a) + P, y) with
-// P = (gamma - 1)(L d_4 - s / 2). A state carries gamma rho e as its last variable, so that H is one multiply-add.
-// A stage of four pairs then takes 60 FP64 instructions instead of 96 (N = 4: about 730 -> 607 a node, counted).
+// L the stencil's moment, so it is not summed at all: f = (L d_2, a + P, b, x), g = (L d_3, b, c + P, y) with
+// P = (gamma - 1)(L d_4 - (a + c) / 2). A state carries gamma rho e as its last variable, so that H is one multiply-add.
+// A stage of four pairs then takes 64 FP64 instructions instead of 96 (N = 4: about 730 -> 626 a node, counted). Summing
+// rho |v|^2 in the place of rho v2^2 saves 4 of them and no time (512^2 5071 against 5078 us a pass of 8 steps, warped
+// 201 x 167 880 against 872), but rounds the small flux of rho v2 by the large one of a stream along x: at Mach 30 the
+// error of its rhs is 2 to 2.5 times that of the mirrored stream (N = 3, 4, 5).
 struct StencilSum {
-    double a, s, b, x, y;
+    double a, c, b, x, y;
 };
 // the products at p plus (SGN = 1) or minus (SGN = -1) those at m; hg = (gamma - 1) / 2, irp, irm = 1 / rho
 template <int SGN>
 __device__ __forceinline__ StencilSum stencil_pair(double hg, const double* p, double irp, const double* m, double irm) {
     const double v1 = p[1] * irp, v2 = p[2] * irp, w1 = m[1] * irm, w2 = m[2] * irm;
-    const double ap = p[1] * v1, am = m[1] * w1;
-    const double sp = fma(p[2], v2, ap), sm = fma(m[2], w2, am);
-    const double hp = fma(-hg, sp, p[3]), hm = SGN * fma(-hg, sm, m[3]);
-    return StencilSum{fma((double)SGN, am, ap), fma((double)SGN, sm, sp), fma(SGN * m[1], w2, p[1] * v2),
+    const double ap = p[1] * v1, am = m[1] * w1, cp = p[2] * v2, cm = m[2] * w2;
+    const double hp = fma(-hg, ap + cp, p[3]), hm = SGN * fma(-hg, am + cm, m[3]);
+    return StencilSum{fma((double)SGN, am, ap), fma((double)SGN, cm, cp), fma(SGN * m[1], w2, p[1] * v2),
                       fma(hm, w1, hp * v1), fma(hm, w2, hp * v2)};
 }
 __device__ __forceinline__ StencilSum stencil_fma(double c, const StencilSum& t, const StencilSum& q) {   // c t + q
-    return StencilSum{fma(c, t.a, q.a), fma(c, t.s, q.s), fma(c, t.b, q.b), fma(c, t.x, q.x), fma(c, t.y, q.y)};
+    return StencilSum{fma(c, t.a, q.a), fma(c, t.c, q.c), fma(c, t.b, q.b), fma(c, t.x, q.x), fma(c, t.y, q.y)};
 }
 __device__ __forceinline__ StencilSum stencil_fmsub(double c, const StencilSum& t, const StencilSum& q) {  // c t - q
-    return StencilSum{fma(c, t.a, -q.a), fma(c, t.s, -q.s), fma(c, t.b, -q.b), fma(c, t.x, -q.x), fma(c, t.y, -q.y)};
+    return StencilSum{fma(c, t.a, -q.a), fma(c, t.c, -q.c), fma(c, t.b, -q.b), fma(c, t.x, -q.x), fma(c, t.y, -q.y)};
 }
 __device__ __forceinline__ void stencil_fluxes(double gm1, double hg, double L, const StencilSum& r, const double* d,
                                                double* f, double* g) {
-    const double P = fma(-hg, r.s, gm1 * (L * d[3]));
+    const double P = fma(-hg, r.a + r.c, gm1 * (L * d[3]));
     f[0] = L * d[1]; f[1] = r.a + P; f[2] = r.b; f[3] = r.x;
-    g[0] = L * d[2]; g[1] = r.b; g[2] = (r.s - r.a) + P; g[3] = r.y;
+    g[0] = L * d[2]; g[1] = r.b; g[2] = r.c + P; g[3] = r.y;
 }
 // the flux pair at u (unscaled rho e) and its products
 __device__ __forceinline__ StencilSum flux_base(double gm1, const double* u, double* f, double* g) {
     const double ir = nr_reciprocal(u[0]);
     const double v1 = u[1] * ir, v2 = u[2] * ir;
-    const double a = u[1] * v1, s = fma(u[2], v2, a), b = u[1] * v2;
-    const double p = gm1 * fma(-0.5, s, u[3]), h = u[3] + p;
+    const double a = u[1] * v1, c = u[2] * v2, b = u[1] * v2;
+    const double p = gm1 * fma(-0.5, a + c, u[3]), h = u[3] + p;
     f[0] = u[1]; f[1] = a + p; f[2] = b; f[3] = h * v1;
-    g[0] = u[2]; g[1] = b; g[2] = fma(u[2], v2, p); g[3] = h * v2;
-    return StencilSum{a, s, b, f[3], g[3]};
+    g[0] = u[2]; g[1] = b; g[2] = c + p; g[3] = h * v2;
+    return StencilSum{a, c, b, f[3], g[3]};
 }
 
 // the four reciprocals of a stage first, as independent chains
