@@ -109,13 +109,34 @@ def mdrk_volume_bytes_per_element(N: int) -> float:
     return 8.0 * (7 * nv * n * n + 2 * 2 * 4 * n * nv)
 
 
+def line_flops(n: int) -> int:
+    """FP64 flops of one line of n nodes through a derivative matrix (FMA = 2): the dense product, or from five nodes on
+    its even-odd form, 2h sums and differences, h rows of two h-term products each for two outputs, the middle row and
+    column where n is odd (h = n // 2)."""
+    h, odd = n // 2, n % 2
+    if n < 5:
+        return n * (2 * n - 1)
+    return 2 * h + h * (2 * (2 * h - 1) + 2 + 2 * odd) + odd * (2 * h - 1)
+
+
+def contraction_flops_per_node(n: int) -> float:
+    """One derivative contraction of four variables in two directions, with the sum of both."""
+    return 2 * 4 * line_flops(n) / n + 4
+
+
+# FP64 flops of the node phases (FMA = 2, divides not counted) in their cheapest known form, the stencils as sums of the
+# five distinct flux products: the flux pair at a state, one pair of perturbed states (u + k d, u - k d) into the sums,
+# one combination of two sums, the fluxes from them
+FLUX_BASE, STENCIL_PAIR, COMBINE, STENCIL_FLUXES = 14, 25, 10, 9
+
+
 def mdrk_volume_flops_per_node(N: int) -> float:
-    """Algorithmic FP64 flops per node of the two MDRK stage kernels of a step (FMA = 2, divides not counted):
-    2 (8 n nv + 5 F_pair + 120) with F_pair = 17, the survey's count for two stages of two line contractions and
-    five flux pairs each. (The compact stages recompute stage 1's five flux pairs in stage 2 instead of storing
-    U2 and F2; those flops are not algorithmic and not counted.)"""
-    n, nv = N + 1, 4
-    return 2 * (8 * n * nv + 5 * 17 + 120)
+    """Algorithmic FP64 flops per node of the two MDRK stage kernels of a step (FMA = 2, divides not counted). (The
+    compact stages recompute stage 1's sums in stage 2 instead of storing U2 and F2; those flops are not algorithmic
+    and not counted.)"""
+    stage = (FLUX_BASE + 2 * contraction_flops_per_node(N + 1) + 5 + (2 + 8 + 16) + 2 * STENCIL_PAIR + COMBINE + STENCIL_FLUXES
+             + 8)
+    return 2 * stage + (24 + 12) + (16 + 8)   # stage 1's F = f / 2 + f_t / 8, U; stage 2's F2 + f_t / 3, U
 
 
 def surface_pass_bytes_per_element(N: int) -> float:
@@ -139,12 +160,15 @@ def ns_volume_bytes_per_element(N: int) -> float:
 
 
 def volume_flops_per_node(N: int) -> float:
-    """Algorithmic FP64 flops per node of the LW volume kernel (FMA = 2, divides not counted):
-    N >= 4: 20 n nv + 17 * 17 + 300; N = 3: 16 n nv + 11 * 17 + 200."""
-    n, nv = N + 1, 4
-    if N >= 4:
-        return 20 * n * nv + 17 * 17 + 300
-    return 16 * n * nv + 11 * 17 + 200
+    """Algorithmic FP64 flops per node of the LW volume kernel of depth min(N, 4) (FMA = 2, divides not counted): per
+    stage the scaled derivative, the four perturbed states, their pairs and combinations, the fluxes and their share of
+    the time averages; the quadrature of U; the update."""
+    depth = min(N, 4)
+    pairs = {1: [1], 2: [1, 1], 3: [2, 1, 2], 4: [2, 2, 2, 2]}[depth]     # pairs of states per stage
+    combos = {1: [0], 2: [0, 1], 3: [1, 1, 1], 4: [1, 2, 1, 2]}[depth]
+    states = 4 if depth >= 3 else 2
+    stages = sum(6 + 8 * states + p * STENCIL_PAIR + c * COMBINE + STENCIL_FLUXES + 10 for p, c in zip(pairs, combos))
+    return FLUX_BASE + 1 + stages + (42 if depth >= 3 else 26) + 8 + (depth + 1) * contraction_flops_per_node(N + 1)
 
 
 def host_link(nbytes: int, stream) -> dict:
