@@ -529,7 +529,7 @@ static __global__ void __launch_bounds__(SurfCfg<N>::THREADS, 4)
 
 // CFL reduction on curvilinear meshes (Trixi max_dt): per element max_nodes |Ja^1 . (l1, l2)| |J^{-1}| +
 // max_nodes |Ja^2 . (l1, l2)| |J^{-1}|, l_d = |v_d| + c. A CTA takes MsCfg<N>::ELEMS elements: a coalesced pass
-// over their nodes into shared memory, then one thread per element reduces its nodes.
+// over their nodes into shared memory, then MsCfg<N>::LANES threads per element reduce its nodes.
 template <int N>
 static __global__ void __launch_bounds__(MS_THREADS) curved_max_speed_kernel(const double* u,
                                                                              const double* __restrict__ metrics,

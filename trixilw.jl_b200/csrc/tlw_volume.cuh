@@ -1,7 +1,7 @@
 // tlw_volume.cuh -- fused per-element LW / MDRK volume kernels for TreeMesh{2} (FP64, sm_100a).
 //
 // Work split inside a CTA of EB whole elements (N=3: 8 x 16 nodes in 128 threads, N=4: 5 x 25 in 128,
-// N=5: 7 x 36 in 256):
+// N=5: 3 x 36 in 128):
 //  * node phase - one thread per GLL node ("owner") evaluates the Euler flux products at the perturbed states
 //    (StencilSum) and keeps the LW stage state (u +- ut, u +- 2ut, the time averages F, G) in registers;
 //  * line phase - each 1-D derivative contraction is done by one thread per (variable, element, line
@@ -165,7 +165,7 @@ __device__ __forceinline__ void contravariant(const double* Ja, const double* f,
 // N = 4 0.4522 -> 0.4495, N = 5 0.7457 -> 0.7303). Threads ask for one 128-byte line each; nothing past the array.
 template <class C>
 __device__ __forceinline__ void prefetch_next(const double* p, int K, int E, int tid) {
-    constexpr int AHEAD = 148 * C::MIN_BLOCKS;
+    constexpr int AHEAD = 148 * C::MIN_BLOCKS;   // (SMs x CTAs)
     const size_t first = ((size_t)blockIdx.x + AHEAD) * C::NODES * K + (size_t)tid * 16;
     if (tid * 16 < C::NODES * K && first < (size_t)E * C::nn * K)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(p + first));
