@@ -78,3 +78,23 @@ def test_split_steps_between_steps(oracle_mod, tl, N, td, periodic, limiter):
         assert integ.t == pytest.approx(t, rel=1e-13)
     a, b = integ.get_state().reshape(-1, 4), ref.reshape(-1, 4)
     assert np.all(np.linalg.norm(a - b, axis=0) < 1e-12 * np.linalg.norm(b, axis=0))
+
+
+def test_recorded_run_after_host_steps(tl):
+    """Host-buffer stepping changes the handle's state buffers and leaves its last download in flight; a recorded run
+    after it (whose graph was captured before) gives the same state and leaves the download alone."""
+    semi = make(tl, 4)
+    integ = tl.LWIntegrator(tl.semidiscretize(semi, semi.time_discretization, (0.0, 1e9)))
+    u = semi.compute_coefficients(0.0)
+    integ.set_state(u, 0.0)
+    first = tl.forward_record(semi, u, 7, 0.2, 3)
+    a, b, c = (integ.pinned_state() for _ in range(3))
+    a[:] = 1.01 * u
+    integ.step_host(a, b, 0.0, 2, 0.2)
+    integ.synchronize()
+    expected = b.copy()
+    for _ in range(2):
+        integ.step_host(a, c, 0.0, 2, 0.2)
+        np.testing.assert_array_equal(tl.forward_record(semi, u, 7, 0.2, 3), first)
+        integ.synchronize()
+        np.testing.assert_array_equal(c, expected)

@@ -1049,6 +1049,11 @@ int adj_ready(tlw_handle* h) {
                      "adjoint: LW or MDRK, FR volume integral, Rusanov flux, periodic conforming TreeMesh, Euler, "
                      "N = 3..5, no positivity limiter");
     TLW_ACUDA(h, cudaSetDevice(h->device));
+    if (h->async_pending) {
+        // the recorded run takes the state buffers: after tlw_step_host's last download
+        TLW_ACUDA(h, cudaStreamWaitEvent(h->stream, h->ev_dl[(h->host_calls - 1) % tlw_handle::HOST_CALLS], 0));
+        h->async_pending = false;
+    }
     AdjointBuffers& A = h->adj;
     if (!A.const_uploaded) {
         Basis all[8];
@@ -1499,9 +1504,11 @@ int tlw_forward_record(tlw_handle* h, const double* u0, int32_t nsteps, double c
         return TLW_OK;
     };
     const long long key = (long long)nsteps * 100003 + ck;
-    if (!A.g_fwd || A.g_fwd_key != key) {
+    if (!A.g_fwd || A.g_fwd_key != key || A.g_fwd_state[0] != h->d_state[0] || A.g_fwd_state[1] != h->d_state[1]) {
         if ((rc = capture_graph(h, A.g_fwd, body))) return rc;
         A.g_fwd_key = key;
+        A.g_fwd_state[0] = h->d_state[0];
+        A.g_fwd_state[1] = h->d_state[1];
     }
     TLW_ACUDA(h, cudaGraphLaunch(A.g_fwd, h->stream));
     A.d_final = seg_state(h, bl, nsteps - last);

@@ -56,6 +56,7 @@ struct AdjointBuffers {
     // they address is replaced
     cudaGraphExec_t g_fwd = nullptr, g_rev = nullptr;
     long long g_fwd_key = -1, g_rev_key = -1;
+    const double* g_fwd_state[2] = {nullptr, nullptr};   // the state buffers it runs in (tlw_step_host changes them)
     bool const_uploaded = false;            // the adjoint translation unit's constant bank is set
 };
 
