@@ -226,9 +226,11 @@ bool use_slots(const tlw_handle* h) {
 #define TLW_MDRK_COMPACT 1
 #endif
 // (shock capturing: meshes of up to 4 million nodes without mortars. Both sides of a face evaluate the blended flux, so
-// the pass pays as long as the traces of U, F and fn_low stay near the caches: Riemann problem, us a step with the sweeps
-// and boundary launches against the pass: 16^2 N = 4 31 / 22.5, 64^2 N = 4 38 / 34, 256^2 N = 3 144 / 135, N = 4 240 / 222,
-// N = 5 332 / 316, N = 6 (3.2 million nodes) 469 / 465; 512^2 N = 3 (4.2 million) 472 / 482, N = 5 1179 / 1186)
+// the pass pays as long as the traces of U, F and fn_low stay near the caches. Us a step with the sweeps and boundary
+// launches against the pass, a smooth wave that blends nothing / four states / a blast between walls: 256^2 N = 3
+// 122.2 122.0 / 122.7 122.7 / 130.4 122.3, N = 4 219 213 / 219 213 / 227 210, N = 5 307 301 / 308 302 / 316 299, N = 6 (3.2
+// million nodes) 440.9 442.9 / 440.4 442.6 / 447.8 443.2, N = 7 (4.2) 478 466 / 477 466; 512^2 N = 3 (4.2) 435 452 / 437
+// 454 / 445 449, N = 4 (6.6) 794 805 / 794 806 / 801 796; four states 16^2 N = 4 31 / 22.5, 64^2 38 / 34)
 bool use_surface_pass(const tlw_handle* h) {
     if (h->sc && (h->nmx + h->nmy > 0 || (int64_t)h->E * h->nn > 4000000)) return false;
     return TLW_SURFACE_PASS && h->d_nbr && !h->curved && h->nh == 0 && (h->nmx + h->nmy == 0 || h->nbr_mortars);
